@@ -28,14 +28,11 @@
 
 #include "df.cuh"
 #include "gfe_internal.cuh"
+#include "mr_jac64.cuh"
+#include "mr_point.cuh"
 #include "tcgen05.cuh"
 
 namespace {
-
-constexpr int NQ = 27;   // quadratic element nodes
-constexpr int NL = 8;    // linear (pressure) element nodes
-constexpr int NG = 27;   // Gauss points (3x3x3)
-constexpr int ND = 89;   // element DOFs
 
 // 16-byte multiple in size, so that a TMA bulk copy can stage the whole table
 template <typename S>
@@ -125,66 +122,6 @@ int device_tables_f(const TablesF** out) {
   return GFE_OK;
 }
 
-// Voigt index of tensor entry (i, j) and the tensor entries of Voigt index v, as arithmetic so that
-// unrolled loops index register arrays with constants: 11 22 33 12 13 23.
-__host__ __device__ constexpr int t2v(int i, int j) { return i == j ? i : i + j + 2; }
-__host__ __device__ constexpr int v2t_a(int v) { return v < 3 ? v : (v == 5 ? 1 : 0); }
-__host__ __device__ constexpr int v2t_b(int v) { return v < 3 ? v : (v == 3 ? 1 : 2); }
-
-// Inverse and determinant with Iron's cofactor formulas (src/maths.F90:2807-2868).
-template <typename S>
-__device__ __forceinline__ S inv3(const S A[3][3], S B[3][3]) {
-  const S det = A[0][0] * A[1][1] * A[2][2] + A[0][1] * A[1][2] * A[2][0] + A[0][2] * A[1][0] * A[2][1] -
-                A[0][0] * A[2][1] * A[1][2] - A[1][0] * A[0][1] * A[2][2] - A[2][0] * A[1][1] * A[0][2];
-  const S r = S(1) / det;
-  B[0][0] = (A[1][1] * A[2][2] - A[2][1] * A[1][2]) * r;
-  B[1][0] = (A[1][2] * A[2][0] - A[2][2] * A[1][0]) * r;
-  B[2][0] = (A[1][0] * A[2][1] - A[2][0] * A[1][1]) * r;
-  B[0][1] = (A[2][1] * A[0][2] - A[0][1] * A[2][2]) * r;
-  B[1][1] = (A[2][2] * A[0][0] - A[0][2] * A[2][0]) * r;
-  B[2][1] = (A[2][0] * A[0][1] - A[0][0] * A[2][1]) * r;
-  B[0][2] = (A[0][1] * A[1][2] - A[1][1] * A[0][2]) * r;
-  B[1][2] = (A[0][2] * A[1][0] - A[1][2] * A[0][0]) * r;
-  B[2][2] = (A[0][0] * A[1][1] - A[1][0] * A[0][1]) * r;
-  return det;
-}
-
-template <typename S>
-__device__ __forceinline__ S det3(const S A[3][3]) {
-  return A[0][0] * A[1][1] * A[2][2] + A[0][1] * A[1][2] * A[2][0] + A[0][2] * A[1][0] * A[2][1] -
-         A[0][0] * A[2][1] * A[1][2] - A[1][0] * A[0][1] * A[2][2] - A[2][0] * A[1][1] * A[0][2];
-}
-
-// Volume Jacobian sqrt|det(M^T M)| (src/coordinate_routines.F90:818-822).
-__device__ __forceinline__ double vol_jacobian(const double M[3][3]) {
-  double G[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) G[i][j] = M[0][i] * M[0][j] + M[1][i] * M[1][j] + M[2][i] * M[2][j];
-  return sqrt(fabs(det3(G)));
-}
-// The FP32 path keeps the volume Jacobian in FP64: the gradient matrix is widened exactly (integer
-// re-packing, no FP64-pipe conversion) and |det M| (= sqrt(det(M^T M)) for a square M) is taken
-// directly, which also avoids the Gram product and the square root.
-__device__ __forceinline__ float vol_jacobian(const float M[3][3]) {
-  double D[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) D[i][j] = f32_to_f64_exact(M[i][j]);
-  return (float)fabs(det3(D));
-}
-
-// Per-Gauss-point kinematics shared by residual and Jacobian.
-template <typename S>
-struct GPT {
-  S Zi[3][3];  // dxi/dz
-  S F[3][3];   // dz/dnu
-  S Jz, Jx, p, w;
-};
-using GP = GPT<double>;
-
 template <typename S>
 __device__ __forceinline__ bool gauss_point(const TablesT<S>& T, int g, const S* sz, const S* sx, const S* sp,
                                             GPT<S>& o) {
@@ -203,60 +140,13 @@ __device__ __forceinline__ bool gauss_point(const TablesT<S>& T, int g, const S*
       Z[c][k] = a;
       X[c][k] = b;
     }
-  o.Jz = vol_jacobian(Z);
-  o.Jx = vol_jacobian(X);
-  const S dz = inv3(Z, o.Zi);
-  // material frame without fibres: dX/dNu columns = normalised DX_DXI columns
-  S N[3][3], NX[3][3], A[3][3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const S n = sqrt(X[0][k] * X[0][k] + X[1][k] * X[1][k] + X[2][k] * X[2][k]);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) N[c][k] = X[c][k] / n;
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) NX[i][j] = N[0][i] * X[0][j] + N[1][i] * X[1][j] + N[2][i] * X[2][j];
-  inv3(NX, A);
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) o.F[i][j] = Z[i][0] * A[0][j] + Z[i][1] * A[1][j] + Z[i][2] * A[2][j];
+  const S dz = point_frame(Z, X, o);
   S p = S(0);
 #pragma unroll
   for (int m = 0; m < NL; ++m) p += T.psi[g][m] * sp[m];
   o.p = p;
   o.w = T.w[g];
   return dz > S(0) && o.Jx > S(0) && isfinite(dz);
-}
-
-// push-forward matrix t (src/finite_elasticity_routines.F90:1343-1375)
-template <typename S>
-__device__ __forceinline__ void push_t(const S F[3][3], S t[6][6]) {
-#pragma unroll
-  for (int j = 0; j < 6; ++j)
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const int ai = v2t_a(i), bi = v2t_b(i), aj = v2t_a(j), bj = v2t_b(j);
-      S v = F[ai][aj] * F[bi][bj];
-      if (j >= 3) v += F[ai][bj] * F[bi][aj];
-      t[i][j] = v;
-    }
-}
-
-template <typename R>
-__device__ __forceinline__ void push_vec(const R t[6][6], R S[6], R J) {
-  R o[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    R s = R(0);
-#pragma unroll
-    for (int j = 0; j < 6; ++j) s += t[i][j] * S[j];
-    o[i] = s / J;
-  }
-#pragma unroll
-  for (int i = 0; i < 6; ++i) S[i] = o[i];
 }
 
 // Cauchy stress of the residual (deviatoric MR + p), src/finite_elasticity_routines.F90:6985-7061.
@@ -536,8 +426,7 @@ mr_row_gather_kernel(int32_t nq2, int32_t nlin, const int32_t* __restrict__ cnt,
   }
 }
 
-template <typename TS>
-__global__ void widen_element_matrices(const TS* __restrict__ src, size_t n, double* __restrict__ dst) {
+__global__ void widen_element_matrices(const float* __restrict__ src, size_t n, double* __restrict__ dst) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[i] = (double)src[i];
 }
@@ -552,32 +441,6 @@ __global__ void widen_element_matrices(const TS* __restrict__ src, size_t n, dou
 // J_z Z^-T.  The element tangent / vector-Jacobian products are then contractions with the
 // constant basis tables.  This is the derivative that Iron's finite-difference Jacobian
 // (src/equations_set_routines.F90:2839-2962) approximates.
-struct Dual {
-  double v, d;
-};
-__device__ __forceinline__ Dual operator+(Dual a, Dual b) { return {a.v + b.v, a.d + b.d}; }
-__device__ __forceinline__ Dual operator-(Dual a, Dual b) { return {a.v - b.v, a.d - b.d}; }
-__device__ __forceinline__ Dual operator-(Dual a) { return {-a.v, -a.d}; }
-__device__ __forceinline__ Dual operator*(Dual a, Dual b) { return {a.v * b.v, a.v * b.d + a.d * b.v}; }
-__device__ __forceinline__ Dual operator*(double a, Dual b) { return {a * b.v, a * b.d}; }
-__device__ __forceinline__ Dual operator*(Dual a, double b) { return {a.v * b, a.d * b}; }
-__device__ __forceinline__ Dual operator/(Dual a, Dual b) {
-  const double r = 1.0 / b.v;
-  return {a.v * r, (a.d - a.v * r * b.d) * r};
-}
-__device__ __forceinline__ Dual operator/(Dual a, double b) { return {a.v / b, a.d / b}; }
-__device__ __forceinline__ Dual operator+(Dual a, double b) { return {a.v + b, a.d}; }
-__device__ __forceinline__ Dual dsqrt(Dual a) {
-  const double s = sqrt(a.v);
-  return {s, a.d / (2.0 * s)};
-}
-__device__ __forceinline__ Dual dabs(Dual a) { return a.v < 0.0 ? -a : a; }
-// x^(-1/3)
-__device__ __forceinline__ Dual dpowm13(Dual a) {
-  const double v = pow(a.v, -1.0 / 3.0);
-  return {v, -v / (3.0 * a.v) * a.d};
-}
-
 template <typename T>
 __device__ __forceinline__ T tdet3(const T A[3][3]) {
   return A[0][0] * A[1][1] * A[2][2] + A[0][1] * A[1][2] * A[2][0] + A[0][2] * A[1][0] * A[2][1] -
@@ -598,7 +461,7 @@ __device__ __forceinline__ void tinv3(const T A[3][3], T B[3][3]) {
   B[2][2] = (A[0][0] * A[1][1] - A[1][0] * A[0][1]) / det;
 }
 
-// The same forward-mode arithmetic in FP32 for the FP32 paths of the consistent tangent.
+// forward-mode dual numbers
 struct DualF {
   float v, d;
 };
@@ -618,46 +481,11 @@ __device__ __forceinline__ DualF dpowm13(DualF a) {
   return {v, -v / (3.0f * a.v) * a.d};
 }
 
-template <typename S>
-struct DualOf {
-  using type = Dual;
-};
-template <>
-struct DualOf<float> {
-  using type = DualF;
-};
-
-// J_z = sqrt|det(Z^T Z)| as Iron forms it (COORDINATE_METRICS_CALCULATE); the FP32 dual path takes
-// |det Z| (the same value for a square Z) in FP64 dual arithmetic on the exactly widened entries.
-template <typename T>
-__device__ __forceinline__ T point_jz(const T (&)[3][3], const T (&G)[3][3]) {
-  return dsqrt(dabs(tdet3(G)));
-}
-__device__ __forceinline__ DualF point_jz(const DualF (&Z)[3][3], const DualF (&)[3][3]) {
-  Dual D[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) D[i][j] = {f32_to_f64_exact(Z[i][j].v), f32_to_f64_exact(Z[i][j].d)};
-  const Dual j = dabs(tdet3(D));
-  return {(float)j.v, (float)j.d};
-}
-
-// P = w Jz Z^-1 sigma(Z, p) of the residual; also returns Jz.  R: type of the constants.  jz_given:
-// J_z (with its derivative) when the caller has formed it already.
-template <typename T, typename R = double>
-__device__ __forceinline__ void point_P(const T (&Z)[3][3], const R A[3][3], R Jx, R w, T p, R c1, R c2, T P[3][3],
-                                        T& Jz, const T* jz_given = nullptr) {
-  if (jz_given) {
-    Jz = *jz_given;
-  } else {
-    T G[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) G[i][j] = Z[0][i] * Z[0][j] + Z[1][i] * Z[1][j] + Z[2][i] * Z[2][j];
-    Jz = point_jz(Z, G);
-  }
+// P = w Jz Z^-1 sigma(Z, p) of the residual in dual numbers; Jz with its derivative from the caller.
+__device__ __forceinline__ void point_P(const DualF (&Z)[3][3], const float A[3][3], float Jx, float w, DualF p,
+                                        float c1, float c2, DualF P[3][3], DualF Jz) {
+  using T = DualF;
+  using R = float;
   T Zi[3][3];
   tinv3(Z, Zi);
   const T J = Jz / Jx;
@@ -771,33 +599,21 @@ __device__ __forceinline__ void jz_seeds(const float (&Zf)[3][3], float jz[10]) 
 }
 
 // dP/d(seed) for seed 0..8 = Z[seed/3][seed%3], seed 9 = p.  out[9] = dP[xi][mh] row-major.
-// jz: J_z and its seed derivatives from jz_seeds (FP32 path), or NULL.
-template <typename S>
-__device__ __forceinline__ void point_dP(const GPInT<S>& in, int seed, S c1, S c2, S out[9], S* Jz_v,
-                                         const float* jz = nullptr) {
-  using D = typename DualOf<S>::type;
-  D Z[3][3];
+// jz: J_z and its seed derivatives from jz_seeds.
+__device__ __forceinline__ void point_dP(const GPInT<float>& in, int seed, float c1, float c2, float out[9],
+                                         const float jz[10]) {
+  DualF Z[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) Z[i][j] = {in.Z[i][j], (i * 3 + j == seed) ? S(1) : S(0)};
-  const D p = {in.p, seed == 9 ? S(1) : S(0)};
-  D P[3][3], Jz;
-  if constexpr (std::is_same<S, float>::value) {
-    if (jz) {
-      const D jg = {jz[0], seed < 9 ? jz[1 + seed] : 0.0f};
-      point_P<D, S>(Z, in.A, in.Jx, in.w, p, c1, c2, P, Jz, &jg);
-    } else {
-      point_P<D, S>(Z, in.A, in.Jx, in.w, p, c1, c2, P, Jz);
-    }
-  } else {
-    point_P<D, S>(Z, in.A, in.Jx, in.w, p, c1, c2, P, Jz);
-  }
+    for (int j = 0; j < 3; ++j) Z[i][j] = {in.Z[i][j], (i * 3 + j == seed) ? 1.0f : 0.0f};
+  const DualF p = {in.p, seed == 9 ? 1.0f : 0.0f};
+  DualF P[3][3];
+  point_P(Z, in.A, in.Jx, in.w, p, c1, c2, P, DualF{jz[0], seed < 9 ? jz[1 + seed] : 0.0f});
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) out[i * 3 + j] = P[i][j].d;
-  if (Jz_v) *Jz_v = Jz.v;
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -1086,122 +902,37 @@ __global__ void sum_dc(const double* __restrict__ dc_elem, int32_t n_elem, int32
 // psi_ns.  Consistent tangent: D_g^(mh,nh)[xi][zeta] = dP[xi][mh]/dZ[nh][zeta] from the forward-mode
 // passes of point_dP, Hv = dP/dp, Pv = w J_z Z^-1.
 
-// Iron's per-Gauss-point tangent blocks in spatial coordinates (src/finite_elasticity_routines.F90:
-// 649-795 and 1072-1192): sub[0..2] = J_z w (c_sub + sigma) for the diagonal component blocks,
-// sub[3..5] = J_z w c_sub for the off-diagonal blocks (mh, nh) = (1,0), (2,0), (2,1);
-// hyd = J_z w push(C^-1).
-template <typename S>
-__device__ void iron_point_tensors(const GPT<S>& q, S c1, S c2, S sub[6][9], S hyd[9], S& jgw) {
-  const S J = q.Jz / q.Jx;
-  // unmodified right Cauchy-Green tensor and its inverse
-  S C[3][3], Ci[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[i][j] = q.F[0][i] * q.F[0][j] + q.F[1][i] * q.F[1][j] + q.F[2][i] * q.F[2][j];
-  const S I3 = inv3(C, Ci);
-  const S L[6] = {C[0][0], C[1][1], C[2][2], C[0][1], C[0][2], C[1][2]};
-  const S U[6] = {Ci[0][0], Ci[1][1], Ci[2][2], Ci[0][1], Ci[0][2], Ci[1][2]};
-  // I3EE as filled by Fortran RESHAPE (column j listed): I3EE[i][j] = col[j][i]
-  const S z0 = S(0), f4 = S(4), f2 = S(2);
-  const S col[6][6] = {{z0, f4 * L[2], f4 * L[1], z0, z0, -f4 * L[5]},
-                       {f4 * L[2], z0, f4 * L[0], z0, -f4 * L[4], z0},
-                       {f4 * L[1], f4 * L[0], z0, -f2 * L[3], z0, z0},
-                       {z0, z0, -f4 * L[3], -f2 * L[2], f2 * L[5], f2 * L[4]},
-                       {z0, -f4 * L[4], z0, f2 * L[5], -f2 * L[1], f2 * L[3]},
-                       {-f4 * L[5], z0, z0, f2 * L[4], f2 * L[3], -f2 * L[0]}};
-  S D[6][6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      S v = S(0);
-      if (i < 3 && j < 3 && i != j) v = f4 * c2;
-      if (i >= 3 && i == j) v = -f2 * c2;
-      D[i][j] = v + q.p * (-f2 * U[i] * U[j] + S(0.5) * col[j][i] / I3);
-    }
-  const S I1 = C[0][0] + C[1][1] + C[2][2];
-  const S t2 = f2 * (c1 + I1 * c2);
-  S Sv[6] = {-f2 * c2 * C[0][0] + t2, -f2 * c2 * C[1][1] + t2, -f2 * c2 * C[2][2] + t2,
-             -f2 * c2 * C[1][0], -f2 * c2 * C[2][0], -f2 * c2 * C[2][1]};
-  S H[6] = {U[0], U[1], U[2], U[3], U[4], U[5]};
-  S t[6][6];
-  push_t(q.F, t);
-  push_vec(t, Sv, J);
-  push_vec(t, H, J);
-  S tD[6][6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      S s = S(0);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) s += t[i][k] * D[k][j];
-      tD[i][j] = s;
-    }
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      S s = S(0);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) s += tD[i][k] * t[j][k];
-      D[i][j] = s / J;
-    }
-  Sv[0] += q.p; Sv[1] += q.p; Sv[2] += q.p;
-  jgw = q.Jz * q.w;
-#pragma unroll
-  for (int nh = 0; nh < 3; ++nh)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) sub[nh][i * 3 + j] = jgw * (D[t2v(i, nh)][t2v(j, nh)] + Sv[t2v(i, j)]);
-  const int om[3] = {1, 2, 2}, on[3] = {0, 0, 1};
-#pragma unroll
-  for (int o = 0; o < 3; ++o)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) sub[3 + o][i * 3 + j] = jgw * D[t2v(i, om[o])][t2v(j, on[o])];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) hyd[i * 3 + j] = jgw * H[t2v(i, j)];
-}
-
 constexpr int kGPElems = 4;                // elements per CTA of mr_gp_kernel
 constexpr uint32_t kTableWaitPolls = 1u << 24;  // bounded wait for the TMA copy of the tables
 constexpr int kGPThreads = kGPElems * NG;  // 108
 constexpr int kGPOut = 81 + 9 + 9;         // D (9 blocks x 9), Hv, Pv per Gauss point
 constexpr int kGPItem = (NG * kGPOut + 3) / 4 * 4;  // per-element stride: a 16-byte multiple (TMA)
 
-template <typename KS>
 struct GPShared {
-  KS x[kGPElems][81], z[kGPElems][81], p[kGPElems][8];
+  float x[kGPElems][81], z[kGPElems][81], p[kGPElems][8];
 };
 
-// One thread per (element, Gauss point).  out[item * kGPItem + g * kGPOut + j] in the contraction type TO:
-// D[(mh*3+nh)*9 + xi*3+zeta], Hv[81 + xi*3+mh], Pv[90 + xi*3+nh].  KS is the kinematics type:
-// double, or float on the FP32 paths (element data rounded once per node when staged, the volume
-// Jacobians det(Z), det(X) still evaluated in FP64 from the exactly widened gradients; for the
-// consistent tangent (EXACT) the forward-mode passes run in FP32 dual numbers, with J_z and its
-// derivative in FP64 dual arithmetic).
-template <typename TO, bool EXACT, typename KS = double>
+// One thread per (element, Gauss point).  out[item * kGPItem + g * kGPOut + j]:
+// D[(mh*3+nh)*9 + xi*3+zeta], Hv[81 + xi*3+mh], Pv[90 + xi*3+nh].  Element data rounded to FP32 once per
+// node when staged, the volume Jacobians det(Z), det(X) still evaluated in FP64 from the exactly widened
+// gradients; for the consistent tangent (EXACT) the forward-mode passes run in FP32 dual numbers, with
+// J_z and its derivatives formed in FP64 once a point (jz_seeds).
+template <bool EXACT>
 __global__ void __launch_bounds__(kGPThreads)
 mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __restrict__ eq2,
              const int32_t* __restrict__ elin, int32_t nq2, const double* __restrict__ xg,
-             const double* __restrict__ dep, const double* __restrict__ cpar, const TablesT<KS>* __restrict__ Tg,
-             TO* __restrict__ out, unsigned* err) {
+             const double* __restrict__ dep, const double* __restrict__ cpar, const TablesF* __restrict__ Tg,
+             float* __restrict__ out, unsigned* err) {
   extern __shared__ __align__(16) double smem_d[];
   unsigned char* sbase = reinterpret_cast<unsigned char*>(smem_d);
-  TablesT<KS>& T = *reinterpret_cast<TablesT<KS>*>(sbase);
-  GPShared<KS>& S = *reinterpret_cast<GPShared<KS>*>(sbase + sizeof(TablesT<KS>));
-  uint64_t* tbar = reinterpret_cast<uint64_t*>(sbase + sizeof(TablesT<KS>) + sizeof(GPShared<KS>));
+  TablesF& T = *reinterpret_cast<TablesF*>(sbase);
+  GPShared& S = *reinterpret_cast<GPShared*>(sbase + sizeof(TablesF));
+  uint64_t* tbar = reinterpret_cast<uint64_t*>(sbase + sizeof(TablesF) + sizeof(GPShared));
   // the basis tables arrive by one TMA bulk copy while the threads gather the element data
   if (threadIdx.x == 0) {
     tc::mbar_init(tbar, 1);
-    tc::mbar_arrive_expect_tx(tbar, (uint32_t)sizeof(TablesT<KS>));
-    tc::bulk_copy_g2s(&T, Tg, (uint32_t)sizeof(TablesT<KS>), tbar);
+    tc::mbar_arrive_expect_tx(tbar, (uint32_t)sizeof(TablesF));
+    tc::bulk_copy_g2s(&T, Tg, (uint32_t)sizeof(TablesF), tbar);
   }
   const int le = threadIdx.x / NG, g = threadIdx.x % NG;
   const int item = blockIdx.x * kGPElems + le;
@@ -1213,15 +944,15 @@ mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __
     const int n = __ldg(eq2 + (size_t)e * NQ + i);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      S.x[l][c * NQ + i] = (KS)__ldg(xg + (size_t)c * nq2 + n);
-      S.z[l][c * NQ + i] = (KS)dep[(size_t)c * nq2 + n];
+      S.x[l][c * NQ + i] = (float)__ldg(xg + (size_t)c * nq2 + n);
+      S.z[l][c * NQ + i] = (float)dep[(size_t)c * nq2 + n];
     }
   }
   for (int t = threadIdx.x; t < kGPElems * NL; t += blockDim.x) {
     const int l = t / NL, i = t % NL, it = blockIdx.x * kGPElems + l;
     if (it >= count) continue;
     const int e = __ldg(elems + it);
-    S.p[l][i] = (KS)dep[(size_t)3 * nq2 + __ldg(elin + (size_t)e * NL + i)];
+    S.p[l][i] = (float)dep[(size_t)3 * nq2 + __ldg(elin + (size_t)e * NL + i)];
   }
   __syncthreads();
   // every thread waits for the tables (so none exits while the copy is in flight); bounded
@@ -1231,12 +962,12 @@ mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __
     return;
   }
   if (item >= count) return;
-  TO* o = out + (size_t)item * kGPItem + (size_t)g * kGPOut;
+  float* o = out + (size_t)item * kGPItem + (size_t)g * kGPOut;
   if constexpr (!EXACT) {
-    const KS c1 = (KS)cpar[0], c2 = (KS)cpar[1];
-    GPT<KS> q;
+    const float c1 = (float)cpar[0], c2 = (float)cpar[1];
+    GPT<float> q;
     if (!gauss_point(T, g, S.z[le], S.x[le], S.p[le], q)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
-    KS sub[6][9], hyd[9], jgw;
+    float sub[6][9], hyd[9], jgw;
     iron_point_tensors(q, c1, c2, sub, hyd, jgw);
     // blocks to xi space: Dxi = Zi sub Zi^T (Zi = dxi/dz); upper blocks as transposes of the lower
 #pragma unroll
@@ -1246,12 +977,12 @@ mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __
         const int blk = mh == nh ? mh : (mh > nh ? 3 + (mh == 1 ? 0 : (nh == 0 ? 1 : 2))
                                                  : 3 + (nh == 1 ? 0 : (mh == 0 ? 1 : 2)));
         const bool tr = mh < nh;
-        KS W[3][3];
+        float W[3][3];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
           for (int z = 0; z < 3; ++z) {
-            KS s = KS(0);
+            float s = float(0);
 #pragma unroll
             for (int j = 0; j < 3; ++j) s += (tr ? sub[blk][j * 3 + i] : sub[blk][i * 3 + j]) * q.Zi[z][j];
             W[i][z] = s;  // (sub Zi^T)[i][zeta]
@@ -1261,41 +992,41 @@ mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __
 #pragma unroll
           for (int z = 0; z < 3; ++z)
             o[(mh * 3 + nh) * 9 + xi * 3 + z] =
-                (TO)(q.Zi[xi][0] * W[0][z] + q.Zi[xi][1] * W[1][z] + q.Zi[xi][2] * W[2][z]);
+                (float)(q.Zi[xi][0] * W[0][z] + q.Zi[xi][1] * W[1][z] + q.Zi[xi][2] * W[2][z]);
       }
 #pragma unroll
     for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
-        o[81 + xi * 3 + m] = (TO)(q.Zi[xi][0] * hyd[m * 3 + 0] + q.Zi[xi][1] * hyd[m * 3 + 1] +
+        o[81 + xi * 3 + m] = (float)(q.Zi[xi][0] * hyd[m * 3 + 0] + q.Zi[xi][1] * hyd[m * 3 + 1] +
                                   q.Zi[xi][2] * hyd[m * 3 + 2]);
-        o[90 + xi * 3 + m] = (TO)(jgw * q.Zi[xi][m]);
+        o[90 + xi * 3 + m] = (float)(jgw * q.Zi[xi][m]);
       }
   } else {
-    const KS c1 = (KS)cpar[0], c2 = (KS)cpar[1];
-    GPInT<KS> in;
+    const float c1 = (float)cpar[0], c2 = (float)cpar[1];
+    GPInT<float> in;
     gauss_inputs(T, g, S.z[le], S.x[le], S.p[le], in);
     float jz[10];
-    if constexpr (std::is_same<KS, float>::value) jz_seeds(in.Z, jz);
+    jz_seeds(in.Z, jz);
     for (int seed = 0; seed < 10; ++seed) {
-      KS d[9], Jz;
-      point_dP(in, seed, c1, c2, d, &Jz, std::is_same<KS, float>::value ? jz : nullptr);
+      float d[9];
+      point_dP(in, seed, c1, c2, d, jz);
       if (seed < 9) {
         const int nh = seed / 3, z = seed % 3;
 #pragma unroll
         for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
-          for (int mh = 0; mh < 3; ++mh) o[(mh * 3 + nh) * 9 + xi * 3 + z] = (TO)d[xi * 3 + mh];
+          for (int mh = 0; mh < 3; ++mh) o[(mh * 3 + nh) * 9 + xi * 3 + z] = (float)d[xi * 3 + mh];
       } else {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) o[81 + k] = (TO)d[k];
-        KS Zi[3][3];
-        const KS dz = inv3(in.Z, Zi);
-        if (!(dz > KS(0)) || !isfinite(dz)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
+        for (int k = 0; k < 9; ++k) o[81 + k] = (float)d[k];
+        float Zi[3][3];
+        const float dz = inv3(in.Z, Zi);
+        if (!(dz > float(0)) || !isfinite(dz)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
 #pragma unroll
         for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
-          for (int nh = 0; nh < 3; ++nh) o[90 + xi * 3 + nh] = (TO)(in.w * Jz * Zi[xi][nh]);
+          for (int nh = 0; nh < 3; ++nh) o[90 + xi * 3 + nh] = (float)(in.w * jz[0] * Zi[xi][nh]);
       }
     }
   }
@@ -1376,73 +1107,66 @@ constexpr int kCTileRows = kCRows / 4;        // 32 row groups of 4
 constexpr int kCTileCols = 7;                 // 7 column groups of 4 (27 columns, padded to 28)
 
 // The arrays read with vector loads (A, G) come first: their rows are multiples of 16 bytes.
-template <typename TS>
 struct ContractShared {
-  TS A[81][kCRows];     // A[(g,zeta)][row] of the current pass
-  TS G[81][28];         // G[(g,xi)][ms]; column 27 zero
-  TS C[2 * kCRows][28]; // C[(mh,nh,ms)][ns]
-  TS HvG[NG][81];       // sum_xi G[(g,xi)][ms] Hv[xi][mh]  -> [g][(mh,ms)]
-  TS PvG[NG][81];       // sum_xi G[(g,xi)][ns] Pv[xi][nh]  -> [g][(nh,ns)]
-  TS Dg[NG][kGPOut];    // this element's Gauss-point blocks
-  TS psi[NG][NL];       // pressure basis at the Gauss points
+  float A[81][kCRows];     // A[(g,zeta)][row] of the current pass
+  float G[81][28];         // G[(g,xi)][ms]; column 27 zero
+  float C[2 * kCRows][28]; // C[(mh,nh,ms)][ns]
+  float HvG[NG][81];       // sum_xi G[(g,xi)][ms] Hv[xi][mh]  -> [g][(mh,ms)]
+  float PvG[NG][81];       // sum_xi G[(g,xi)][ns] Pv[xi][nh]  -> [g][(nh,ns)]
+  float Dg[NG][kGPOut];    // this element's Gauss-point blocks
+  float psi[NG][NL];       // pressure basis at the Gauss points
 };
 static_assert(sizeof(float) * kCRows % 16 == 0 && sizeof(float) * 28 % 16 == 0, "vector rows");
 static_assert(sizeof(float) * 81 * kCRows % 16 == 0, "G follows A on a 16-byte boundary");
 
-template <typename TS>
-__device__ __forceinline__ void load4(const TS* p, TS (&v)[4]) {
-  if constexpr (std::is_same<TS, float>::value) {
-    const float4 q = *reinterpret_cast<const float4*>(p);
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-  } else {
-    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
 
 // Element matrices of `count` elements into Kel[e][89][89] (element number e = elems[item]).
-template <typename TS, bool EXACT>
+template <bool EXACT>
 __global__ void __launch_bounds__(kCThreads)
 mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Tables* __restrict__ Tg,
-                   const TS* __restrict__ gp, TS* __restrict__ Kel) {
+                   const float* __restrict__ gp, float* __restrict__ Kel) {
   extern __shared__ __align__(16) unsigned char craw[];
-  ContractShared<TS>& S = *reinterpret_cast<ContractShared<TS>*>(craw);
+  ContractShared& S = *reinterpret_cast<ContractShared*>(craw);
   const int tid = threadIdx.x;
   for (int t = tid; t < 81 * 28; t += blockDim.x) {
     const int k = t / 28, ms = t % 28;
-    S.G[k][ms] = ms < 27 ? (TS)Tg->dphi[k / 3][k % 3][ms] : TS(0);
+    S.G[k][ms] = ms < 27 ? (float)Tg->dphi[k / 3][k % 3][ms] : 0.0f;
   }
-  for (int t = tid; t < NG * NL; t += blockDim.x) S.psi[t / NL][t % NL] = (TS)Tg->psi[t / NL][t % NL];
+  for (int t = tid; t < NG * NL; t += blockDim.x) S.psi[t / NL][t % NL] = (float)Tg->psi[t / NL][t % NL];
   const int rq = tid / kCTileCols, cq = tid % kCTileCols;  // product tile of this thread
   const bool in_product = tid < kCTileRows * kCTileCols;
   for (int item = blockIdx.x; item < count; item += gridDim.x) {
     __syncthreads();
-    const TS* src = gp + (size_t)item * kGPItem;
+    const float* src = gp + (size_t)item * kGPItem;
     for (int t = tid; t < NG * kGPOut; t += blockDim.x) (&S.Dg[0][0])[t] = src[t];
     __syncthreads();
-    form_up_coefficients<TS, 28>(S.G, S.Dg, S.HvG, S.PvG);
+    form_up_coefficients<float, 28>(S.G, S.Dg, S.HvG, S.PvG);
     for (int pass = 0; pass < 2; ++pass) {
       // operand rows [pass * kCRows, pass * kCRows + kCRows); rows past 242 are zero
       for (int t = tid; t < 81 * kCRows; t += blockDim.x) {
         const int k = t / kCRows, rl = t % kCRows, row = pass * kCRows + rl;
-        TS v = TS(0);
+        float v = 0.0f;
         if (row < 243) {
           const int pair = row / 27, ms = row % 27, g = k / 3, zeta = k % 3;
-          const TS* D = &S.Dg[g][pair * 9 + zeta];
+          const float* D = &S.Dg[g][pair * 9 + zeta];
           v = S.G[g * 3 + 0][ms] * D[0] + S.G[g * 3 + 1][ms] * D[3] + S.G[g * 3 + 2][ms] * D[6];
         }
         S.A[k][rl] = v;
       }
       __syncthreads();
       if (in_product) {
-        TS acc[4][4];
+        float acc[4][4];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = TS(0);
+          for (int b = 0; b < 4; ++b) acc[a][b] = 0.0f;
 #pragma unroll 3
         for (int k = 0; k < 81; ++k) {
-          TS av[4], bv[4];
+          float av[4], bv[4];
           load4(&S.A[k][rq * 4], av);
           load4(&S.G[k][cq * 4], bv);
 #pragma unroll
@@ -1457,9 +1181,9 @@ mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Table
       }
       __syncthreads();  // A is rewritten by the next pass
     }
-    TS* Ke = Kel + (size_t)__ldg(elems + item) * ND * ND;
-    write_up_blocks<TS, TS>(Ke, S.HvG, S.PvG, S.psi);
-    write_uu_block<EXACT, TS, TS, 28>(Ke, S.C);
+    float* Ke = Kel + (size_t)__ldg(elems + item) * ND * ND;
+    write_up_blocks<float, float>(Ke, S.HvG, S.PvG, S.psi);
+    write_uu_block<EXACT, float, float, 28>(Ke, S.C);
   }
 }
 
@@ -1765,27 +1489,41 @@ int gather_rows(int32_t n_elem, const int32_t* elems, const int32_t* eq2, const 
   return GFE_OK;
 }
 
-template <typename TS>
-int jacobian_impl(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2, int32_t nlin,
-                  const double* xg, const int32_t* elems, const double* dep, const double* cpar,
-                  const int32_t* slots, const int32_t* row_ptr, double* values, double* K_out, cudaStream_t s,
-                  const char* fn, int tc_mode = 0) {
+// FP64: mr_jac64.cu forms the element matrices, straight into K_out when it is given.
+int jacobian_f64(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2, int32_t nlin,
+                 const double* xg, const int32_t* elems, const double* dep, const double* cpar, const int32_t* slots,
+                 const int32_t* row_ptr, double* values, double* K_out, cudaStream_t s, const char* fn) {
+  if (n_elem == 0) return GFE_OK;
+  int rc;
+  double* Kel = K_out;
+  if (!K_out && (rc = gfe::scratch_alloc((void**)&Kel, sizeof(double) * (size_t)n_elem * ND * ND, s, "element matrices")))
+    return rc;
+  unsigned* err = gfe::device_error_word();
+  void* prof = gfe::stage_begin(GFE_STAGE_MR_JACOBIAN, s);
+  int launches = 0;
+  rc = mr64::element_matrices(mode != 0, n_elem, elems, eq2, elin, nq2, xg, dep, cpar, Kel, s, err, &launches);
+  if (!rc && values) rc = gather_rows<double>(n_elem, elems, eq2, elin, nq2, nlin, Kel, slots, row_ptr, values, s, err);
+  gfe::stage_end(GFE_STAGE_MR_JACOBIAN, prof, s, launches + (values ? 3 : 0));
+  if (!K_out) gfe::scratch_free(Kel, s);
+  if (rc) return rc;
+  GFE_LAUNCH_CHECK(fn);
+  return GFE_OK;
+}
+
+// FP32 kinematics and contraction (tc_mode 0: CUDA cores, else the tensor cores).
+int jacobian_f32(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2, int32_t nlin,
+                 const double* xg, const int32_t* elems, const double* dep, const double* cpar, const int32_t* slots,
+                 const int32_t* row_ptr, double* values, double* K_out, cudaStream_t s, const char* fn, int tc_mode) {
   const Tables* T = nullptr;
   int rc = device_tables(&T);
   if (rc) return rc;
-  // Iron's analytic tangent on the FP32 paths: FP32 kinematics from the FP32 tables
-  using KF = typename std::conditional<std::is_same<TS, float>::value, float, double>::type;
-  const TablesT<KF>* TK = nullptr;
-  if constexpr (std::is_same<KF, float>::value) {
-    if ((rc = device_tables_f(&TK))) return rc;
-  } else {
-    TK = T;
-  }
+  const TablesF* TK = nullptr;
+  if ((rc = device_tables_f(&TK))) return rc;
   if (n_elem == 0) return GFE_OK;
-  const size_t gsm_k = sizeof(TablesT<KF>) + sizeof(GPShared<KF>) + 16;  // + the tables' mbarrier
-  const size_t csm = sizeof(ContractShared<TS>);
-  const void* gk = mode == 0 ? (const void*)mr_gp_kernel<TS, false, KF> : (const void*)mr_gp_kernel<TS, true, KF>;
-  const void* ck = mode == 0 ? (const void*)mr_contract_kernel<TS, false> : (const void*)mr_contract_kernel<TS, true>;
+  const size_t gsm_k = sizeof(TablesF) + sizeof(GPShared) + 16;  // + the tables' mbarrier
+  const size_t csm = sizeof(ContractShared);
+  const void* gk = mode == 0 ? (const void*)mr_gp_kernel<false> : (const void*)mr_gp_kernel<true>;
+  const void* ck = mode == 0 ? (const void*)mr_contract_kernel<false> : (const void*)mr_contract_kernel<true>;
   if ((rc = set_smem(gk, gsm_k)) || (rc = set_smem(ck, csm))) return rc;
   if (tc_mode) {
     const void* tk[4] = {(const void*)mr_contract_tc_kernel<false, false>, (const void*)mr_contract_tc_kernel<false, true>,
@@ -1794,20 +1532,12 @@ int jacobian_impl(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* e
       if ((rc = set_smem(k, sizeof(TCShared)))) return rc;
   }
   const int chunk = std::min(n_elem, kElemChunk);
-  // element matrices: straight into K_out when it has the contraction's type
-  constexpr bool kDirect = std::is_same<TS, double>::value;
-  TS* Kel = nullptr;
-  bool own_kel = true;
-  if (kDirect && K_out) {
-    Kel = reinterpret_cast<TS*>(K_out);
-    own_kel = false;
-  } else if ((rc = gfe::scratch_alloc((void**)&Kel, sizeof(TS) * (size_t)n_elem * ND * ND, s, "element matrices"))) {
-    return rc;
-  }
-  TS* gpbuf = nullptr;
-  if ((rc = gfe::scratch_alloc((void**)&gpbuf, sizeof(TS) * (size_t)chunk * kGPItem + 16, s,
+  float* Kel = nullptr;
+  if ((rc = gfe::scratch_alloc((void**)&Kel, sizeof(float) * (size_t)n_elem * ND * ND, s, "element matrices"))) return rc;
+  float* gpbuf = nullptr;
+  if ((rc = gfe::scratch_alloc((void**)&gpbuf, sizeof(float) * (size_t)chunk * kGPItem + 16, s,
                                "Gauss-point tangent blocks"))) {
-    if (own_kel) gfe::scratch_free(Kel, s);
+    gfe::scratch_free(Kel, s);
     return rc;
   }
   unsigned* err = gfe::device_error_word();
@@ -1818,44 +1548,39 @@ int jacobian_impl(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* e
     const int cnt = std::min(chunk, n_elem - c0);
     const int ggrid = (cnt + kGPElems - 1) / kGPElems;
     if (mode == 0)
-      mr_gp_kernel<TS, false, KF><<<ggrid, kGPThreads, gsm_k, s>>>(elems + c0, cnt, eq2, elin, nq2, xg, dep, cpar, TK,
-                                                                   gpbuf, err);
+      mr_gp_kernel<false><<<ggrid, kGPThreads, gsm_k, s>>>(elems + c0, cnt, eq2, elin, nq2, xg, dep, cpar, TK, gpbuf, err);
     else
-      mr_gp_kernel<TS, true, KF><<<ggrid, kGPThreads, gsm_k, s>>>(elems + c0, cnt, eq2, elin, nq2, xg, dep, cpar, TK,
-                                                                  gpbuf, err);
-    if constexpr (std::is_same<TS, float>::value) {
-      if (tc_mode) {
-        const int tgrid = std::min(cnt, sms);
-        if (mode == 0) {
-          if (tc_mode == GFE_TC_TF32X3) launch_contract_tc<false, true>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
-          else launch_contract_tc<false, false>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
-        } else {
-          if (tc_mode == GFE_TC_TF32X3) launch_contract_tc<true, true>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
-          else launch_contract_tc<true, false>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
-        }
-        launches += 2;
-        continue;
+      mr_gp_kernel<true><<<ggrid, kGPThreads, gsm_k, s>>>(elems + c0, cnt, eq2, elin, nq2, xg, dep, cpar, TK, gpbuf, err);
+    launches += 2;
+    if (tc_mode) {
+      const int tgrid = std::min(cnt, sms);
+      if (mode == 0) {
+        if (tc_mode == GFE_TC_TF32X3) launch_contract_tc<false, true>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
+        else launch_contract_tc<false, false>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
+      } else {
+        if (tc_mode == GFE_TC_TF32X3) launch_contract_tc<true, true>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
+        else launch_contract_tc<true, false>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
       }
+      continue;
     }
     const int cgrid = std::min(cnt, 8 * sms);
     if (mode == 0)
-      mr_contract_kernel<TS, false><<<cgrid, kCThreads, csm, s>>>(elems + c0, cnt, T, gpbuf, Kel);
+      mr_contract_kernel<false><<<cgrid, kCThreads, csm, s>>>(elems + c0, cnt, T, gpbuf, Kel);
     else
-      mr_contract_kernel<TS, true><<<cgrid, kCThreads, csm, s>>>(elems + c0, cnt, T, gpbuf, Kel);
-    launches += 2;
+      mr_contract_kernel<true><<<cgrid, kCThreads, csm, s>>>(elems + c0, cnt, T, gpbuf, Kel);
   }
   gfe::scratch_free(gpbuf, s);
-  if (values && (rc = gather_rows<TS>(n_elem, elems, eq2, elin, nq2, nlin, Kel, slots, row_ptr, values, s, err))) {
-    if (own_kel) gfe::scratch_free(Kel, s);
+  if (values && (rc = gather_rows<float>(n_elem, elems, eq2, elin, nq2, nlin, Kel, slots, row_ptr, values, s, err))) {
+    gfe::scratch_free(Kel, s);
     return rc;
   }
-  if (K_out && own_kel) {
+  if (K_out) {
     const size_t n = (size_t)n_elem * ND * ND;
-    widen_element_matrices<TS><<<8 * sms, 256, 0, s>>>(Kel, n, K_out);
+    widen_element_matrices<<<8 * sms, 256, 0, s>>>(Kel, n, K_out);
     ++launches;
   }
   gfe::stage_end(GFE_STAGE_MR_JACOBIAN, prof, s, launches + (values ? 3 : 0));
-  if (own_kel) gfe::scratch_free(Kel, s);
+  gfe::scratch_free(Kel, s);
   GFE_LAUNCH_CHECK(fn);
   return GFE_OK;
 }
@@ -1878,10 +1603,10 @@ int jacobian_entry_point(int mode, int32_t n_elem, const int32_t* eq2, const int
     return gfe::set_error(GFE_ERR_ARG, "%s: precision must be GFE_FP64, GFE_MIXED, GFE_TC_TF32X3 or GFE_TC_TF32", fn);
   cudaStream_t s = gfe::as_stream(stream);
   if (precision == GFE_FP64)
-    return jacobian_impl<double>(mode, n_elem, eq2, elin, nq2, nlin, xg, color_elems, dep, cpar, slots, row_ptr,
-                                 values, K_out, s, fn);
-  return jacobian_impl<float>(mode, n_elem, eq2, elin, nq2, nlin, xg, color_elems, dep, cpar, slots, row_ptr, values,
-                              K_out, s, fn, precision == GFE_MIXED ? 0 : precision);
+    return jacobian_f64(mode, n_elem, eq2, elin, nq2, nlin, xg, color_elems, dep, cpar, slots, row_ptr, values, K_out, s,
+                        fn);
+  return jacobian_f32(mode, n_elem, eq2, elin, nq2, nlin, xg, color_elems, dep, cpar, slots, row_ptr, values, K_out, s,
+                      fn, precision == GFE_MIXED ? 0 : precision);
 }
 
 }  // namespace

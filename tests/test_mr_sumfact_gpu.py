@@ -3,7 +3,10 @@
 The finite-difference Jacobian splits an element over 1, 3 or 9 CTAs by the number of elements and
 adds the columns all at once through element matrices (up to 4,096 elements) or colour by colour;
 every branch is compared with the oracle's element matrices on sampled elements, and the assembled
-values with the sum of the dense element matrices.  Tolerances: the difference quotient amplifies the
+values with the sum of the dense element matrices.  The FP64 tangent takes eight elements a CTA and the
+contraction two CTAs an SM; it is compared with automatic differentiation of the element residual
+written in plain torch, at element counts around those edges.  Tolerances: FP64 on both sides, summed in
+different orders, 1e-12 x max|K| as in test_mr_gpu; the difference quotient amplifies the
 rounding of two FP64 residuals by 1 / delta (1e-9 x max|K|, as in test_mr_fd_jacobian_gpu); sums of at
 most 8 FP64 element entries in another order agree to 8 eps max|K|.
 """
@@ -44,5 +47,53 @@ def test_fd_jacobian_size_rules(gfe_cuda, ne):
         Ko = oracle.mr_element_jacobian_fd(*_element(A, dep, e), C1, C2, delta)
         assert np.abs(K[e].cpu().numpy() - Ko).max() <= 1e-9 * np.abs(Ko).max(), e
     v = A.jacobian_fd(d, [C1, C2])
+    ref = torch.zeros_like(v).index_add_(0, A.slots.reshape(-1).long(), K.reshape(-1))
+    assert float((v - ref).abs().max()) <= 8 * EPS * float(K.abs().max())
+
+
+def _point_tables():
+    """Basis gradients [27, 3, 27], pressure functions [27, 8] and weights [27], xi1 fastest."""
+    x, w = np.polynomial.legendre.leggauss(3)
+    x, w = (x + 1) / 2, w / 2
+    V = np.stack([2 * (x - 0.5) * (x - 1), 4 * x * (1 - x), 2 * x * (x - 0.5)], axis=1)
+    D = np.stack([4 * x - 3, 4 - 8 * x, 4 * x - 1], axis=1)
+    L = np.stack([1 - x, x], axis=1)
+    kron = lambda a, b, c: np.einsum("gi,hj,kl->khglji", a, b, c).reshape(27, -1)  # noqa: E731
+    G = np.stack([kron(D, V, V), kron(V, D, V), kron(V, V, D)], axis=1)
+    return torch.from_numpy(G), torch.from_numpy(kron(L, L, L)), torch.from_numpy(np.einsum("g,h,k->khg", w, w, w).ravel())
+
+
+def _torch_residual(u, xe):
+    G, psi, w = _point_tables()
+    Z = torch.einsum("cn,gkn->gck", u[:81].reshape(3, 27), G)
+    X = torch.einsum("cn,gkn->gck", xe, G)
+    Jz, Jx = torch.linalg.det(Z).abs(), torch.linalg.det(X).abs()
+    N = X / X.norm(dim=1, keepdim=True)
+    F = Z @ torch.linalg.inv(N.transpose(1, 2) @ X)
+    J = Jz / Jx
+    Fb = F * J[:, None, None] ** (-1.0 / 3.0)
+    C = Fb.transpose(1, 2) @ Fb
+    eye = torch.eye(3, dtype=torch.float64)
+    I1 = C.diagonal(dim1=1, dim2=2).sum(1)
+    S = -2 * C2 * C + 2 * (C1 + I1 * C2)[:, None, None] * eye
+    sg = Fb @ S @ Fb.transpose(1, 2) / J[:, None, None]
+    p = psi @ u[81:]
+    sg = sg + (p - sg.diagonal(dim1=1, dim2=2).sum(1) / 3)[:, None, None] * eye
+    P = (w * Jz)[:, None, None] * (torch.linalg.inv(Z) @ sg)
+    return torch.cat([torch.einsum("gkm,gkn->mn", P, G).reshape(-1), (w * (Jz - Jx)) @ psi])
+
+
+@pytest.mark.parametrize("ne", [(1, 1, 1), (7, 1, 1), (2, 2, 2), (3, 3, 1), (7, 8, 6)])
+def test_tangent_fp64_element_counts(gfe_cuda, ne):
+    A = MooneyRivlinAssembly.from_regular_mesh(ne, extent=(1.0, 1.3, 0.8))
+    dep = _state(A, 5)
+    d = torch.from_numpy(dep).cuda()
+    K = A.element_tangents(d, [C1, C2], precision="fp64")
+    for e in sorted({0, A.n_elements // 2, A.n_elements - 1}):
+        xe, ze, pe = _element(A, dep, e)
+        u = torch.from_numpy(np.r_[ze.ravel(), pe])
+        Kt = torch.autograd.functional.jacobian(lambda v: _torch_residual(v, torch.from_numpy(xe)), u)
+        assert float((K[e].cpu() - Kt).abs().max()) <= 1e-12 * float(Kt.abs().max()), e
+    v = A.tangent(d, [C1, C2], precision="fp64")
     ref = torch.zeros_like(v).index_add_(0, A.slots.reshape(-1).long(), K.reshape(-1))
     assert float((v - ref).abs().max()) <= 8 * EPS * float(K.abs().max())
