@@ -1,9 +1,10 @@
-// mr.cu -- K4 / K5: Mooney-Rivlin (mixed u-p, triquadratic u + trilinear p) residual and Iron's
-// analytic Jacobian, batched over elements (and over parameter sets for the residual).
+// mr.cu -- K5: Mooney-Rivlin (mixed u-p, triquadratic u + trilinear p) Jacobians: FP32 Gauss-point and
+// contraction kernels (CUDA cores and tcgen05), the slot map, the row-owning assembly and the entry
+// points.  FP64 element matrices are formed by mr_jac64.cu, the residual and its adjoint by
+// mr_residual.cu, Iron's finite-difference Jacobian by mr_fd.cu.
 //
-// Reference: FiniteElasticity_FiniteElementResidualEvaluate, MOONEY_RIVLIN_SUBTYPE branch
-// (src/finite_elasticity_routines.F90:1669-1756), FINITE_ELASTICITY_GAUSS_STRESS_TENSOR (:6985-7061),
-// FiniteElasticity_GaussDeformationGradientTensor (:5148-5215) with the material frame of
+// Reference: FiniteElasticity_GaussDeformationGradientTensor
+// (src/finite_elasticity_routines.F90:5148-5215) with the material frame of
 // Coordinates_MaterialSystemCalculate (src/coordinate_routines.F90:3841-3947),
 // FiniteElasticity_FiniteElementJacobianEvaluate (:1016-1274) and
 // FINITE_ELASTICITY_GAUSS_ELASTICITY_TENSOR (:649-795).
@@ -12,17 +13,6 @@
 // positions z1, z2, z3 over the n_q2 quadratic nodes followed by the pressure over the n_lin
 // linear (corner) nodes; the geometric field x is [3][n_q2].  Element DOF order: 27 z1, 27 z2,
 // 27 z3, 8 p (Iron's element parameter order, local nodes xi1 fastest).
-//
-// Residual: one warp per (element, parameter set).  Lane g < 27 evaluates Gauss point g (metrics,
-// deformation gradient, stress) and leaves P_g = J_z w_g Z^-1 sigma (3x3) and
-// J_x w_g (J_z/J_x - 1) in shared memory; the lanes then form the 89 entries as sums over Gauss
-// points in a fixed order (deterministic) and scatter them into the global residual.  Elements
-// are processed colour by colour, so no two elements of a launch share a DOF.
-//
-// Jacobian: one CTA per element.  Threads 0..26 build, per Gauss point, the spatial basis
-// gradients dphi/dz and the 3x3 blocks J_z w (c + sigma) of Iron's analytic tangent; all threads
-// then form the lower u-u triangle and the u-p / p-u blocks and add them into the CSR values
-// through a precomputed per-element slot map (u-u upper triangle mirrored, p-p structurally zero).
 #include <mutex>
 #include <type_traits>
 
@@ -147,128 +137,6 @@ __device__ __forceinline__ bool gauss_point(const TablesT<S>& T, int g, const S*
   o.p = p;
   o.w = T.w[g];
   return dz > S(0) && o.Jx > S(0) && isfinite(dz);
-}
-
-// Cauchy stress of the residual (deviatoric MR + p), src/finite_elasticity_routines.F90:6985-7061.
-__device__ __forceinline__ void residual_stress(const GP& q, double c1, double c2, double sig[6]) {
-  const double J = q.Jz / q.Jx;
-  const double s = pow(J, -1.0 / 3.0);
-  double Fb[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Fb[i][j] = q.F[i][j] * s;
-  double C[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[i][j] = Fb[0][i] * Fb[0][j] + Fb[1][i] * Fb[1][j] + Fb[2][i] * Fb[2][j];
-  const double I1 = C[0][0] + C[1][1] + C[2][2];
-  const double t1 = -2.0 * c2, t2 = 2.0 * (c1 + I1 * c2);
-  sig[0] = t1 * C[0][0] + t2; sig[1] = t1 * C[1][1] + t2; sig[2] = t1 * C[2][2] + t2;
-  sig[3] = t1 * C[1][0]; sig[4] = t1 * C[2][0]; sig[5] = t1 * C[2][1];
-  double t[6][6];
-  push_t(Fb, t);
-  push_vec(t, sig, J);
-  const double tr3 = (sig[0] + sig[1] + sig[2]) / 3.0;
-  sig[0] = sig[0] - tr3 + q.p; sig[1] = sig[1] - tr3 + q.p; sig[2] = sig[2] - tr3 + q.p;
-}
-
-// ----------------------------------------------------------------------------------------------
-// residual
-// ----------------------------------------------------------------------------------------------
-constexpr int kResWarps = 4;
-
-// One warp: the 89 residual entries of one element from its staged geometry sx[81], deformed
-// positions sz[81] and pressures sp[8] (shared memory), with Gauss-point scratch sP[27*9] and
-// stp[27].  Lane g < 27 evaluates Gauss point g (metrics, deformation gradient, stress) and leaves
-// P_g = J_z w_g Z^-1 sigma (3x3) and J_x w_g (J_z/J_x - 1); then lane i forms entries i, i + 32,
-// i + 64 as sums over the Gauss points in a fixed order and hands each to emit(i, value).
-template <typename Emit>
-__device__ __forceinline__ void warp_element_residual(const Tables& T, int lane, const double* sx, const double* sz,
-                                                      const double* sp, double c1, double c2, double* sP, double* stp,
-                                                      unsigned* err, Emit emit) {
-  if (lane < NG) {
-    GP q;
-    if (!gauss_point(T, lane, sz, sx, sp, q)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
-    double sig[6];
-    residual_stress(q, c1, c2, sig);
-    const double jgw = q.Jz * q.w;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int mh = 0; mh < 3; ++mh)
-        sP[lane * 9 + k * 3 + mh] = jgw * (q.Zi[k][0] * sig[t2v(0, mh)] + q.Zi[k][1] * sig[t2v(1, mh)] +
-                                           q.Zi[k][2] * sig[t2v(2, mh)]);
-    stp[lane] = q.Jx * q.w * (q.Jz / q.Jx - 1.0);
-  }
-  __syncwarp();
-  for (int i = lane; i < ND; i += 32) {
-    double s = 0.0;
-    if (i < 81) {
-      const int ms = i % NQ, mh = i / NQ;
-      for (int g = 0; g < NG; ++g)
-        s += T.dphi[g][0][ms] * sP[g * 9 + 0 + mh] + T.dphi[g][1][ms] * sP[g * 9 + 3 + mh] +
-             T.dphi[g][2][ms] * sP[g * 9 + 6 + mh];
-    } else {
-      const int ms = i - 81;
-      for (int g = 0; g < NG; ++g) s += stp[g] * T.psi[g][ms];
-    }
-    emit(i, s);
-  }
-  __syncwarp();
-}
-
-__global__ void __launch_bounds__(kResWarps * 32)
-mr_residual_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t batch, const int32_t* __restrict__ eq2,
-                   const int32_t* __restrict__ elin, int32_t nq2, int32_t nlin, const double* __restrict__ xg,
-                   const double* __restrict__ dep, const double* __restrict__ cpar, const Tables* __restrict__ Tg,
-                   double* __restrict__ R, int64_t dep_stride, unsigned* err) {
-  extern __shared__ double smem[];
-  Tables& T = *reinterpret_cast<Tables*>(smem);
-  double* wbase = smem + sizeof(Tables) / sizeof(double);
-  // stage the tables
-  {
-    const double* src = reinterpret_cast<const double*>(Tg);
-    double* dst = smem;
-    for (int i = threadIdx.x; i < (int)(sizeof(Tables) / sizeof(double)); i += blockDim.x) dst[i] = src[i];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // per-warp scratch: x[81], z[81], p[8], P[27][9], tp[27], dofs (int) [89]
-  double* sx = wbase + w * (81 + 81 + 8 + NG * 9 + NG + 48);
-  double* sz = sx + 81;
-  double* sp = sz + 81;
-  double* sP = sp + 8;
-  double* stp = sP + NG * 9;
-  int* sd = reinterpret_cast<int*>(stp + NG);
-  const long long total = (long long)count * batch;
-  for (long long item = (long long)blockIdx.x * kResWarps + w; item < total; item += (long long)gridDim.x * kResWarps) {
-    const int b = (int)(item / count);
-    const int e = __ldg(elems + (item % count));
-    const double* d = dep + b * dep_stride;
-    for (int i = lane; i < NQ; i += 32) {
-      const int n = __ldg(eq2 + (size_t)e * NQ + i);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        sx[c * NQ + i] = __ldg(xg + (size_t)c * nq2 + n);
-        sz[c * NQ + i] = d[(size_t)c * nq2 + n];
-        sd[c * NQ + i] = c * nq2 + n;
-      }
-    }
-    if (lane < NL) {
-      const int n = __ldg(elin + (size_t)e * NL + lane);
-      sp[lane] = d[(size_t)3 * nq2 + n];
-      sd[81 + lane] = 3 * nq2 + n;
-    }
-    const double c1 = cpar[2 * b], c2 = cpar[2 * b + 1];
-    __syncwarp();
-    double* Rb = R + b * dep_stride;
-    warp_element_residual(T, lane, sx, sz, sp, c1, c2, sP, stp, err, [&](int i, double s) {
-      if (!isfinite(s)) gfe_raise(err, GFE_DEVERR_NONFINITE);
-      Rb[sd[i]] += s;
-    });
-  }
 }
 
 // slot map: for each element and each (r, c), the 0-based CSR position of (dof_r, dof_c); -1 when
@@ -432,14 +300,13 @@ __global__ void widen_element_matrices(const float* __restrict__ src, size_t n, 
 }
 
 // ----------------------------------------------------------------------------------------------
-// Consistent tangent and adjoint of Iron's residual (forward-mode dual numbers per Gauss point)
+// Consistent tangent of Iron's residual in FP32 (forward-mode dual numbers per Gauss point)
 // ----------------------------------------------------------------------------------------------
 // Per Gauss point the u-rows of the residual are R(ms,mh) += sum_xi g_ms[xi] P[xi][mh] with
 // P = w J_z Z^-1 sigma(Z, p) (Z = dz/dxi, g = reference basis gradients) and the p-rows
 // R(ms) += w (J_z - J_x) psi_ms.  The exact derivatives dP/dZ (81 numbers) and dP/dp (9) are
 // obtained by 10 forward-mode passes through the same formulas with dual numbers; dJ_z/dZ =
-// J_z Z^-T.  The element tangent / vector-Jacobian products are then contractions with the
-// constant basis tables.  This is the derivative that Iron's finite-difference Jacobian
+// J_z Z^-T.  The element tangent is then a contraction with the constant basis tables.  This is the derivative that Iron's finite-difference Jacobian
 // (src/equations_set_routines.F90:2839-2962) approximates.
 template <typename T>
 __device__ __forceinline__ T tdet3(const T A[3][3]) {
@@ -530,8 +397,6 @@ template <typename S>
 struct GPInT {
   S Z[3][3], A[3][3], Jx, w, p;
 };
-using GPIn = GPInT<double>;
-
 template <typename S>
 __device__ __forceinline__ void gauss_inputs(const TablesT<S>& T, int g, const S* sz, const S* sx, const S* sp,
                                              GPInT<S>& o) {
@@ -617,283 +482,17 @@ __device__ __forceinline__ void point_dP(const GPInT<float>& in, int seed, float
 }
 
 // ----------------------------------------------------------------------------------------------
-// Reverse-mode adjoint of the residual (one reverse sweep per Gauss point)
-// ----------------------------------------------------------------------------------------------
-// For a cotangent v of the element residual, the u-rows give the cotangent of P_g,
-// V_g[xi][mh] = sum_ms v(mh, ms) g_ms[xi], and the p-rows that of w (J_z - J_x), Vp_g = sum_ms
-// v_p(ms) psi_ms.  One reverse sweep through the formulas of point_P, in the opposite order,
-// yields Zbar = dL/dZ (3x3), pbar = dL/dp and the material cotangents (c1bar, c2bar) at the cost
-// of a few forward evaluations, instead of the 10 forward-mode passes of the tangent.  The
-// element's du is then sum_g Zbar_g[c][k] g_ms[k] (u) and sum_g pbar_g psi_ms (p).
-//   Q = Z^-1 sgd,  P = w J_z Q                      Qbar = w J_z V,  Jzbar += w V:Q
-//   sgd = sg - tr(sg)/3 I + p I                    sgbar = dev(sgdbar), pbar = tr(sgdbar)
-//   sg = Fb S Fb^T / J                             Hbar = sgbar / J, FSbar = Hbar Fb, Fbbar = Hbar^T FS
-//   S = t1 C + t2 I, C = Fb^T Fb, t1 = -2 c2, t2 = 2 (I1 c2 + c1), I1 = tr C
-//   Fb = s Z A, s = J^(-1/3), J = J_z / J_x, J_z = |det Z| (dJ_z/dZ = J_z Z^-T)
-__device__ __forceinline__ void mm3(const double A[3][3], const double B[3][3], double C[3][3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[i][j] = A[i][0] * B[0][j] + A[i][1] * B[1][j] + A[i][2] * B[2][j];
-}
-// C = A^T B
-__device__ __forceinline__ void mtm3(const double A[3][3], const double B[3][3], double C[3][3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[i][j] = A[0][i] * B[0][j] + A[1][i] * B[1][j] + A[2][i] * B[2][j];
-}
-// C = A B^T
-__device__ __forceinline__ void mmt3(const double A[3][3], const double B[3][3], double C[3][3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[i][j] = A[i][0] * B[j][0] + A[i][1] * B[j][1] + A[i][2] * B[j][2];
-}
-__device__ __forceinline__ double dot9(const double A[3][3], const double B[3][3]) {
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) s += A[i][j] * B[i][j];
-  return s;
-}
-
-__device__ __forceinline__ void point_P_vjp(const GPIn& in, double c1, double c2, const double V[3][3], double Vp,
-                                            double Zb[3][3], double& pb, double& c1b, double& c2b) {
-  // forward
-  double G[3][3];
-  mtm3(in.Z, in.Z, G);
-  const double Jz = sqrt(fabs(det3(G)));
-  double Zi[3][3];
-  inv3(in.Z, Zi);
-  const double J = Jz / in.Jx;
-  const double s = pow(J, -1.0 / 3.0);
-  double M[3][3], Fb[3][3];
-  mm3(in.Z, in.A, M);
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Fb[i][j] = M[i][j] * s;
-  double C[3][3];
-  mtm3(Fb, Fb, C);
-  const double I1 = C[0][0] + C[1][1] + C[2][2];
-  const double t1 = -2.0 * c2, t2 = 2.0 * (I1 * c2 + c1);
-  double S[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) S[i][j] = t1 * C[i][j] + (i == j ? t2 : 0.0);
-  double FS[3][3], sg[3][3];
-  mm3(Fb, S, FS);
-  mmt3(FS, Fb, sg);
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) sg[i][j] /= J;
-  const double tr3 = (sg[0][0] + sg[1][1] + sg[2][2]) / 3.0;
-  double sgd[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) sgd[i][j] = sg[i][j] - (i == j ? tr3 - in.p : 0.0);
-  double Q[3][3];
-  mm3(Zi, sgd, Q);
-  const double wj = Jz * in.w;
-  // reverse
-  double Jzb = in.w * (dot9(V, Q) + Vp);  // P = wj Q and the p-row term w (J_z - J_x)
-  double Qb[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Qb[i][j] = wj * V[i][j];
-  double Zib[3][3], sgdb[3][3];
-  mmt3(Qb, sgd, Zib);  // Q = Zi sgd: Zibar = Qbar sgd^T, sgdbar = Zi^T Qbar
-  mtm3(Zi, Qb, sgdb);
-  const double trb = sgdb[0][0] + sgdb[1][1] + sgdb[2][2];
-  pb = trb;
-  double sgb[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) sgb[i][j] = sgdb[i][j] - (i == j ? trb / 3.0 : 0.0);
-  // sg = H / J with H = FS Fb^T
-  double Jb = -dot9(sgb, sg) / J;
-  double Hb[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Hb[i][j] = sgb[i][j] / J;
-  double FSb[3][3], Fbb[3][3], T1[3][3];
-  mm3(Hb, Fb, FSb);   // H = FS Fb^T: FSbar = Hbar Fb
-  mtm3(Hb, FS, Fbb);  // Fbbar += Hbar^T FS
-  // FS = Fb S: Fbbar += FSbar S^T (S symmetric), Sbar = Fb^T FSbar
-  mm3(FSb, S, T1);
-  double Sb[3][3];
-  mtm3(Fb, FSb, Sb);
-  const double t2b = Sb[0][0] + Sb[1][1] + Sb[2][2];
-  const double t1b = dot9(Sb, C);
-  const double I1b = 2.0 * c2 * t2b;
-  c1b = 2.0 * t2b;
-  c2b = 2.0 * I1 * t2b - 2.0 * t1b;
-  double Cb[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Cb[i][j] = t1 * Sb[i][j] + (i == j ? I1b : 0.0);
-  // C = Fb^T Fb: Fbbar += Fb (Cbar + Cbar^T)
-  double Cs[3][3], T2[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Cs[i][j] = Cb[i][j] + Cb[j][i];
-  mm3(Fb, Cs, T2);
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Fbb[i][j] += T1[i][j] + T2[i][j];
-  // Fb = s M: sbar = Fbbar : M, Mbar = s Fbbar; M = Z A: Zbar += Mbar A^T
-  const double sb = dot9(Fbb, M);
-  double Mb[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Mb[i][j] = s * Fbb[i][j];
-  mmt3(Mb, in.A, Zb);
-  // s = J^(-1/3), J = J_z / J_x
-  Jb += sb * (-s / (3.0 * J));
-  Jzb += Jb / in.Jx;
-  // Zi = Z^-1: Zbar -= Zi^T Zibar Zi^T;  J_z = |det Z|: Zbar += Jzbar J_z Zi^T
-  double T3[3][3], T4[3][3];
-  mtm3(Zi, Zib, T3);   // Zi^T Zibar
-  mmt3(T3, Zi, T4);    // (Zi^T Zibar) Zi^T
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Zb[i][j] += -T4[i][j] + Jzb * Jz * Zi[j][i];
-}
-
-constexpr int kAdjWarps = 4;
-
-struct AdjWarpShared {
-  double x[81], z[81], p[8], v[ND];
-  double Zb[NG][9], pb[NG], cb[NG][2];
-  int dofs[ND];
-};
-
-// Reverse-mode vector-Jacobian products: one warp per (element, parameter set) of a colour.
-__global__ void __launch_bounds__(kAdjWarps * 32)
-mr_vjp_reverse_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t batch,
-                      const int32_t* __restrict__ eq2, const int32_t* __restrict__ elin, int32_t nq2, int32_t nlin,
-                      const double* __restrict__ xg, const double* __restrict__ dep, const double* __restrict__ cpar,
-                      const double* __restrict__ v, const Tables* __restrict__ Tg, double* __restrict__ du,
-                      double* __restrict__ dc_elem, int32_t n_elem, unsigned* err) {
-  extern __shared__ double smem[];
-  Tables& T = *reinterpret_cast<Tables*>(smem);
-  AdjWarpShared* W = reinterpret_cast<AdjWarpShared*>(smem + sizeof(Tables) / sizeof(double));
-  for (int i = threadIdx.x; i < (int)(sizeof(Tables) / sizeof(double)); i += blockDim.x)
-    smem[i] = reinterpret_cast<const double*>(Tg)[i];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  AdjWarpShared& S = W[w];
-  const int64_t ndof = 3ll * nq2 + nlin;
-  const long long total = (long long)count * batch;
-  for (long long item = (long long)blockIdx.x * kAdjWarps + w; item < total; item += (long long)gridDim.x * kAdjWarps) {
-    const int b = (int)(item / count);
-    const int e = __ldg(elems + (item % count));
-    const double* d = dep + b * ndof;
-    const double* vb = v + b * ndof;
-    for (int i = lane; i < NQ; i += 32) {
-      const int n = __ldg(eq2 + (size_t)e * NQ + i);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        S.x[c * NQ + i] = __ldg(xg + (size_t)c * nq2 + n);
-        S.z[c * NQ + i] = d[(size_t)c * nq2 + n];
-        S.dofs[c * NQ + i] = c * nq2 + n;
-        S.v[c * NQ + i] = vb[(size_t)c * nq2 + n];
-      }
-    }
-    if (lane < NL) {
-      const int n = __ldg(elin + (size_t)e * NL + lane);
-      S.p[lane] = d[(size_t)3 * nq2 + n];
-      S.dofs[81 + lane] = 3 * nq2 + n;
-      S.v[81 + lane] = vb[(size_t)3 * nq2 + n];
-    }
-    const double c1 = cpar[2 * b], c2 = cpar[2 * b + 1];
-    __syncwarp();
-    if (lane < NG) {
-      const int g = lane;
-      GPIn in;
-      gauss_inputs(T, g, S.z, S.x, S.p, in);
-      double V[3][3];
-#pragma unroll
-      for (int xi = 0; xi < 3; ++xi)
-#pragma unroll
-        for (int mh = 0; mh < 3; ++mh) {
-          double t = 0.0;
-          for (int ms = 0; ms < NQ; ++ms) t += S.v[mh * NQ + ms] * T.dphi[g][xi][ms];
-          V[xi][mh] = t;
-        }
-      double Vp = 0.0;
-#pragma unroll
-      for (int ms = 0; ms < NL; ++ms) Vp += S.v[81 + ms] * T.psi[g][ms];
-      double Zb[3][3], pb, c1b, c2b;
-      point_P_vjp(in, c1, c2, V, Vp, Zb, pb, c1b, c2b);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) S.Zb[g][i * 3 + k] = Zb[i][k];
-      S.pb[g] = pb;
-      S.cb[g][0] = c1b;
-      S.cb[g][1] = c2b;
-    }
-    __syncwarp();
-    if (lane < 2) {
-      double t = 0.0;
-      for (int g = 0; g < NG; ++g) t += S.cb[g][lane];
-      dc_elem[((size_t)b * n_elem + e) * 2 + lane] = t;
-    }
-    double* dub = du + b * ndof;
-    for (int i = lane; i < ND; i += 32) {
-      double t = 0.0;
-      if (i < 81) {
-        const int c = i / NQ, ns = i % NQ;
-        for (int g = 0; g < NG; ++g)
-          t += S.Zb[g][c * 3 + 0] * T.dphi[g][0][ns] + S.Zb[g][c * 3 + 1] * T.dphi[g][1][ns] +
-               S.Zb[g][c * 3 + 2] * T.dphi[g][2][ns];
-      } else {
-        const int ns = i - 81;
-        for (int g = 0; g < NG; ++g) t += S.pb[g] * T.psi[g][ns];
-      }
-      if (!isfinite(t)) gfe_raise(err, GFE_DEVERR_NONFINITE);
-      dub[S.dofs[i]] += t;
-    }
-    __syncwarp();
-  }
-}
-
-__global__ void sum_dc(const double* __restrict__ dc_elem, int32_t n_elem, int32_t batch, double* __restrict__ dc) {
-  const int b = blockIdx.x, q = threadIdx.x & 1;
-  if (threadIdx.x >= 2) return;
-  double s = 0.0;
-  for (int e = 0; e < n_elem; ++e) s += dc_elem[((size_t)b * n_elem + e) * 2 + q];
-  dc[b * 2 + q] = s;
-}
-
-// ----------------------------------------------------------------------------------------------
 // Element Jacobians: Iron's analytic tangent and the consistent tangent
 // ----------------------------------------------------------------------------------------------
 // Both are sums over Gauss points of  K(ms mh, ns nh) = g_ms^T D_g^(mh,nh) g_ns  (u-u block) with
 // the reference basis gradients g (constant tables) and 3x3 blocks D_g expressed in xi space, plus
 // the u-p / p-u blocks.  The work is split in two kernels:
-//  * mr_gp_kernel, one thread per (element, Gauss point): kinematics and material tangent in FP64,
-//    written as D_g (9 blocks x 9), Hv_g (u-p coefficients) and Pv_g (p-u coefficients);
-//  * mr_contract_kernel, one CTA per element: H_g = D_g G_g (per Gauss point, 3 x 81 x 81 values
-//    in shared memory), then the contraction K_mh^T = H_mh^T G^T against the constant table
-//    G[(g,xi)][ms] (a 81 x 27 x 81 product per displacement component), the u-p / p-u blocks, and
-//    the scatter into CSR through the per-element slot map.
-// The contraction runs in FP64 (GFE_FP64) or FP32 (GFE_MIXED; the kinematics and det(F) stay FP64,
-// the assembled values are accumulated in FP64).
+//  * mr_gp_kernel, one thread per (element, Gauss point): kinematics and material tangent, written as
+//    D_g (9 blocks x 9), Hv_g (u-p coefficients) and Pv_g (p-u coefficients);
+//  * mr_contract_kernel / mr_contract_tc_kernel, one CTA per element: the contraction with the constant
+//    table G[(g,xi)][ms] and the u-p / p-u blocks.
+// The kernels here serve the FP32 paths (FP32 kinematics with det(F) in FP64, FP32 or TF32 contraction,
+// FP64 assembled values).
 //
 // Iron's analytic tangent (src/finite_elasticity_routines.F90:1016-1274): the spatial blocks
 // J_z w (c + sigma) / J_z w c of FINITE_ELASTICITY_GAUSS_ELASTICITY_TENSOR (:649-795) mapped to xi
@@ -1382,8 +981,6 @@ mr_contract_tc_kernel(const int32_t* __restrict__ elems, int32_t count, const Ta
   if (warp == 0 && S.abort < 2) tc::tmem_dealloc(tmem, 64);
 }
 
-size_t residual_smem() { return sizeof(Tables) + kResWarps * sizeof(double) * (81 + 81 + 8 + NG * 9 + NG + 48); }
-
 int check_mesh(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2, int32_t nlin, const double* xg,
                const char* fn) {
   if (n_elem < 0 || nq2 <= 0 || nlin <= 0 || (n_elem > 0 && (!eq2 || !elin || !xg)))
@@ -1397,41 +994,6 @@ int set_smem(const void* kernel, size_t bytes) {
 }
 
 }  // namespace
-
-extern "C" int gfe_mr_residual(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2, int32_t nlin,
-                               const double* xg, const int32_t* color_elems, const int32_t* color_ptr_host,
-                               int32_t n_colors, int32_t batch, const double* dep, const double* cpar, double* R,
-                               void* stream) {
-  const char* fn = "gfe_mr_residual";
-  int rc = check_mesh(n_elem, eq2, elin, nq2, nlin, xg, fn);
-  if (rc) return rc;
-  if (batch <= 0 || !dep || !cpar || !R || (n_elem > 0 && (!color_elems || !color_ptr_host || n_colors <= 0)))
-    return gfe::set_error(GFE_ERR_ARG, "%s: invalid arguments", fn);
-  if (color_ptr_host[0] != 0 || color_ptr_host[n_colors] != n_elem)
-    return gfe::set_error(GFE_ERR_ARG, "%s: colour offsets must run from 0 to n_elem", fn);
-  const Tables* T = nullptr;
-  if ((rc = device_tables(&T))) return rc;
-  cudaStream_t s = gfe::as_stream(stream);
-  const int64_t ndof = 3ll * nq2 + nlin;
-  GFE_CUDA_TRY(cudaMemsetAsync(R, 0, sizeof(double) * ndof * batch, s));
-  const size_t sm = residual_smem();
-  if ((rc = set_smem((const void*)mr_residual_kernel, sm))) return rc;
-  unsigned* err = gfe::device_error_word();
-  void* prof = gfe::stage_begin(GFE_STAGE_MR_RESIDUAL, s);
-  int launches = 0;
-  for (int c = 0; c < n_colors; ++c) {
-    const int c0 = color_ptr_host[c], cnt = color_ptr_host[c + 1] - c0;
-    if (cnt <= 0) continue;
-    const long long items = (long long)cnt * batch;
-    const int grid = (int)std::min<long long>((items + kResWarps - 1) / kResWarps, 16ll * gfe::sm_count());
-    mr_residual_kernel<<<grid, kResWarps * 32, sm, s>>>(color_elems + c0, cnt, batch, eq2, elin, nq2, nlin, xg, dep,
-                                                       cpar, T, R, ndof, err);
-    ++launches;
-  }
-  gfe::stage_end(GFE_STAGE_MR_RESIDUAL, prof, s, launches);
-  GFE_LAUNCH_CHECK(fn);
-  return GFE_OK;
-}
 
 extern "C" int gfe_mr_slot_map(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2,
                                const int32_t* color_elems, const int32_t* row_ptr, const int32_t* col_idx,
@@ -1627,40 +1189,4 @@ extern "C" int gfe_mr_tangent(int32_t n_elem, const int32_t* eq2, const int32_t*
                               void* stream) {
   return jacobian_entry_point(1, n_elem, eq2, elin, nq2, nlin, xg, color_elems, color_ptr_host, n_colors, dep, cpar,
                               slots, row_ptr, values, nnz, K_out, precision, stream, "gfe_mr_tangent");
-}
-
-extern "C" int gfe_mr_residual_vjp(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2,
-                                   int32_t nlin, const double* xg, const int32_t* color_elems,
-                                   const int32_t* color_ptr_host, int32_t n_colors, int32_t batch, const double* dep,
-                                   const double* cpar, const double* v, double* du, double* dc, void* stream) {
-  const char* fn = "gfe_mr_residual_vjp";
-  int rc = check_mesh(n_elem, eq2, elin, nq2, nlin, xg, fn);
-  if (rc) return rc;
-  if (batch <= 0 || !dep || !cpar || !v || !du || !dc || (n_elem > 0 && (!color_elems || !color_ptr_host)))
-    return gfe::set_error(GFE_ERR_ARG, "%s: invalid arguments", fn);
-  if (color_ptr_host[0] != 0 || color_ptr_host[n_colors] != n_elem)
-    return gfe::set_error(GFE_ERR_ARG, "%s: colour offsets must run from 0 to n_elem", fn);
-  const Tables* T = nullptr;
-  if ((rc = device_tables(&T))) return rc;
-  cudaStream_t s = gfe::as_stream(stream);
-  const int64_t ndof = 3ll * nq2 + nlin;
-  GFE_CUDA_TRY(cudaMemsetAsync(du, 0, sizeof(double) * ndof * batch, s));
-  double* dc_elem = nullptr;
-  if ((rc = gfe::scratch_alloc((void**)&dc_elem, sizeof(double) * 2 * (size_t)n_elem * batch, s, "vjp partials")))
-    return rc;
-  const size_t sm = sizeof(Tables) + kAdjWarps * sizeof(AdjWarpShared);
-  if ((rc = set_smem((const void*)mr_vjp_reverse_kernel, sm))) { gfe::scratch_free(dc_elem, s); return rc; }
-  unsigned* err = gfe::device_error_word();
-  for (int c = 0; c < n_colors; ++c) {
-    const int c0 = color_ptr_host[c], cnt = color_ptr_host[c + 1] - c0;
-    if (cnt <= 0) continue;
-    const long long items = (long long)cnt * batch;
-    const int grid = (int)std::min<long long>((items + kAdjWarps - 1) / kAdjWarps, 16ll * gfe::sm_count());
-    mr_vjp_reverse_kernel<<<grid, kAdjWarps * 32, sm, s>>>(color_elems + c0, cnt, batch, eq2, elin, nq2, nlin, xg,
-                                                           dep, cpar, v, T, du, dc_elem, n_elem, err);
-  }
-  sum_dc<<<batch, 32, 0, s>>>(dc_elem, n_elem, batch, dc);
-  gfe::scratch_free(dc_elem, s);
-  GFE_LAUNCH_CHECK(fn);
-  return GFE_OK;
 }

@@ -220,7 +220,7 @@ __device__ __forceinline__ double point_pressure(int g, const double* p) {
 // With Z = dz/dxi, X = dx/dxi and Iron's fibre-free material frame A = (N^T X)^-1, N the columns of X
 // normalised (src/coordinate_routines.F90:3841-3947), the residual's Cauchy stress
 // (src/finite_elasticity_routines.F90:6985-7061) depends on F = Z A only through F F^T = Z H Z^T with
-// H = A A^T = GU diag(G_jj) GU, G = X^T X, GU = G^-1: no square root, six numbers a point.  With
+// H = A A^T = (G D^-1 G)^-1, G = X^T X, D = diag(G): no square root, six numbers a point.  With
 // J = J_z / J_x, r = J^(-1/3) and B = r^2 Z H Z^T,
 //   sigma = dev((t1 B^2 + t2 B) / J) + p I,  t1 = -2 c2,  t2 = 2 (c1 + tr(B) c2),
 // and the first Piola form of the residual is P[xi][m] = w J_z (Z^-1 sigma)[xi][m] =
@@ -241,33 +241,38 @@ __device__ __forceinline__ double cofactors(const double (&Z)[3][3], double (&co
   return Z[0][0] * cof[0][0] + Z[0][1] * cof[0][1] + Z[0][2] * cof[0][2];
 }
 
-// H (packed) and J_x of a reference gradient matrix
+// H (packed) and J_x of a reference gradient matrix.  H = (G D^-1 G)^-1 with D = diag(G): the
+// diagonal of K = G D^-1 G is G_ii plus small terms, so H's entries differ by the rounding of one or
+// two products; rounding common to all of them only scales B, which the deviator does not amplify
+// (near the undeformed state it amplifies differences between B's diagonal entries).
 __device__ __forceinline__ double geometry(const double (&X)[3][3], double (&H)[6]) {
-  double cof[3][3];
-  const double det = cofactors(X, cof);
-  const double q = 1.0 / (det * det);
-  double U[3][3];  // GU
+  double G[6];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+  for (int i = 0; i < 3; ++i) G[i] = X[0][i] * X[0][i] + X[1][i] * X[1][i] + X[2][i] * X[2][i];
+  G[3] = X[0][0] * X[0][1] + X[1][0] * X[1][1] + X[2][0] * X[2][1];
+  G[4] = X[0][0] * X[0][2] + X[1][0] * X[1][2] + X[2][0] * X[2][2];
+  G[5] = X[0][1] * X[0][2] + X[1][1] * X[1][2] + X[2][1] * X[2][2];
+  const double g01 = G[0] * G[1], d = 1.0 / (g01 * G[2]);
+  const double i0 = G[1] * G[2] * d, i1 = G[0] * G[2] * d, i2 = g01 * d;  // 1 / G_kk
+  const double a3 = G[3] * i1, a4 = G[4] * i2, b3 = G[3] * i0, b5 = G[5] * i2, c4 = G[4] * i0, c5 = G[5] * i1;
+  double K[6];
+  K[0] = G[0] + fma(G[3], a3, G[4] * a4);
+  K[1] = G[1] + fma(G[3], b3, G[5] * b5);
+  K[2] = G[2] + fma(G[4], c4, G[5] * c5);
+  K[3] = fma(2.0, G[3], G[5] * a4);
+  K[4] = fma(2.0, G[4], G[5] * a3);
+  K[5] = fma(2.0, G[5], G[4] * b3);
+  H[0] = K[1] * K[2] - K[5] * K[5];
+  H[1] = K[0] * K[2] - K[4] * K[4];
+  H[2] = K[0] * K[1] - K[3] * K[3];
+  H[3] = K[4] * K[5] - K[3] * K[2];
+  H[4] = K[3] * K[5] - K[4] * K[1];
+  H[5] = K[3] * K[4] - K[5] * K[0];
+  const double q = 1.0 / (K[0] * H[0] + K[3] * H[3] + K[4] * H[4]);
 #pragma unroll
-    for (int j = i; j < 3; ++j) {
-      U[i][j] = (cof[0][i] * cof[0][j] + cof[1][i] * cof[1][j] + cof[2][i] * cof[2][j]) * q;
-      U[j][i] = U[i][j];
-    }
-  double T[3][3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const double G = X[0][j] * X[0][j] + X[1][j] * X[1][j] + X[2][j] * X[2][j];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) T[i][j] = U[i][j] * G;
-  }
-  H[0] = T[0][0] * U[0][0] + T[0][1] * U[0][1] + T[0][2] * U[0][2];
-  H[1] = T[1][0] * U[1][0] + T[1][1] * U[1][1] + T[1][2] * U[1][2];
-  H[2] = T[2][0] * U[2][0] + T[2][1] * U[2][1] + T[2][2] * U[2][2];
-  H[3] = T[0][0] * U[1][0] + T[0][1] * U[1][1] + T[0][2] * U[1][2];
-  H[4] = T[0][0] * U[2][0] + T[0][1] * U[2][1] + T[0][2] * U[2][2];
-  H[5] = T[1][0] * U[2][0] + T[1][1] * U[2][1] + T[1][2] * U[2][2];
-  return fabs(det);
+  for (int i = 0; i < 6; ++i) H[i] *= q;
+  return fabs(X[0][0] * (X[1][1] * X[2][2] - X[1][2] * X[2][1]) + X[0][1] * (X[1][2] * X[2][0] - X[1][0] * X[2][2]) +
+              X[0][2] * (X[1][0] * X[2][1] - X[1][1] * X[2][0]));
 }
 
 // row of Z times H
