@@ -388,6 +388,12 @@ __device__ __forceinline__ float tp_rsqrt<float>(float a) {
   return rsqrtf(a);
 }
 
+}  // namespace
+
+#include "laplace_tp_sf.cuh"
+
+namespace {
+
 // Element group of GROUP threads: GROUP = kTPThreads gives one element a block (triquadratic,
 // tricubic and Hermite elements: up to 64 nodes, 2,080 entry pairs); GROUP = 32 gives one element
 // a warp, eight a block (elements of at most kSmallNns nodes and kSmallNg Gauss points: linear and
@@ -838,6 +844,13 @@ int launch_tp(const int32_t* order, const int32_t* ngauss, int32_t n_nodes, cons
               const double* scale, const double* kappa, const int32_t* color_elems, const int32_t* color_ptr_host, int32_t n_colors,
               const int32_t* rp, const int32_t* ci, const int32_t* slots, double* values, cudaStream_t s,
               int* launches) {
+  if constexpr (!std::is_same<T, float>::value) {
+    const int sf = sf_functions(order, ngauss);
+    if (sf)
+      return (sf == 3 ? launch_tp_sf<T, 3> : launch_tp_sf<T, 4>)(order, ngauss, n_nodes, en, coords, scale, kappa,
+                                                                 color_elems, color_ptr_host, n_colors, rp, ci, slots,
+                                                                 values, s, launches);
+  }
   const TPTables<T>* t = nullptr;
   if (int rc = tp_tables<T>(order, ngauss, &t)) return rc;
   unsigned* err = gfe::device_error_word();

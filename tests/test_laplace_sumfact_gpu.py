@@ -1,0 +1,67 @@
+"""Sum-factorised basis-generic assembly (quadratic and cubic hexahedra, FP64 and float-float) against the
+oracle: every mixture of cubic Lagrange and cubic Hermite directions (element parameter order and scale
+factors), element counts around the kernel's forms (all elements at once through scratch, or colour by
+colour beyond 256 MB of element matrices), with the slot map and with the row search.  Tolerance 1e-12
+relative to max|K|, as for the same precisions in test_laplace_tp_gpu.
+"""
+import itertools
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from iron_gb300.laplace import LaplaceAssembly
+from iron_gb300.mesh import RegularMesh
+
+pytestmark = pytest.mark.gpu
+
+
+def _separate_elements(order, E, seed):
+    """E disjoint curved elements of one basis: parameters of a perturbed identity map."""
+    rng = np.random.default_rng(seed)
+    nn = [2 if o == 4 else o + 1 for o in order]
+    herm = [d for d in range(3) if order[d] == 4]
+    rows = []
+    for a3, a2, a1 in itertools.product(range(nn[2]), range(nn[1]), range(nn[0])):
+        for k in range(2 ** len(herm)):
+            on = [d for i, d in enumerate(herm) if (k >> i) & 1]
+            at = (a1, a2, a3)
+            rows.append([at[c] / (nn[c] - 1) if not on else float(on == [c]) for c in range(3)])
+    base = np.array(rows).T  # [3][nns]
+    nns = base.shape[1]
+    x = base[:, None, :] + rng.uniform(-0.02, 0.02, (3, E, nns))
+    return np.arange(E * nns, dtype=np.int32).reshape(E, nns), x.reshape(3, -1), rng.uniform(0.8, 1.25, (E, nns)), rng
+
+
+@pytest.mark.parametrize("order", [(2, 2, 2), (3, 3, 3), (4, 4, 4), (4, 3, 3), (3, 4, 3), (3, 3, 4), (3, 4, 4), (4, 3, 4)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed_df"])
+@pytest.mark.parametrize("E,slot_map,scaled", [(1, True, False), (5, False, True)])
+def test_bases_match_oracle(gfe_cuda, order, precision, E, slot_map, scaled):
+    ep, x, sf, rng = _separate_elements(order, E, 3)
+    kap = rng.uniform(0.5, 2.0, E)
+    ng = [o + 1 if o < 4 else 4 for o in order]
+    scale = sf if scaled else None
+    if scaled:  # scaled parameters interpolate the same geometry
+        x = x / sf.reshape(1, -1)
+    A = LaplaceAssembly(ep, x, kappa=kap, order=order, n_gauss=ng, scale=scale, slot_map=slot_map)
+    v = A.assemble(precision).cpu().numpy()
+    rp, ci = oracle.csr_structure(ep, x.shape[1])
+    ov = oracle.laplace_assemble_scaled(3, list(order), ng, ep, x, scale, kap, rp, ci, 1)
+    assert np.abs(v - ov).max() <= 1e-12 * np.abs(ov).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed_df"])
+@pytest.mark.parametrize("order,ne", [(2, (46, 45, 44)), (3, (26, 25, 25))])
+def test_colour_by_colour_beyond_scratch(gfe_cuda, order, ne, precision):
+    m = RegularMesh(ne, order=order)
+    m.jitter_interior(1)
+    kap = np.random.default_rng(2).uniform(0.5, 2.0, m.n_elements)
+    A = LaplaceAssembly.from_regular_mesh(m, kappa=kap)
+    nns = (order + 1) ** 3
+    assert 8 * m.n_elements * nns * (nns + 1) // 2 > 256 << 20
+    v = A.assemble(precision).cpu().numpy()
+    rp, ci = A.row_ptr.cpu().numpy(), A.col_idx.cpu().numpy()
+    ov = oracle.laplace_assemble_scaled(3, [order] * 3, [order + 1] * 3, m.elem_nodes, m.coords, None, kap, rp, ci, 16)
+    assert np.abs(v - ov).max() <= 1e-12 * np.abs(ov).max()
+    assert torch.equal(A.values, A.assemble(precision))
