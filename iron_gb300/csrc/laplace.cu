@@ -38,6 +38,10 @@
 namespace {
 
 constexpr int kBlock = 128;
+// 1D basis values at the points of the 2-point rule: p = (1 + 1/sqrt3) / 2, q = (1 - 1/sqrt3) / 2
+constexpr double kGaussQ = 0.21132486540518711775;
+constexpr double kPoverQ = 3.73205080756887729353;           // p / q = 2 + sqrt(3)
+constexpr double kPP1 = kPoverQ * kPoverQ - 1.0;             // (p / q)^2 - 1
 
 __host__ __device__ constexpr int tri(int m, int n) {  // packed upper-triangular index, m <= n < 8
   return m * 8 - (m * (m - 1)) / 2 + (n - m);
@@ -54,8 +58,16 @@ __device__ __forceinline__ T wwv(int k, int g, T p, T q) {
   return (k == 0) == (g == 0) ? p * p : q * q;
 }
 
-// Metrics of one trilinear hexahedron at its 8 Gauss points: M[g] = GU Jacobian w kappa as the six
-// entries 00 11 22 01 02 12 of the symmetric 3x3 matrix.  x[c][m]: coordinates of local node m
+// The double and float-float contraction works with the 1D values divided by q (p / q and 1), which
+// leaves one operation for each product by 1: the metrics carry the factor q^4 that every entry needs.
+// FP32 keeps the values p and q themselves.
+template <typename T>
+__device__ __forceinline__ constexpr double metric_scale() {
+  return std::is_same<T, float>::value ? 1.0 : kGaussQ * kGaussQ * kGaussQ * kGaussQ;
+}
+
+// Metrics of one trilinear hexahedron at its 8 Gauss points: M[g] = GU Jacobian w kappa (times
+// metric_scale) as the six entries 00 11 22 01 02 12 of the symmetric 3x3 matrix.  x[c][m]: coordinates of local node m
 // (m = m1 + 2 m2 + 4 m3, Iron's local node order).  Returns false if det(GL) <= 0.
 template <typename T>
 __device__ __forceinline__ bool hex8_metrics(const T (&x)[3][8], T kappa, T p, T q, T (&M)[8][6]) {
@@ -75,18 +87,36 @@ __device__ __forceinline__ bool hex8_metrics(const T (&x)[3][8], T kappa, T p, T
           const int m0 = (i << d1) | (j << d2);
           D[i][j] = x[c][m0 | (1 << a)] - x[c][m0];
         }
+      if constexpr (std::is_same<T, double>::value) {
+        // d0 p + d1 q = d0 + q (d1 - d0) and d0 q + d1 p = d0 + p (d1 - d0): three operations for both
+        // points instead of four
+        double E[2][2];
 #pragma unroll
-      for (int g2 = 0; g2 < 2; ++g2) {
-        T E0 = D[0][0] * wv(0, g2, p, q) + D[0][1] * wv(1, g2, p, q);
-        T E1 = D[1][0] * wv(0, g2, p, q) + D[1][1] * wv(1, g2, p, q);
+        for (int i = 0; i < 2; ++i) {
+          const double d = D[i][1] - D[i][0];
+          E[i][0] = fma(q, d, D[i][0]);
+          E[i][1] = fma(p, d, D[i][0]);
+        }
 #pragma unroll
-        for (int g1 = 0; g1 < 2; ++g1) Jt[c][a][g1][g2] = E0 * wv(0, g1, p, q) + E1 * wv(1, g1, p, q);
+        for (int g2 = 0; g2 < 2; ++g2) {
+          const double d = E[1][g2] - E[0][g2];
+          Jt[c][a][0][g2] = fma(q, d, E[0][g2]);
+          Jt[c][a][1][g2] = fma(p, d, E[0][g2]);
+        }
+      } else {
+#pragma unroll
+        for (int g2 = 0; g2 < 2; ++g2) {
+          T E0 = D[0][0] * wv(0, g2, p, q) + D[0][1] * wv(1, g2, p, q);
+          T E1 = D[1][0] * wv(0, g2, p, q) + D[1][1] * wv(1, g2, p, q);
+#pragma unroll
+          for (int g1 = 0; g1 < 2; ++g1) Jt[c][a][g1][g2] = E0 * wv(0, g1, p, q) + E1 * wv(1, g1, p, q);
+        }
       }
     }
   }
   // M_g[ab] for the 8 Gauss points, symmetric: 00 11 22 01 02 12
   bool ok = true;
-  const T eighth = kappa * from_double<T>(0.125);
+  const T eighth = kappa * from_double<T>(0.125 * metric_scale<T>());
 #pragma unroll
   for (int g = 0; g < 8; ++g) {
     const int gb[3] = {g & 1, (g >> 1) & 1, (g >> 2) & 1};
@@ -208,9 +238,121 @@ __device__ __forceinline__ void hex8_contract_at(MetricAt Mg, T p, T q, T (&K)[3
   for (int k = 0; k < 36; ++k) finish(K[k]);
 }
 
+// a x + y
+__device__ __forceinline__ double axpy(double a, double x, double y) { return fma(a, x, y); }
+__device__ __forceinline__ f2 axpy(f2 a, f2 x, f2 y) { return a * x + y; }
+
+// o[k] = sum over the two points of products of the scaled 1D values keyed by k = m + n: s0 (p/q)^2 + s1,
+// (s0 + s1) p/q, s0 + s1 (p/q)^2
+template <typename T>
+__device__ __forceinline__ void pair_sums(T s0, T s1, T r, T pp1, T (&o)[3]) {
+  const T s = s0 + s1;
+  o[0] = axpy(pp1, s0, s);
+  o[1] = r * s;
+  o[2] = axpy(pp1, s1, s);
+}
+
+// hex8_contract_at in FP64 and float-float with fewer operations (about 390 instead of 590): scaled 1D
+// values (metric_scale), the symmetric part of each entry formed once per distinct triple of pairs (27 of
+// the 36 entries) and the two orders of each off-diagonal term added before they meet the entries.
+// 128^3 float-float assembly 1.27 -> 1.22 ms.
+template <typename T, typename MetricAt>
+__device__ __forceinline__ void hex8_contract_scaled(MetricAt Mg, T (&K)[36]) {
+  const T r = from_double<T>(kPoverQ), pp1 = from_double<T>(kPP1);
+  // symmetric part by (k1, k2, k3), k = 0: both nodes 0, 1: different, 2: both 1
+  T Sy[3][3][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int d1 = a == 0 ? 1 : 0, d2 = a == 2 ? 1 : 2;
+    T Tt[2][3];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int g0 = j << d2, g1 = g0 | (1 << d1);
+      pair_sums(Mg(g0, a) + Mg(g0 | (1 << a), a), Mg(g1, a) + Mg(g1 | (1 << a), a), r, pp1, Tt[j]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      T V[3];
+      pair_sums(Tt[0][k1], Tt[1][k1], r, pp1, V);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; ++k2)
+#pragma unroll
+        for (int ka = 0; ka < 3; ++ka) {
+          int k[3];
+          k[a] = ka;
+          k[d1] = k1;
+          k[d2] = k2;
+          T& o = Sy[k[0]][k[1]][k[2]];
+          if (a == 0) o = ka == 1 ? -V[k2] : V[k2];
+          else if (ka == 1) accum_sub(o, V[k2]);
+          else accum(o, V[k2]);
+        }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int n = m; n < 8; ++n)
+      K[tri(m, n)] = Sy[(m & 1) + (n & 1)][((m >> 1) & 1) + ((n >> 1) & 1)][(m >> 2) + (n >> 2)];
+  // off-diagonal pairs (a,b), a < b, c the third direction; M index 3:(0,1) 4:(0,2) 5:(1,2)
+#pragma unroll
+  for (int pr = 0; pr < 3; ++pr) {
+    const int a = pr == 2 ? 1 : 0, b = pr == 0 ? 1 : 2, c = 3 - a - b, mi = 3 + pr;
+    T W[2][2][3];  // [n_a][m_b][k]
+    {
+      T U[2][2][2];  // [i = n_a][gb][gc]
+#pragma unroll
+      for (int gb = 0; gb < 2; ++gb)
+#pragma unroll
+        for (int gc = 0; gc < 2; ++gc) {
+          const int g0 = (gb << b) | (gc << c);
+          const T m0 = Mg(g0, mi), m1 = Mg(g0 | (1 << a), mi);
+          U[0][gb][gc] = axpy(r, m0, m1);
+          U[1][gb][gc] = axpy(r, m1, m0);
+        }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        pair_sums(axpy(r, U[i][0][0], U[i][1][0]), axpy(r, U[i][0][1], U[i][1][1]), r, pp1, W[i][0]);
+        pair_sums(axpy(r, U[i][1][0], U[i][0][0]), axpy(r, U[i][1][1], U[i][0][1]), r, pp1, W[i][1]);
+      }
+    }
+    // C_ab(m,n) + C_ab(n,m) = s(m_a) s(n_b) W[n_a][m_b][k] + s(n_a) s(m_b) W[m_a][n_b][k], s(1) = 1, s(0) = -1
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int ma = 0; ma < 2; ++ma)
+#pragma unroll
+        for (int mb = 0; mb < 2; ++mb)
+#pragma unroll
+          for (int na = 0; na < 2; ++na)
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) {
+              if (ma * 2 + mb > na * 2 + nb) continue;  // the other order of the same sum
+              const bool sa = ma == nb, sb = na == mb;
+              const T t1 = W[na][mb][k], t2 = W[ma][nb][k];
+              const T x = sa == sb ? t1 + t2 : (sa ? t1 - t2 : t2 - t1);
+              // the entries with these (a, b) indices, in either order, and pair k in direction c
+#pragma unroll
+              for (int mc = 0; mc < 2; ++mc)
+#pragma unroll
+                for (int nc = 0; nc < 2; ++nc) {
+                  if (mc + nc != k) continue;
+                  const int m = (ma << a) | (mb << b) | (mc << c), n = (na << a) | (nb << b) | (nc << c);
+                  if (ma == na && mb == nb && mc > nc) continue;  // the same entry in its other order
+                  T& o = K[m <= n ? tri(m, n) : tri(n, m)];
+                  if (!sa && !sb) accum_sub(o, x);
+                  else accum(o, x);
+                }
+            }
+  }
+#pragma unroll
+  for (int k = 0; k < 36; ++k) finish(K[k]);
+}
+
 template <typename T>
 __device__ __forceinline__ void hex8_contract(const T (&M)[8][6], T p, T q, T (&K)[36]) {
-  hex8_contract_at<T>([&](int g, int k) { return M[g][k]; }, p, q, K);
+  if constexpr (std::is_same<T, float>::value) hex8_contract_at<T>([&](int g, int k) { return M[g][k]; }, p, q, K);
+  else hex8_contract_scaled<T>([&](int g, int k) { return M[g][k]; }, K);
 }
 
 // Element stiffness of one trilinear hexahedron (metrics, then contraction).  Returns the 36
@@ -593,20 +735,164 @@ laplace_metric_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__ 
 // Element matrices of element layers [ez0, ez1) from their metrics into Kel[36][E] (entry
 // tri(m, n) of element e at tri(m, n) E + e).
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 4)
 laplace_contract_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__ metrics, T* __restrict__ Kel,
                         int32_t ez0, int32_t ez1) {
   const long long EXY = (long long)nx * ny, E = EXY * nz;
-  T p, q;
-  gauss_pq(p, q);
   for (long long e = ez0 * EXY + blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ez1 * EXY;
        e += (long long)gridDim.x * blockDim.x) {
     // a direction's component is loaded where the contraction uses it, not all 48 entries up front
     const T* src = metrics + (e >> 5) * (48 * 32) + (e & 31);
     T K[36];
-    hex8_contract_at<T>([&](int g, int k) { return load_coord(src + (k * 8 + g) * 32); }, p, q, K);
+    hex8_contract_scaled<T>([&](int g, int k) { return load_coord(src + (k * 8 + g) * 32); }, K);
 #pragma unroll
     for (int k = 0; k < 36; ++k) Kel[k * E + e] = K[k];
+  }
+}
+
+// FP64 element matrices of every element into Kel[36][E], metrics and contraction in one kernel (the code
+// fits the instruction cache): a thread an element.  Bound by the FP64 pipe: about 960 operations an
+// element.
+__global__ void __launch_bounds__(128)
+laplace_element64_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __restrict__ coords,
+                         const double* __restrict__ kappa, double* __restrict__ Kel, unsigned* err) {
+  const long long EXY = (long long)nx * ny, E = EXY * nz;
+  const long long NX = nx + 1, NXY = NX * (ny + 1), N = NXY * (nz + 1);
+  double p, q;
+  gauss_pq(p, q);
+  bool bad = false, nonfinite = false;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E; e += (long long)gridDim.x * blockDim.x) {
+    const long long ex = e % nx, ey = (e / nx) % ny, ez = e / EXY;
+    double x[3][8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const long long n = (ex + (m & 1)) + (ey + ((m >> 1) & 1)) * NX + (ez + (m >> 2)) * NXY;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) x[c][m] = __ldg(coords + c * N + n);
+    }
+    const double kd = kappa ? __ldg(kappa + e) : 1.0;
+    if (!isfinite(kd)) nonfinite = true;
+    double K[36];
+    if (!laplace_hex8<double>(x, kd, p, q, K)) bad = true;
+#pragma unroll
+    for (int k = 0; k < 36; ++k) Kel[k * E + e] = K[k];
+  }
+  if (bad) gfe_raise(err, GFE_DEVERR_JACOBIAN);
+  if (nonfinite) gfe_raise(err, GFE_DEVERR_NONFINITE);
+}
+
+// The same for meshes too small to give every SM sub-partition a warp of elements: eight lanes an element,
+// a Gauss point each for the metrics, then the 63 directional sums of the contraction and the 36 entries
+// spread over the lanes.  On an idle GPU a kernel's time is its longest chain at one FP64 instruction in
+// 64 cycles: about 270 instructions here, 960 for a thread an element.
+__global__ void __launch_bounds__(128)
+laplace_element64_small_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __restrict__ coords,
+                               const double* __restrict__ kappa, double* __restrict__ Kel, unsigned* err) {
+  __shared__ double sx[16][24], sM[16][6][8], sV[16][63];
+  const int le = threadIdx.x >> 3, g = threadIdx.x & 7;
+  const long long EXY = (long long)nx * ny, E = EXY * nz;
+  const long long NX = nx + 1, NXY = NX * (ny + 1), N = NXY * (nz + 1);
+  const long long e = blockIdx.x * 16ll + le;
+  const bool on = e < E;
+  double p, q, kd = 1.0;
+  gauss_pq(p, q);
+  if (on) {
+    const long long ex = e % nx, ey = (e / nx) % ny, ez = e / EXY;
+    const long long n = (ex + (g & 1)) + (ey + ((g >> 1) & 1)) * NX + (ez + (g >> 2)) * NXY;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sx[le][c * 8 + g] = __ldg(coords + c * N + n);
+    kd = kappa ? __ldg(kappa + e) : 1.0;
+    if (!isfinite(kd)) gfe_raise(err, GFE_DEVERR_NONFINITE);
+  }
+  __syncwarp();
+  {
+    // Gauss point g = (g1, g2, g3): weights of node 1 in each direction
+    const double t[3] = {g & 1 ? p : q, g & 2 ? p : q, g & 4 ? p : q};
+    double J[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const int d1 = a == 0 ? 1 : 0, d2 = a == 2 ? 1 : 2;
+        const double* x = sx[le] + c * 8;
+        double D[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int m0 = (i << d1) | (j << d2);
+            D[i][j] = x[m0 | (1 << a)] - x[m0];
+          }
+        const double E0 = fma(t[d2], D[0][1] - D[0][0], D[0][0]), E1 = fma(t[d2], D[1][1] - D[1][0], D[1][0]);
+        J[c][a] = fma(t[d1], E1 - E0, E0);
+      }
+    const double G00 = J[0][0] * J[0][0] + J[1][0] * J[1][0] + J[2][0] * J[2][0];
+    const double G11 = J[0][1] * J[0][1] + J[1][1] * J[1][1] + J[2][1] * J[2][1];
+    const double G22 = J[0][2] * J[0][2] + J[1][2] * J[1][2] + J[2][2] * J[2][2];
+    const double G01 = J[0][0] * J[0][1] + J[1][0] * J[1][1] + J[2][0] * J[2][1];
+    const double G02 = J[0][0] * J[0][2] + J[1][0] * J[1][2] + J[2][0] * J[2][2];
+    const double G12 = J[0][1] * J[0][2] + J[1][1] * J[1][2] + J[2][1] * J[2][2];
+    const double A00 = G11 * G22 - G12 * G12, A11 = G00 * G22 - G02 * G02, A22 = G00 * G11 - G01 * G01;
+    const double A01 = G02 * G12 - G01 * G22, A02 = G01 * G12 - G02 * G11, A12 = G01 * G02 - G00 * G12;
+    const double det = G00 * A00 + G01 * A01 + G02 * A02;
+    if (on && !(det > 0.0)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
+    const double sc = kd * (0.125 * metric_scale<double>()) * rsqrt(det);
+    sM[le][0][g] = A00 * sc; sM[le][1][g] = A11 * sc; sM[le][2][g] = A22 * sc;
+    sM[le][3][g] = A01 * sc; sM[le][4][g] = A02 * sc; sM[le][5][g] = A12 * sc;
+  }
+  __syncwarp();
+  // scaled value products: ww(k, g) = (p/q)^2, p/q or 1
+  auto ww = [](int k, int gp) { return k == 1 ? kPoverQ : ((k == 0) == (gp == 0) ? kPoverQ * kPoverQ : 1.0); };
+  auto wv1 = [](int m, int gp) { return m == gp ? kPoverQ : 1.0; };
+  for (int u = g; u < 63; u += 8) {
+    double v = 0.0;
+    if (u < 27) {  // V_a[k1][k2]
+      const int a = u / 9, k1 = (u % 9) / 3, k2 = u % 3, d1 = a == 0 ? 1 : 0, d2 = a == 2 ? 1 : 2;
+      const double* M = sM[le][a];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int g0 = (i << d1) | (j << d2);
+          v = fma(ww(k1, i) * ww(k2, j), M[g0] + M[g0 | (1 << a)], v);
+        }
+    } else {  // W[n_a][m_b][k] of the pair pr
+      const int w = u - 27, pr = w / 12, i = (w % 12) / 6, j = (w % 6) / 3, k = w % 3;
+      const int a = pr == 2 ? 1 : 0, b = pr == 0 ? 1 : 2, c = 3 - a - b;
+      const double* M = sM[le][3 + pr];
+#pragma unroll
+      for (int gg = 0; gg < 8; ++gg)
+        v = fma(wv1(i, (gg >> a) & 1) * wv1(j, (gg >> b) & 1) * ww(k, (gg >> c) & 1), M[gg], v);
+    }
+    sV[le][u] = v;
+  }
+  __syncwarp();
+  if (!on) return;
+  // entry t of the packed upper triangle: m is the row, n the column
+  for (int t = g; t < 36; t += 8) {
+    int m = 0, rest = t;
+    while (rest >= 8 - m) {
+      rest -= 8 - m;
+      ++m;
+    }
+    const int n = m + rest;
+    double s = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int d1 = a == 0 ? 1 : 0, d2 = a == 2 ? 1 : 2;
+      const double v = sV[le][a * 9 + 3 * (((m >> d1) & 1) + ((n >> d1) & 1)) + ((m >> d2) & 1) + ((n >> d2) & 1)];
+      s += ((m ^ n) >> a) & 1 ? -v : v;
+    }
+#pragma unroll
+    for (int pr = 0; pr < 3; ++pr) {
+      const int a = pr == 2 ? 1 : 0, b = pr == 0 ? 1 : 2, c = 3 - a - b;
+      const int ma = (m >> a) & 1, mb = (m >> b) & 1, na = (n >> a) & 1, nb = (n >> b) & 1;
+      const int k = ((m >> c) & 1) + ((n >> c) & 1);
+      const double* W = sV[le] + 27 + pr * 12 + k;
+      const double t1 = W[na * 6 + mb * 3], t2 = W[ma * 6 + nb * 3];
+      s += (ma == nb ? t1 : -t1) + (na == mb ? t2 : -t2);
+    }
+    Kel[t * E + e] = s;
   }
 }
 
@@ -779,9 +1065,9 @@ int check_device_errors(cudaStream_t s, const char* fn, bool sync) {
   return GFE_OK;
 }
 
-// Workspace of the FP32-pipe precisions: the converted coordinates and, for float-float, behind
-// them at a 256-byte boundary the Gauss-point metrics (48 float-float numbers an element) and the
-// element matrices (36) of every element.  0 for FP64.
+// Workspace: for FP64 the element matrices (36 numbers an element); for the FP32-pipe precisions the
+// converted coordinates and, for float-float, behind them at a 256-byte boundary the Gauss-point metrics
+// (48 float-float numbers an element) and the element matrices (36) of every element.
 size_t regular_coords_bytes(int32_t nx, int32_t ny, int32_t nz, int precision) {
   const size_t n3 = 3ull * (nx + 1) * (ny + 1) * (nz + 1);
   if (precision == GFE_FP64) return 0;
@@ -791,6 +1077,7 @@ size_t regular_metric_entries(int32_t nx, int32_t ny, int32_t nz) {  // 48 per e
   return 48ull * (((size_t)nx * ny * nz + 31) & ~size_t(31));
 }
 size_t regular_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, int precision) {
+  if (precision == GFE_FP64) return 36ull * nx * ny * nz * sizeof(double);
   const size_t cb = regular_coords_bytes(nx, ny, nz, precision);
   if (precision != GFE_MIXED_DF) return cb;
   return cb + (regular_metric_entries(nx, ny, nz) + 36ull * nx * ny * nz) * sizeof(f2);
@@ -815,18 +1102,22 @@ void launch_elements_f2(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, cons
   laplace_contract_kernel<f2><<<cgrid, kContractThreads, 0, s>>>(nx, ny, nz, metrics, Kel, ez0, ez1);
 }
 
-void launch_gather_f2(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const void* ws, const int32_t* rp,
-                      double* values, float* values32, double* rhs, int32_t l0, int32_t l1) {
+// Rows of node layers [l0, l1) from the element matrices Kel.
+template <typename T>
+void launch_gather(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const T* Kel, const int32_t* rp, double* values,
+                   float* values32, double* rhs, int32_t l0, int32_t l1) {
   if (l1 <= l0) return;
   const long long rows = (long long)(l1 - l0) * (nx + 1) * (ny + 1);
   const int grid = (int)std::min<long long>((rows + kGatherWarps * 32 - 1) / (kGatherWarps * 32),
                                             8ll * gfe::sm_count());
-  const f2* Kel = reinterpret_cast<const f2*>(static_cast<const char*>(ws) +
-                                              regular_coords_bytes(nx, ny, nz, GFE_MIXED_DF)) +
-                  regular_metric_entries(nx, ny, nz);
-  const size_t smem = (size_t)kGatherWarps * kGatherStage * sizeof(f2);
-  cudaFuncSetAttribute((const void*)laplace_gather_kernel<f2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  laplace_gather_kernel<f2><<<grid, kGatherWarps * 32, smem, s>>>(nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
+  const size_t smem = (size_t)kGatherWarps * kGatherStage * sizeof(T);
+  cudaFuncSetAttribute((const void*)laplace_gather_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  laplace_gather_kernel<T><<<grid, kGatherWarps * 32, smem, s>>>(nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
+}
+
+const f2* element_matrices_f2(const void* ws, int32_t nx, int32_t ny, int32_t nz) {
+  return reinterpret_cast<const f2*>(static_cast<const char*>(ws) + regular_coords_bytes(nx, ny, nz, GFE_MIXED_DF)) +
+         regular_metric_entries(nx, ny, nz);
 }
 
 // Node layers [l0, l1) (l0 a multiple of kRZ).  ws: caller workspace of regular_workspace_bytes(),
@@ -850,7 +1141,7 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
   if (split || !ws) split_coords<T><<<4 * gfe::sm_count(), 256, 0, s>>>(n3, coords, ct);
   if constexpr (DF) {
     launch_elements_f2(s, nx, ny, nz, ct, kappa, base, std::max(l0 - 1, 0), std::min(l1, nz), err);
-    launch_gather_f2(s, nx, ny, nz, base, rp, values, values32, rhs, l0, l1);
+    launch_gather<f2>(s, nx, ny, nz, element_matrices_f2(base, nx, ny, nz), rp, values, values32, rhs, l0, l1);
   } else {
     const size_t smem = 2 * 36 * kRThreads * sizeof(typename StoreOf<T>::type);
     GFE_CUDA_TRY(cudaFuncSetAttribute((const void*)laplace_regular_kernel<T>,
@@ -864,10 +1155,26 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
   return GFE_OK;
 }
 
+// FP64 with a workspace, whole mesh: the element matrices once (the tiled kernel forms a third of them
+// twice in its halo), then the row gather: 90 x 77 x 101 elements 2.56 ms (colour kernel on general
+// connectivity) -> 1.27 ms, 4 x 4 x 4 0.71 -> 0.06 ms (eight colours, each one chain of 90 us).  Without a workspace, or for a slab, the row-owning tiled kernel, which needs no memory.
+// Below 64 elements an SM (two warps of four elements to each SM sub-partition, 8 lanes an element) the
+// kernel with eight lanes an element has the shorter chain.
 template <>
 int launch_regular<double>(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const double* coords,
                            const double* kappa, const int32_t* rp, double* values, float* values32, double* rhs,
-                           unsigned* err, void*, int32_t l0, int32_t l1, bool) {
+                           unsigned* err, void* ws, int32_t l0, int32_t l1, bool) {
+  if (ws && l0 == 0 && l1 == nz + 1) {
+    double* Kel = static_cast<double*>(ws);
+    const long long E = (long long)nx * ny * nz;
+    if (E <= 64ll * gfe::sm_count())
+      laplace_element64_small_kernel<<<(int)((E + 15) / 16), 128, 0, s>>>(nx, ny, nz, coords, kappa, Kel, err);
+    else
+      laplace_element64_kernel<<<(int)std::min<long long>((E + 127) / 128, 1 << 20), 128, 0, s>>>(nx, ny, nz, coords,
+                                                                                               kappa, Kel, err);
+    launch_gather<double>(s, nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
+    return GFE_OK;
+  }
   const size_t smem = 2 * 36 * kRThreads * sizeof(double);
   GFE_CUDA_TRY(cudaFuncSetAttribute((const void*)laplace_regular_kernel<double>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1129,7 +1436,7 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
       rc = launch_regular<float>(cs, nx, ny, nz, coords, kappa, row_ptr, values, nullptr, rhs, err, workspace,
                                  l0, l1, false);
     else {
-      launch_gather_f2(cs, nx, ny, nz, workspace, row_ptr, values, nullptr, rhs, l0, l1);
+      launch_gather<f2>(cs, nx, ny, nz, element_matrices_f2(workspace, nx, ny, nz), row_ptr, values, nullptr, rhs, l0, l1);
       rc = GFE_OK;
     }
     if (rc) return rc;

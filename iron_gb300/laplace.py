@@ -187,14 +187,20 @@ class LaplaceAssembly:
             return self.values
         if path == "regular" and self.regular is None:
             raise GfeError(-1, "the regular-mesh kernel needs Iron's regular generated mesh")
+        ws = None
         if path == "auto":
-            # FP64 element arithmetic is bound by GB300's FP64 pipe: the colour kernel computes each
-            # element once, while the tiled kernel recomputes its halo elements.  The FP32-pipe
-            # precisions are bound by memory traffic, which the tiled kernel minimises.
-            path = "general" if (prec == GFE_FP64 or self.regular is None) else "regular"
+            path = "general" if self.regular is None else "regular"
+            if path == "regular" and prec == GFE_FP64:
+                # element matrices in a workspace, then a row gather; without room for it (288 bytes an
+                # element) the colour kernel, which computes each element once as well
+                try:
+                    ws = self._regular_workspace(prec)
+                except torch.OutOfMemoryError:
+                    path = "general"
         if path == "regular":
             nx, ny, nz = self.regular
-            ws = self._regular_workspace(prec) if prec != GFE_FP64 else None
+            if prec != GFE_FP64:
+                ws = self._regular_workspace(prec)
             _lib.call("gfe_laplace_assemble_regular_ws", nx, ny, nz, _lib.ptr(self.coords), _lib.ptr(self.kappa),
                       _lib.ptr(self.row_ptr), _lib.ptr(self.values), _lib.ptr(v32), _lib.ptr(self.rhs), prec,
                       _lib.ptr(ws), _lib.stream_handle(stream))
@@ -267,8 +273,8 @@ class LaplaceAssembly:
 
     def _regular_workspace(self, prec: int) -> torch.Tensor:
         """Device workspace of the regular-mesh kernels for precision code `prec`, allocated once per
-        precision and kept (the float-float one also holds every element's Gauss-point metrics and
-        element matrix: 672 bytes an element)."""
+        precision and kept (FP64: every element's matrix, 288 bytes an element; float-float: also its
+        Gauss-point metrics, 672 bytes)."""
         cache = self.__dict__.setdefault("_ws_cache", {})
         if prec not in cache:
             nx, ny, nz = self.regular

@@ -65,3 +65,26 @@ def test_colour_by_colour_beyond_scratch(gfe_cuda, order, ne, precision):
     ov = oracle.laplace_assemble_scaled(3, [order] * 3, [order + 1] * 3, m.elem_nodes, m.coords, None, kap, rp, ci, 16)
     assert np.abs(v - ov).max() <= 1e-12 * np.abs(ov).max()
     assert torch.equal(A.values, A.assemble(precision))
+
+
+@pytest.mark.parametrize("ne", [(1, 1, 1), (4, 4, 4), (33, 1, 7), (16, 2, 1), (22, 21, 21), (22, 22, 21), (40, 17, 31)])
+@pytest.mark.parametrize("with_kappa", [True, False])
+def test_fp64_regular_mesh_forms(gfe_cuda, ne, with_kappa):
+    """FP64 on the regular mesh: eight lanes an element up to 64 elements an SM (22 x 21 x 21 lies below,
+    22 x 22 x 21 above on 152 SMs), a thread an element beyond, then the row gather, against the colour
+    kernel and the tiled kernel (sums of at most 8 element entries of FP64 arithmetic in other orders:
+    1e-13 relative to max|K|) and, on small meshes, the oracle."""
+    m = RegularMesh(ne, extent=(1.0, 0.7, 1.3))
+    m.jitter_interior(4)
+    kap = np.random.default_rng(5).uniform(0.1, 10.0, m.n_elements) if with_kappa else None
+    A = LaplaceAssembly.from_regular_mesh(m, kappa=kap)
+    A.rhs.fill_(1.0)
+    v = A.assemble("fp64", fp32_copy=True).clone()
+    assert float(A.rhs.abs().max()) == 0.0 and torch.equal(A.values32, v.float())
+    for path in ("general", "regular"):
+        w = A.assemble("fp64", path=path)
+        assert float((v - w).abs().max()) <= 1e-13 * float(w.abs().max()), path
+    if m.n_elements < 1000:
+        rp, ci = oracle.csr_structure(m.elem_nodes, m.n_nodes)
+        ov, _ = oracle.laplace_assemble(3, [1, 1, 1], [2, 2, 2], m.elem_nodes, m.coords, kap, rp, ci)
+        assert np.abs(v.cpu().numpy() - ov).max() <= 1e-13 * np.abs(ov).max()
