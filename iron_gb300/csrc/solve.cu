@@ -358,27 +358,57 @@ __global__ void norm2_kernel(int n, const double* __restrict__ v, double* red, S
 // caller's CSR (the values change with every assembly).
 constexpr int kSell = 32;
 
-template <typename TM>
+// Columns are stored as 16-bit offsets from the row where all of them fit (bandwidth up to 32,767: the 27-point
+// stencil up to 180^2 nodes a layer), else as 1-based 32-bit numbers: 6 or 8 bytes an FP32 entry.
+template <typename IT>
+struct SellIndex;
+template <>
+struct SellIndex<int32_t> {
+  static constexpr int32_t pad = 0;
+  static __device__ __forceinline__ int32_t of(int col1, int) { return col1; }
+  static __device__ __forceinline__ int column(int32_t c, int) { return c - 1; }
+};
+template <>
+struct SellIndex<int16_t> {
+  static constexpr int16_t pad = -32768;
+  static __device__ __forceinline__ int16_t of(int col1, int row) { return (int16_t)(col1 - 1 - row); }
+  static __device__ __forceinline__ int column(int16_t c, int row) { return row + c; }
+};
+
+template <typename TM, typename IT = int32_t>
 struct SellMatrix {
   const long long* sptr;  // [n_slices] first entry of each slice
   const int32_t* slen;    // [n_slices] entries of each slice (32 x its longest row)
-  const int32_t* col;     // 1-based column, 0 = padding
+  const IT* col;
   const TM* val;
 };
+// the copy in one of its two forms
+template <typename TM>
+struct SellCopy {
+  SellMatrix<TM, int16_t> near;
+  SellMatrix<TM, int32_t> far;
+  bool is_near = false;
+};
 
-__global__ void sell_slice_len(int n, const int32_t* __restrict__ rp, int32_t* __restrict__ slen) {
+// slice lengths, and the largest |column - row| of the matrix
+__global__ void sell_slice_len(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                               int32_t* __restrict__ slen, int* __restrict__ reach) {
   const int n_pad = (n + kSell - 1) / kSell * kSell;
+  int far = 0;
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n_pad; row += gridDim.x * blockDim.x) {
-    const int len = row < n ? __ldg(rp + row + 1) - __ldg(rp + row) : 0;
+    const int k0 = row < n ? __ldg(rp + row) - 1 : 0, len = row < n ? __ldg(rp + row + 1) - 1 - k0 : 0;
+    for (int k = 0; k < len; ++k) far = max(far, abs(__ldg(ci + k0 + k) - 1 - row));
     const int mx = __reduce_max_sync(0xffffffffu, len);
     if ((row & (kSell - 1)) == 0) slen[row / kSell] = mx * kSell;
   }
+  far = __reduce_max_sync(0xffffffffu, far);
+  if ((threadIdx.x & 31) == 0 && far > 0) atomicMax(reach, far);
 }
 
-template <typename TM>
+template <typename TM, typename IT>
 __global__ void sell_fill(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                           const TM* __restrict__ val, const long long* __restrict__ sptr,
-                          const int32_t* __restrict__ slen, int32_t* __restrict__ col, TM* __restrict__ sval) {
+                          const int32_t* __restrict__ slen, IT* __restrict__ col, TM* __restrict__ sval) {
   const int n_pad = (n + kSell - 1) / kSell * kSell;
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n_pad; row += gridDim.x * blockDim.x) {
     const int sl = row / kSell, lane = row & (kSell - 1);
@@ -387,7 +417,7 @@ __global__ void sell_fill(int n, const int32_t* __restrict__ rp, const int32_t* 
     const int k0 = row < n ? __ldg(rp + row) - 1 : 0, len = row < n ? __ldg(rp + row + 1) - 1 - k0 : 0;
     for (int k = 0; k < L; ++k) {
       const bool in = k < len;
-      col[base + (long long)k * kSell] = in ? __ldg(ci + k0 + k) : 0;
+      col[base + (long long)k * kSell] = in ? SellIndex<IT>::of(__ldg(ci + k0 + k), row) : SellIndex<IT>::pad;
       sval[base + (long long)k * kSell] = in ? __ldg(val + k0 + k) : TM(0);
     }
   }
@@ -395,11 +425,11 @@ __global__ void sell_fill(int n, const int32_t* __restrict__ rp, const int32_t* 
 
 // q = A p on free rows (0 on fixed rows) from the sliced-ELL copy, partial <p, q> and alpha as
 // cg_spmv; each row's entries in column order, kSellUnroll loads in flight a lane.
-constexpr int kSellUnroll = 8;
+constexpr int kSellUnroll = 9;  // three rounds for the 27-point stencil
 
-template <typename TM, typename TV>
+template <typename TM, typename TV, typename IT>
 __global__ void __launch_bounds__(kThreads)
-cg_spmv_sell(int n, SellMatrix<TM> A, const TV* __restrict__ p, TV* __restrict__ q,
+cg_spmv_sell(int n, SellMatrix<TM, IT> A, const TV* __restrict__ p, TV* __restrict__ q,
              const uint8_t* __restrict__ fixed, double* red, Scalars* sc) {
   if (sc->done) return;
   const int n_pad = (n + kSell - 1) / kSell * kSell;
@@ -412,17 +442,17 @@ cg_spmv_sell(int n, SellMatrix<TM> A, const TV* __restrict__ p, TV* __restrict__
     TV acc = TV(0);
     for (int k0 = 0; k0 < L; k0 += kSellUnroll) {
       TM v[kSellUnroll];
-      int c[kSellUnroll];
+      IT c[kSellUnroll];
 #pragma unroll
       for (int u = 0; u < kSellUnroll; ++u) {
         const bool in = k0 + u < L;
         const long long at = base + (long long)(k0 + u) * kSell;
         v[u] = in ? __ldcs(A.val + at) : TM(0);
-        c[u] = in ? __ldcs(A.col + at) : 0;
+        c[u] = in ? __ldcs(A.col + at) : SellIndex<IT>::pad;
       }
 #pragma unroll
       for (int u = 0; u < kSellUnroll; ++u)
-        if (c[u] > 0) acc += (TV)v[u] * p[c[u] - 1];
+        if (c[u] != SellIndex<IT>::pad) acc += (TV)v[u] * p[SellIndex<IT>::column(c[u], row)];
     }
     if (row < n) {
       if (fixed && fixed[row]) acc = TV(0);
@@ -443,41 +473,65 @@ cg_spmv_sell(int n, SellMatrix<TM> A, const TV* __restrict__ p, TV* __restrict__
   }
 }
 
+// scalars of the MINRES iteration (below)
+struct MinresScalars {
+  double gamma, gamma_old, delta, c, c_old, s, s_old, eta, tol;
+  double zs_prev, a1, a2, a3, ceta;
+  int done, pending, it, ticket1, ticket2, bad;
+};
+
+constexpr int kNodalBatch = 8;  // entries a lane loads at once in the MINRES products
+
+}  // namespace
+
+#include "krylov_resident.cuh"
+
+namespace {
+
 // Builds the sliced-ELL copy of (rp, ci, val) in two scratch allocations bufs[0], bufs[1] (the
 // caller frees both with scratch_free).  Synchronises the stream once (the copy's size).
 template <typename TM>
 int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaStream_t s, void* bufs[2],
-               SellMatrix<TM>* out) {
+               SellCopy<TM>* out) {
   using namespace gfe;
   bufs[0] = bufs[1] = nullptr;
   const long long n_slices = (n + kSell - 1) / kSell;
   char* head = nullptr;
-  const size_t head_bytes = ((sizeof(long long) * (n_slices + 1) + 255) & ~size_t(255)) +
-                            ((sizeof(int32_t) * n_slices + 255) & ~size_t(255));
-  int rc = scratch_alloc((void**)&head, head_bytes, s, "sliced-ELL offsets");
+  // offsets, the total and the reach, then the lengths
+  const size_t ptr_bytes = (sizeof(long long) * (n_slices + 2) + 255) & ~size_t(255);
+  int rc = scratch_alloc((void**)&head, ptr_bytes + sizeof(int32_t) * n_slices, s, "sliced-ELL offsets");
   if (rc) return rc;
   long long* sptr = (long long*)head;
-  int32_t* slen = (int32_t*)(head + ((sizeof(long long) * (n_slices + 1) + 255) & ~size_t(255)));
+  int32_t* slen = (int32_t*)(head + ptr_bytes);
   const int grid = 8 * sm_count();
-  sell_slice_len<<<grid, kThreads, 0, s>>>(n, rp, slen);
-  if ((rc = exclusive_scan(slen, n_slices, sptr, sptr + n_slices, s))) { scratch_free(head, s); return rc; }
-  long long total = 0;
-  cudaError_t e = cudaMemcpyAsync(&total, sptr + n_slices, sizeof(long long), cudaMemcpyDeviceToHost, s);
+  struct {
+    long long total, reach;
+  } size = {0, 0};
+  cudaError_t e = cudaMemsetAsync(sptr + n_slices, 0, sizeof(size), s);
+  if (e == cudaSuccess) {
+    sell_slice_len<<<grid, kThreads, 0, s>>>(n, rp, ci, slen, reinterpret_cast<int*>(sptr + n_slices + 1));
+    if ((rc = exclusive_scan(slen, n_slices, sptr, sptr + n_slices, s))) { scratch_free(head, s); return rc; }
+    e = cudaMemcpyAsync(&size, sptr + n_slices, sizeof(size), cudaMemcpyDeviceToHost, s);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) { scratch_free(head, s); return set_error(GFE_ERR_CUDA, "sliced-ELL size: %s", cudaGetErrorString(e)); }
+  out->is_near = size.reach <= 32767;
+  const size_t val_bytes = (sizeof(TM) * (size_t)size.total + 255) & ~size_t(255);
   char* body = nullptr;
-  const size_t col_bytes = ((sizeof(int32_t) * (size_t)total + 255) & ~size_t(255));
-  if ((rc = scratch_alloc((void**)&body, col_bytes + sizeof(TM) * (size_t)total + 256, s, "sliced-ELL copy"))) {
+  if ((rc = scratch_alloc((void**)&body, val_bytes + (out->is_near ? 2 : 4) * (size_t)size.total + 256, s, "sliced-ELL copy"))) {
     scratch_free(head, s);
     return rc;
   }
-  int32_t* col = (int32_t*)body;
-  TM* sval = (TM*)(body + col_bytes);
-  sell_fill<TM><<<grid, kThreads, 0, s>>>(n, rp, ci, val, sptr, slen, col, sval);
-  out->sptr = sptr;
-  out->slen = slen;
-  out->col = col;
-  out->val = sval;
+  TM* sval = (TM*)body;
+  if (out->is_near) {
+    int16_t* col = (int16_t*)(body + val_bytes);
+    sell_fill<TM, int16_t><<<grid, kThreads, 0, s>>>(n, rp, ci, val, sptr, slen, col, sval);
+    out->near = {sptr, slen, col, sval};
+  } else {
+    int32_t* col = (int32_t*)(body + val_bytes);
+    sell_fill<TM, int32_t><<<grid, kThreads, 0, s>>>(n, rp, ci, val, sptr, slen, col, sval);
+    out->far = {sptr, slen, col, sval};
+  }
   bufs[0] = head;
   bufs[1] = body;
   return GFE_OK;
@@ -489,6 +543,7 @@ int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaS
 // slower); FP64 with 2 lanes a row, 14 entries a lane and two rows a group (152 us, 216 us for one
 // thread a row with the per-row loop; the shuffle of the 2-lane sum is one FP64 add a row).
 // Longer FP32 rows keep the per-row loop with 16 or 32 lanes; longer FP64 rows one thread a row.
+constexpr long long kResidentBytes = 100ll << 20;  // matrix of a resident solve: within the 129 MB L2
 constexpr int kSpmvShort32 = -1;
 constexpr int kSpmvShort64 = -2;
 
@@ -535,13 +590,14 @@ void residual64(bool short_rows, int grid, cudaStream_t s, int n, const int32_t*
 template <typename TM, typename TV, typename TX>
 int run_cg(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, const TM* val, const uint8_t* fixed,
            const TV* dinv, TX* x, TV* r, TV* z, TV* p, TV* q, double* red, double* red2, Scalars* sc,
-           Scalars* sc_host, int lpr, int grid, int max_iters, int chunk, const SellMatrix<TM>* sell = nullptr) {
+           Scalars* sc_host, int lpr, int grid, int max_iters, int chunk, const SellCopy<TM>* sell = nullptr) {
   int launched = 0;
   while (launched < max_iters) {
     int k = chunk < max_iters - launched ? chunk : max_iters - launched;
     for (int i = 0; i < k; ++i) {
       void* prof = gfe::stage_begin(GFE_STAGE_SPMV, s);
-      if (sell) cg_spmv_sell<TM, TV><<<grid, kThreads, 0, s>>>(n, *sell, p, q, fixed, red, sc);
+      if (sell && sell->is_near) cg_spmv_sell<TM, TV, int16_t><<<grid, kThreads, 0, s>>>(n, sell->near, p, q, fixed, red, sc);
+      else if (sell) cg_spmv_sell<TM, TV, int32_t><<<grid, kThreads, 0, s>>>(n, sell->far, p, q, fixed, red, sc);
       else launch_spmv<TM, TV>(lpr, grid, s, n, rp, ci, val, p, q, fixed, red, sc);
       gfe::stage_end(GFE_STAGE_SPMV, prof, s, 1);
       cg_update<TX, TV><<<grid, kThreads, 0, s>>>(n, x, r, z, p, q, dinv, red, red2, sc);
@@ -551,6 +607,44 @@ int run_cg(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, const TM
     GFE_CUDA_TRY(cudaGetLastError());
     GFE_CUDA_TRY(cudaMemcpyAsync(sc_host, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
     GFE_CUDA_TRY(cudaStreamSynchronize(s));
+    if (sc_host->done) break;
+  }
+  return GFE_OK;
+}
+
+// CG iterations in resident kernels of at most kResidentIters each, until convergence; *ran is false when
+// the first launch was not possible.
+constexpr int kResidentIters = 200;
+
+template <typename TM, typename TV>
+int run_cg_resident(cudaStream_t s, int n, const SellCopy<TM>& A, const uint8_t* fixed, const TV* dinv, TV* x, TV* r,
+                    TV* z, TV* p, TV* q, Scalars* sc, Scalars* sc_host, ResBarrier* bar, int max_iters, bool fresh,
+                    bool* ran) {
+  const int slices = (n + kSell - 1) / kSell;
+  const int grid = std::min({gfe::sm_count(), kResMaxGrid, (slices + kCgWorkers - 1) / kCgWorkers});
+  const int rounds = ((slices + grid - 1) / grid + kCgWorkers - 1) / kCgWorkers;  // slices a warp
+  *ran = true;
+  for (int done = 0; done < max_iters;) {
+    const int k = std::min(kResidentIters, max_iters - done);
+    GFE_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(ResBarrier), s));
+    void* prof = gfe::stage_begin(GFE_STAGE_SPMV, s);
+#define GFE_CG_RESIDENT(R)                                                                                            \
+  (A.is_near ? launch_resident(cg_resident<TM, TV, int16_t, R>, grid, kCgThreads, s, n, A.near, x, r, z, p, q, dinv, fixed, \
+                               sc, bar, k, fresh)                                                                     \
+             : launch_resident(cg_resident<TM, TV, int32_t, R>, grid, kCgThreads, s, n, A.far, x, r, z, p, q, dinv, fixed, \
+                               sc, bar, k, fresh))
+    const bool ok = rounds == 1 ? GFE_CG_RESIDENT(1) : (rounds == 2 ? GFE_CG_RESIDENT(2) : (rounds == 3 && GFE_CG_RESIDENT(3)));
+#undef GFE_CG_RESIDENT
+    gfe::stage_end(GFE_STAGE_SPMV, prof, s, 1);
+    if (!ok) {
+      *ran = done > 0;
+      return done > 0 ? gfe::set_error(GFE_ERR_CUDA, "launch of the resident CG kernel failed") : GFE_OK;
+    }
+    fresh = false;
+    done += k;
+    GFE_CUDA_TRY(cudaMemcpyAsync(sc_host, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
+    GFE_CUDA_TRY(cudaStreamSynchronize(s));
+    if (sc_host->bad == 2) return gfe::set_error(GFE_ERR_TIMEOUT, "a wait between the CTAs of the CG kernel ran out");
     if (sc_host->done) break;
   }
   return GFE_OK;
@@ -604,15 +698,19 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
   // Laplace: 104 -> 91 us a product, 103 -> 93 ms a solve); the FP64 product, bound by FP64 work
   // as much as by its loads, gained nothing from it and keeps the batched CSR form
   const bool use_sell = precision == GFE_MIXED && (double)(nnz1 - 1) / n <= 32.0 && n >= 4 * kSell;
+  // short rows and a matrix that stays in L2: the iterations run in resident kernels on the sliced-ELL copy
+  // (64^3, 59 MB in FP32: a solve takes 6.5 ms instead of 16.4; 128^3, 460 MB, is bound by HBM, where the launched
+  // form already runs at the bandwidth)
+  bool resident = short_rows && (long long)(nnz1 - 1) * (precision == GFE_FP64 ? 12 : 8) <= kResidentBytes;
   void* sell_bufs[2] = {nullptr, nullptr};
 
   // scratch: dinv, r64, then vector set (FP64 or FP32) and an FP32 copy of dinv
   const size_t vbytes = precision == GFE_FP64 ? sizeof(double) : sizeof(float);
   char* buf = nullptr;
   const size_t nb = (size_t)n;
-  // eleven carved pieces, each rounded up to 256 bytes
+  // twelve carved pieces, each rounded up to 256 bytes
   const size_t bytes = nb * sizeof(double) * 2 + nb * vbytes * 6 + sizeof(double) * grid * 2 + sizeof(Scalars) +
-                       12 * 256;
+                       sizeof(ResBarrier) + 13 * 256;
   int rc = scratch_alloc((void**)&buf, bytes, s, "CG vectors");
   if (rc) return rc;
   auto carve = [&](size_t b) {
@@ -632,6 +730,7 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
   double* red = (double*)carve(sizeof(double) * grid);
   double* red2 = (double*)carve(sizeof(double) * grid);
   Scalars* sc = (Scalars*)carve(sizeof(Scalars));
+  ResBarrier* bar = (ResBarrier*)carve(sizeof(ResBarrier));
   Scalars sh{};
   double b2 = 0.0, r2 = 0.0;
   int total_it = 0;
@@ -655,12 +754,21 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
     // and, while the true residual is above it, replaces the recurrence residual by the true one
     // and continues along the same search direction (a reliable update).
     double r2_start = b2;
+    SellCopy<double> sell{};
+    if (resident && build_sell<double>(n, row_ptr, col_idx, values, s, sell_bufs, &sell)) resident = false;
     for (int round = 0; round < 4 && rc == GFE_OK; ++round) {
       cg_start<double, double><<<grid, kThreads, 0, s>>>(n, r64, dinv, r, z, p, x, false, round > 0, red, red2, sc,
                                                          0.25 * rtol * rtol * b2 / r2_start);
-      if (round > 0) cg_direction<double><<<grid, kThreads, 0, s>>>(n, p, z, sc);
-      rc = run_cg<double, double, double>(s, n, row_ptr, col_idx, values, fixed, dinv, x, r, z, p, q, red, red2, sc,
-                                          &sh, lpr, grid, max_iters - total_it, chunk);
+      bool ran = false;
+      if (resident)
+        rc = run_cg_resident<double, double>(s, n, sell, fixed, dinv, x, r, z, p, q, sc, &sh, bar,
+                                             max_iters - total_it, round == 0, &ran);
+      if (!ran) {
+        resident = false;
+        if (round > 0) cg_direction<double><<<grid, kThreads, 0, s>>>(n, p, z, sc);
+        rc = run_cg<double, double, double>(s, n, row_ptr, col_idx, values, fixed, dinv, x, r, z, p, q, red, red2, sc,
+                                            &sh, lpr, grid, max_iters - total_it, chunk);
+      }
       total_it += sh.it;
       if (rc || sh.bad || total_it >= max_iters) break;
       residual64(short_rows, grid, s, n, row_ptr, col_idx, values, f, fixed, x, r64);
@@ -681,8 +789,8 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
     // iterations with the best restart tolerance, 1e-5).  Reductions of 1e-1 to 1e-3 per update
     // all take 727-742 iterations; 1e-3 needs the fewest updates.
     const double inner_rtol = 1e-3;
-    SellMatrix<float> sell{};
-    if (use_sell) rc = build_sell<float>(n, row_ptr, col_idx, values32, s, sell_bufs, &sell);
+    SellCopy<float> sell{};
+    if (use_sell || resident) rc = build_sell<float>(n, row_ptr, col_idx, values32, s, sell_bufs, &sell);
     for (int outer = 0; outer < 200 && rc == GFE_OK; ++outer) {
       if (outer > 0) {
         residual64(short_rows, grid, s, n, row_ptr, col_idx, values, f, fixed, x, r64);
@@ -694,9 +802,16 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
       }
       cg_start<float, float><<<grid, kThreads, 0, s>>>(n, r64, dinv, r, z, p, d, true, outer > 0, red, red2, sc,
                                                        inner_rtol * inner_rtol);
-      if (outer > 0) cg_direction<float><<<grid, kThreads, 0, s>>>(n, p, z, sc);
-      rc = run_cg<float, float, float>(s, n, row_ptr, col_idx, values32, fixed, dinv32, d, r, z, p, q, red, red2, sc,
-                                       &sh, lpr, grid, max_iters - total_it, chunk, use_sell ? &sell : nullptr);
+      bool ran = false;
+      if (resident)
+        rc = run_cg_resident<float, float>(s, n, sell, fixed, dinv32, d, r, z, p, q, sc, &sh, bar,
+                                           max_iters - total_it, outer == 0, &ran);
+      if (!ran) {
+        resident = false;
+        if (outer > 0) cg_direction<float><<<grid, kThreads, 0, s>>>(n, p, z, sc);
+        rc = run_cg<float, float, float>(s, n, row_ptr, col_idx, values32, fixed, dinv32, d, r, z, p, q, red, red2, sc,
+                                         &sh, lpr, grid, max_iters - total_it, chunk, use_sell ? &sell : nullptr);
+      }
       total_it += sh.it;
       if (sh.bad) break;
       add_correction<<<grid, kThreads, 0, s>>>(n, x, d, fixed);
@@ -841,14 +956,6 @@ extern "C" int gfe_cg_status(int32_t n, void* workspace, gfe_cg_state* state_hos
 // buffers rotate between two copies on the host side; the kernels return at once after `done`, so
 // iterations are launched in chunks exactly like the CG.
 namespace {
-
-struct MinresScalars {
-  double gamma, gamma_old, delta, c, c_old, s, s_old, eta, tol;
-  double zs_prev, a1, a2, a3, ceta;
-  int done, pending, it, ticket1, ticket2, bad;
-};
-
-constexpr int kNodalBatch = 8;  // entries a lane loads at once in the MINRES products
 
 // (A): pending w / x update of the previous iteration, then q = A z / gamma (0 on fixed rows) and
 // delta = <q, z / gamma>.
@@ -1212,6 +1319,49 @@ int run_minres(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, cons
   return GFE_OK;
 }
 
+// MINRES iterations in resident kernels, as run_cg_resident; vectors started as for run_minres.
+template <typename TM, typename TV, typename TX>
+int run_minres_resident(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, const TM* val,
+                        const uint8_t* fixed, const TV* minv, TX* x, TV* const V[2], TV* const Z[2], TV* const W[2],
+                        MinresScalars* sc, MinresScalars* sc_host, ResBarrier* bar, int max_iters,
+                        NodalRows nodal, bool* ran) {
+  const bool nodes = nodal.n_node > 0 && nodal.nc == 3;
+  const int n_node = nodes ? nodal.n_node : 0, groups = nodes ? n - 2 * n_node : n, sms = gfe::sm_count();
+  // lanes a group: FP64 8 (the shuffle sums run on the FP64 pipe); FP32 a warp, or half a warp where that lets
+  // one pass of a CTA cover its groups.  At least eight groups a CTA: below that the barriers cost more
+  const int grid = std::min({sms, kResMaxGrid, (groups + 7) / 8});
+  const long long units = nodes ? n_node + 2ll * (groups - n_node) : groups;
+  const int share = (int)((units + grid - 1) / grid);  // groups a CTA at most
+  const int lpr = std::is_same<TV, double>::value ? 8 : (share > kMinresWorkers && share <= 2 * kMinresWorkers ? 16 : 32);
+  *ran = share * (nodes ? 3 : 1) <= kMinresWorkers * 32;  // a thread a row
+  if (!*ran) return GFE_OK;
+  int j = 1;
+  while (j <= max_iters) {
+    const int k = std::min(kResidentIters, max_iters - j + 1);
+    GFE_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(ResBarrier), s));
+    void* prof = gfe::stage_begin(GFE_STAGE_SPMV, s);
+    bool ok;
+#define GFE_MINRES_RESIDENT(L, C)                                                                                     \
+  launch_resident(minres_resident<TM, TV, TX, L, C>, grid, kMinresThreads, s, n, n_node, rp, ci, val, fixed, minv, x, \
+                  V[0], V[1], Z[0], Z[1], W[0], W[1], sc, bar, j, k)
+    if constexpr (std::is_same<TV, double>::value) ok = GFE_MINRES_RESIDENT(8, 1);
+    else if (nodes) ok = lpr == 16 ? GFE_MINRES_RESIDENT(16, 3) : GFE_MINRES_RESIDENT(32, 3);
+    else ok = lpr == 16 ? GFE_MINRES_RESIDENT(16, 1) : GFE_MINRES_RESIDENT(32, 1);
+#undef GFE_MINRES_RESIDENT
+    gfe::stage_end(GFE_STAGE_SPMV, prof, s, 1);
+    if (!ok) {
+      *ran = j > 1;
+      return j > 1 ? gfe::set_error(GFE_ERR_CUDA, "launch of the resident MINRES kernel failed") : GFE_OK;
+    }
+    j += k;
+    GFE_CUDA_TRY(cudaMemcpyAsync(sc_host, sc, sizeof(MinresScalars), cudaMemcpyDeviceToHost, s));
+    GFE_CUDA_TRY(cudaStreamSynchronize(s));
+    if (sc_host->bad == 2) return gfe::set_error(GFE_ERR_TIMEOUT, "a wait between the CTAs of the MINRES kernel ran out");
+    if (sc_host->done) break;
+  }
+  return GFE_OK;
+}
+
 // lanes per row of the MINRES SpMV: long rows (the u-p tangent has ~200 entries a row) use 8 lanes
 // in FP64, so the shuffle reduction adds little to the FP64-pipe work, and a full warp in FP32
 int minres_lpr(double avg, bool fp64) {
@@ -1269,10 +1419,15 @@ int minres_solve(const char* fn, int32_t n, int32_t n_node, int32_t n_comp, cons
   const int chunk = 50;
   const size_t nb = (size_t)n, vbytes = fp64 ? sizeof(double) : sizeof(float);
   // pieces: m64, m32, r64, eight vectors of the working type (V0 V1 Z0 Z1 W0 W1 q d), the block
-  // partials, the MINRES scalars, a Scalars block for the norm kernel and the norm result
-  const int pieces = 15;
+  // partials, the MINRES scalars, a Scalars block for the norm kernel, the norm result, the nodal flag and
+  // the grid barrier
+  const int pieces = 16;
   const size_t bytes = nb * sizeof(double) * 2 + nb * sizeof(float) + nb * vbytes * 8 + sizeof(double) * grid +
-                       sizeof(MinresScalars) + sizeof(Scalars) + sizeof(double) + sizeof(int) + (pieces + 2) * 256;
+                       sizeof(MinresScalars) + sizeof(Scalars) + sizeof(double) + sizeof(int) + sizeof(ResBarrier) +
+                       (pieces + 2) * 256;
+  // long rows and a matrix that stays in L2: resident kernels (a Newton solve at 8^3: 22.5 ms instead of 55; at
+  // 32^3 the matrix, 1.2 GB in FP32, streams from HBM)
+  bool resident = (double)(nnz1 - 1) / n >= 48.0 && (long long)(nnz1 - 1) * (fp64 ? 12 : 8) <= kResidentBytes;
   char* buf = nullptr;
   int rc = scratch_alloc((void**)&buf, bytes, s, "MINRES vectors");
   if (rc) return rc;
@@ -1292,6 +1447,7 @@ int minres_solve(const char* fn, int32_t n, int32_t n_node, int32_t n_comp, cons
   Scalars* nsc = (Scalars*)carve(sizeof(Scalars));
   double* r2dev = (double*)carve(sizeof(double));
   int* nodal_ok = (int*)carve(sizeof(int));
+  ResBarrier* bar = (ResBarrier*)carve(sizeof(ResBarrier));
   MinresScalars sh{};
   double b2 = 0.0, r2 = 0.0;
   int total_it = 0;
@@ -1343,8 +1499,15 @@ int minres_solve(const char* fn, int32_t n, int32_t n_node, int32_t n_comp, cons
     for (int round = 0; round < 6 && rc == GFE_OK; ++round) {
       minres_start<double, double><<<grid, kThreads, 0, s>>>(n, r64, m64, V[1], V[0], Z[1], W[0], W[1], x, false, red,
                                                              sc, 0.7 * rtol * std::sqrt(b2 / r2));
-      rc = run_minres<double, double, double>(s, n, row_ptr, col_idx, values, fixed, m64, x, V, Z, W, q, red, sc, &sh,
-                                              lpr, grid, max_iters - total_it, chunk, nodal);
+      bool ran = false;
+      if (resident)
+        rc = run_minres_resident<double, double, double>(s, n, row_ptr, col_idx, values, fixed, m64, x, V, Z, W, sc,
+                                                         &sh, bar, max_iters - total_it, nodal, &ran);
+      if (!ran) {
+        resident = false;
+        rc = run_minres<double, double, double>(s, n, row_ptr, col_idx, values, fixed, m64, x, V, Z, W, q, red, sc, &sh,
+                                                lpr, grid, max_iters - total_it, chunk, nodal);
+      }
       total_it += sh.it;
       if (rc) break;
       rc = true_residual();
@@ -1364,8 +1527,15 @@ int minres_solve(const char* fn, int32_t n, int32_t n_node, int32_t n_comp, cons
       const double inner_rtol = std::max(0.7 * rtol * std::sqrt(b2 / r2), 5e-6);
       minres_start<float, float><<<grid, kThreads, 0, s>>>(n, r64, m32, V[1], V[0], Z[1], W[0], W[1], d, true, red, sc,
                                                            inner_rtol);
-      rc = run_minres<float, float, float>(s, n, row_ptr, col_idx, values32, fixed, m32, d, V, Z, W, q, red, sc, &sh,
-                                           lpr, grid, max_iters - total_it, chunk, nodal);
+      bool ran = false;
+      if (resident)
+        rc = run_minres_resident<float, float, float>(s, n, row_ptr, col_idx, values32, fixed, m32, d, V, Z, W, sc,
+                                                      &sh, bar, max_iters - total_it, nodal, &ran);
+      if (!ran) {
+        resident = false;
+        rc = run_minres<float, float, float>(s, n, row_ptr, col_idx, values32, fixed, m32, d, V, Z, W, q, red, sc, &sh,
+                                             lpr, grid, max_iters - total_it, chunk, nodal);
+      }
       total_it += sh.it;
       if (rc) break;
       add_correction<<<grid, kThreads, 0, s>>>(n, x, d, fixed);
