@@ -13,6 +13,7 @@
 // positions z1, z2, z3 over the n_q2 quadratic nodes followed by the pressure over the n_lin
 // linear (corner) nodes; the geometric field x is [3][n_q2].  Element DOF order: 27 z1, 27 z2,
 // 27 z3, 8 p (Iron's element parameter order, local nodes xi1 fastest).
+#include <climits>
 #include <mutex>
 #include <type_traits>
 
@@ -177,10 +178,13 @@ __global__ void mr_slot_kernel(const int32_t* __restrict__ elems, int32_t count,
 // slot-map row are read once, contiguously.  Node incidence: for node k (quadratic nodes 0..nq2-1,
 // then linear nodes nq2 + l) up to kMaxInc entries (e * 64 + local index; local 0..26 quadratic,
 // 27..34 linear), sorted by element.
+// FP32 element matrices lie kKelF floats apart (a 16-byte multiple: they leave by TMA), FP64 ones 89 * 89.
+constexpr int kKelF = (ND * ND + 3) / 4 * 4;
+template <typename TS>
+constexpr int kKelStride = std::is_same<TS, float>::value ? kKelF : ND * ND;
 constexpr int kMaxInc = 16;       // elements around one node (8 on a hexahedral grid)
 constexpr int kRowWarps = 8;      // warps (rows in flight) per CTA of mr_row_gather_kernel
 constexpr int kMaxRowLen = 512;   // entries of one Jacobian row (at most 402 on a regular Q2/Q1 grid)
-constexpr int kGatherGroup = 4;   // element rows whose loads are in flight together
 
 __global__ void mr_incidence_fill(const int32_t* __restrict__ elems, int32_t count, const int32_t* __restrict__ eq2,
                                   const int32_t* __restrict__ elin, int32_t nq2, int32_t* __restrict__ cnt,
@@ -218,77 +222,114 @@ __global__ void mr_incidence_sort(int32_t n_nodes, const int32_t* __restrict__ c
 // row mh * 27 + node index; pressure rows local row 81 + corner index.  The pressure-pressure block
 // is not assembled (zero in Iron's matrix).  Every entry of every row is written, so the values
 // need no zeroing first.  FP32 element matrices are summed in FP32 (at most 8 terms an entry,
-// against the 5e-6 of their own contraction) and widened exactly with integer operations
-// (f32_to_f64_exact): the FP64 additions and conversions kept the FP64 pipe 77 % busy and bounded
+// against the 5e-6 of their own contraction) and widened exactly with integer operations: the FP64 additions and conversions kept the FP64 pipe 77 % busy and bounded
 // the kernel.
+//
+// DRAM bounds it (element matrices and slot map read once, values written once); the instructions come second, so a
+// row takes its elements four, two or one at a time (a node has 1, 2, 4 or 8), 32-bit offsets and 16-byte stores, which
+// the row's place in shared memory is shifted for: 794 -> 705 us at 32^3 (3.4 GB).  Additions without a branch to a
+// spare entry, or that skip absent elements of a fixed group of four, were slower (820, 768 us).
+__device__ __forceinline__ double widen(float f) {  // as f32_to_f64_exact, with one rare branch: 734 -> 705 us
+  const unsigned u = __float_as_uint(f), t = u & 0x7fffffffu;
+  if (t - 0x00800000u >= 0x7f000000u && t != 0u) return (double)f;  // subnormal, infinite or NaN
+  const unsigned hi = t == 0u ? 0u : (t >> 3) + (896u << 20);
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double f) { return f; }
+
+template <int G, typename TS>
+__device__ __forceinline__ bool add_element_rows(TS* B, int r0, int len, int list, int i, int mh,
+                                                 const TS* __restrict__ Kel, const int32_t* __restrict__ slots) {
+  const int lane = threadIdx.x & 31;
+  int at[G][3];  // place in the row; INT_MIN: nothing to add, else outside it: a wrong slot
+  TS val[G][3];
+  bool ok = true;
+  // every load of the group is issued before its additions, which then run in ascending element order
+#pragma unroll
+  for (int u = 0; u < G; ++u) {
+    const int packed = __shfl_sync(0xffffffffu, list, i + u);
+    const int e = packed >> 6, loc = packed & 63;
+    const int lr = loc < NQ ? mh * NQ + loc : 81 + loc - NQ;
+    const int32_t* srow = slots + ((size_t)e * (ND * ND) + lr * ND) + lane;
+    const TS* krow = Kel + ((size_t)e * kKelStride<TS> + lr * ND) + lane;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const bool in = j < 2 || lane + 64 < (lr >= 81 ? 81 : ND);
+      at[u][j] = in ? __ldg(srow + 32 * j) - r0 : INT_MIN;
+      val[u][j] = in ? __ldg(krow + 32 * j) : TS(0);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < G; ++u) {
+    // an element row's columns are distinct: its loads need not wait for its stores
+    bool inside[3];
+    TS sum[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      inside[j] = (unsigned)at[u][j] < (unsigned)len;
+      ok &= inside[j] || at[u][j] == INT_MIN;
+      sum[j] = (inside[j] ? B[at[u][j]] : TS(0)) + val[u][j];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (inside[j]) B[at[u][j]] = sum[j];
+    __syncwarp();  // the next element may add to the same entries
+  }
+  return ok;
+}
+
 template <typename TS>
-__global__ void __launch_bounds__(kRowWarps * 32)
+__global__ void __launch_bounds__(kRowWarps * 32, sizeof(TS) == 4 ? 5 : 4)
 mr_row_gather_kernel(int32_t nq2, int32_t nlin, const int32_t* __restrict__ cnt, const int32_t* __restrict__ list,
                      const TS* __restrict__ Kel, const int32_t* __restrict__ slots, const int32_t* __restrict__ rp,
-                     double* __restrict__ values, float* __restrict__ values32, unsigned* err) {
-  __shared__ TS buf[kRowWarps][kMaxRowLen];
+                     double* __restrict__ values, unsigned* err) {
+  __shared__ __align__(16) TS buf[kRowWarps][kMaxRowLen + 4];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  TS* B = buf[w];
-  const long long n_rows = 3ll * nq2 + nlin;
-  for (long long row = (long long)blockIdx.x * kRowWarps + w; row < n_rows; row += (long long)gridDim.x * kRowWarps) {
-    int node, mh;
-    if (row < 3ll * nq2) {
-      mh = (int)(row / nq2);
-      node = (int)(row - (long long)mh * nq2);
-    } else {
-      mh = 0;
-      node = nq2 + (int)(row - 3ll * nq2);
-    }
-    const long long r0 = __ldg(rp + row) - 1;
-    const int len = (int)(__ldg(rp + row + 1) - 1 - r0);
-    if (len > kMaxRowLen) {
-      if (lane == 0) gfe_raise(err, GFE_DEVERR_SLOT);
+  const int n_rows = 3 * nq2 + nlin, step = gridDim.x * kRowWarps;
+  // what a row needs to start (its bounds and its node's elements, a lane an entry), loaded one row ahead
+  struct Head {
+    int mh, r0, r1, m, list;
+  };
+  static_assert(kMaxInc <= 32, "a lane an element");
+  auto head = [&](int row) {
+    Head h;
+    h.mh = row < 3 * nq2 ? (row >= nq2) + (row >= 2 * nq2) : 0;
+    const int node = row < 3 * nq2 ? row - h.mh * nq2 : nq2 + row - 3 * nq2;
+    h.r0 = __ldg(rp + row) - 1;
+    h.r1 = __ldg(rp + row + 1) - 1;
+    h.m = min(__ldg(cnt + node), kMaxInc);
+    h.list = lane < kMaxInc ? __ldg(list + (size_t)node * kMaxInc + lane) : 0;
+    return h;
+  };
+  Head next{};
+  if (blockIdx.x * kRowWarps + w < n_rows) next = head(blockIdx.x * kRowWarps + w);
+  for (int row = blockIdx.x * kRowWarps + w; row < n_rows; row += step) {
+    const Head h = next;
+    if (row + step < n_rows) next = head(row + step);
+    const int r0 = h.r0, len = h.r1 - r0, m = h.m, mh = h.mh;
+    bool ok = len <= kMaxRowLen;
+    if (!ok) {
+      gfe_raise(err, GFE_DEVERR_SLOT);
       continue;
     }
-    for (int j = lane; j < len; j += 32) B[j] = TS(0);
+    // entry o of the row is B[o]; B - shift is 16-byte aligned and so is its place in `values`
+    double* out = values + r0;
+    const int shift = (int)((reinterpret_cast<uintptr_t>(out) >> 3) & 1);
+    TS* B = buf[w] + shift;
+    for (int j = lane * 2; j < len + shift; j += 64) buf[w][j] = buf[w][j + 1] = TS(0);
     __syncwarp();
-    const int m = min(__ldg(cnt + node), kMaxInc);
-    const int32_t* L = list + (size_t)node * kMaxInc;
-    // groups of kGatherGroup element rows: every slot and value load of a group is issued before
-    // the group's additions, which then run in ascending element order
-    for (int i0 = 0; i0 < m; i0 += kGatherGroup) {
-      int pos[kGatherGroup][3];
-      TS val[kGatherGroup][3];
+    int i = 0;
+    for (; m - i >= 4; i += 4) ok &= add_element_rows<4>(B, r0, len, h.list, i, mh, Kel, slots);
+    if (m & 2) ok &= add_element_rows<2>(B, r0, len, h.list, i, mh, Kel, slots);
+    if (m & 1) ok &= add_element_rows<1>(B, r0, len, h.list, m - 1, mh, Kel, slots);
+    if (!ok) gfe_raise(err, GFE_DEVERR_SLOT);
+    for (int j = lane * 2 - shift; j < len; j += 64) {
+      double v[2];
 #pragma unroll
-      for (int u = 0; u < kGatherGroup; ++u) {
-        const int i = i0 + u;
-        const int32_t packed = i < m ? __ldg(L + i) : -1;
-        const int e = packed >> 6, loc = packed & 63;
-        const int lr = loc < NQ ? mh * NQ + loc : 81 + loc - NQ;
-        const size_t base = ((size_t)(packed < 0 ? 0 : e) * ND + lr) * ND;
-        const int cmax = packed < 0 ? 0 : (lr >= 81 ? 81 : ND);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int c = lane + 32 * j;
-          pos[u][j] = -2;  // nothing to add
-          val[u][j] = TS(0);
-          if (c < cmax) {
-            pos[u][j] = __ldg(slots + base + c);
-            val[u][j] = __ldg(Kel + base + c);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kGatherGroup; ++u) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const long long o = (long long)pos[u][j] - r0;
-          if (pos[u][j] >= 0 && o >= 0 && o < len) B[o] += val[u][j];
-          else if (pos[u][j] != -2) gfe_raise(err, GFE_DEVERR_SLOT);
-        }
-        __syncwarp();  // the next element may add to the same entries
-      }
-    }
-    for (int j = lane; j < len; j += 32) {
-      const TS v = B[j];
-      if constexpr (std::is_same<TS, float>::value) values[r0 + j] = f32_to_f64_exact(v);
-      else values[r0 + j] = v;
-      if (values32) values32[r0 + j] = (float)v;
+      for (int k = 0; k < 2; ++k) v[k] = widen(B[j + k]);
+      if (j >= 0 && j + 1 < len) *reinterpret_cast<double2*>(out + j) = make_double2(v[0], v[1]);
+      else if (j >= 0) out[j] = v[0];
+      else if (len > 0) out[0] = v[1];
     }
     __syncwarp();
   }
@@ -296,7 +337,7 @@ mr_row_gather_kernel(int32_t nq2, int32_t nlin, const int32_t* __restrict__ cnt,
 
 __global__ void widen_element_matrices(const float* __restrict__ src, size_t n, double* __restrict__ dst) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = (double)src[i];
+    dst[i] = (double)src[i / (ND * ND) * kKelF + i % (ND * ND)];
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -489,7 +530,7 @@ __device__ __forceinline__ void point_dP(const GPInT<float>& in, int seed, float
 // the u-p / p-u blocks.  The work is split in two kernels:
 //  * mr_gp_kernel, one thread per (element, Gauss point): kinematics and material tangent, written as
 //    D_g (9 blocks x 9), Hv_g (u-p coefficients) and Pv_g (p-u coefficients);
-//  * mr_contract_kernel / mr_contract_tc_kernel, one CTA per element: the contraction with the constant
+//  * mr_contract_kernel / mr_contract_tc_kernel, one element at a time a CTA: the contraction with the constant
 //    table G[(g,xi)][ms] and the u-p / p-u blocks.
 // The kernels here serve the FP32 paths (FP32 kinematics with det(F) in FP64, FP32 or TF32 contraction,
 // FP64 assembled values).
@@ -504,20 +545,30 @@ __device__ __forceinline__ void point_dP(const GPInT<float>& in, int seed, float
 constexpr int kGPElems = 4;                // elements per CTA of mr_gp_kernel
 constexpr uint32_t kTableWaitPolls = 1u << 24;  // bounded wait for the TMA copy of the tables
 constexpr int kGPThreads = kGPElems * NG;  // 108
-constexpr int kGPOut = 81 + 9 + 9;         // D (9 blocks x 9), Hv, Pv per Gauss point
-constexpr int kGPItem = (NG * kGPOut + 3) / 4 * 4;  // per-element stride: a 16-byte multiple (TMA)
+// Gauss-point blocks of an element, floats: D[mh * 3 + nh][g][xi * 3 + zeta] (g padded to 28 with zeros, so that four
+// points are nine 16-byte words), Hv[mh][g][xi], Pv[nh][g][xi] (xi padded to 4)
+constexpr int kGPBlock = 28 * 9;
+constexpr int kGPHv = 9 * kGPBlock;
+constexpr int kGPPv = kGPHv + 3 * NG * 4;
+constexpr int kGPItem = kGPPv + 3 * NG * 4;  // 2916: a 16-byte multiple (TMA)
+static_assert(kGPBlock % 4 == 0 && kGPItem % 4 == 0, "TMA bulk copies");
 
 struct GPShared {
+  alignas(16) float out[2][kGPElems][3 * kGPBlock];  // staging of the blocks: three (mh, nh) pairs, or Hv and Pv
   float x[kGPElems][81], z[kGPElems][81], p[kGPElems][8];
 };
+static_assert(kGPItem - kGPHv <= 3 * kGPBlock, "Hv and Pv fit one stage");
 
-// One thread per (element, Gauss point).  out[item * kGPItem + g * kGPOut + j]:
-// D[(mh*3+nh)*9 + xi*3+zeta], Hv[81 + xi*3+mh], Pv[90 + xi*3+nh].  Element data rounded to FP32 once per
+// One thread per (element, Gauss point), blocks at out[item * kGPItem].  They leave through shared memory, the three
+// blocks of one nh at a time, by TMA bulk copies: a thread's own stores are 4 bytes 36 apart, a sector each (32^3
+// elements: 498 -> 419 us; now bound by the FP32 instructions of the ten passes at 16 warps an SM; three seeds a pass
+// take 235 registers, 548 us).  Element data
+// rounded to FP32 once per
 // node when staged, the volume Jacobians det(Z), det(X) still evaluated in FP64 from the exactly widened
 // gradients; for the consistent tangent (EXACT) the forward-mode passes run in FP32 dual numbers, with
 // J_z and its derivatives formed in FP64 once a point (jz_seeds).
 template <bool EXACT>
-__global__ void __launch_bounds__(kGPThreads)
+__global__ void __launch_bounds__(kGPThreads, 4)
 mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __restrict__ eq2,
              const int32_t* __restrict__ elin, int32_t nq2, const double* __restrict__ xg,
              const double* __restrict__ dep, const double* __restrict__ cpar, const TablesF* __restrict__ Tg,
@@ -560,89 +611,140 @@ mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __
     tc::mbar_wait(tbar, 0, kTableWaitPolls);
     return;
   }
-  if (item >= count) return;
-  float* o = out + (size_t)item * kGPItem + (size_t)g * kGPOut;
+  const bool live = item < count;
+  const int n_live = min(kGPElems, count - (int)blockIdx.x * kGPElems);
+  // stage nh of the element's blocks, o[mh * kGPBlock + g * 9 + xi * 3 + zeta], or (nh = 3) Hv and Pv; then the
+  // copies of one stage run while the next is formed in the other half
+  auto stage = [&](int nh) { return S.out[nh & 1][le] + (nh < 3 ? g * 9 : g * 4); };
+  auto begin_stage = [&](int nh) {
+    if (nh >= 2) {
+      if (threadIdx.x == 0) tc::bulk_wait_read<1>();
+      __syncthreads();
+    }
+  };
+  auto end_stage = [&](int nh) {
+    if (nh < 3 && g == NG - 1)
+      for (int mh = 0; mh < 3; ++mh)
+        for (int k = 0; k < 9; ++k) S.out[nh & 1][le][mh * kGPBlock + NG * 9 + k] = 0.0f;
+    tc::fence_proxy_async();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int l = 0; l < n_live; ++l) {
+        float* dst = out + ((size_t)blockIdx.x * kGPElems + l) * kGPItem;
+        if (nh < 3) {
+          for (int mh = 0; mh < 3; ++mh)
+            tc::bulk_copy_s2g(dst + (mh * 3 + nh) * kGPBlock, S.out[nh & 1][l] + mh * kGPBlock, kGPBlock * 4);
+        } else {
+          tc::bulk_copy_s2g(dst + kGPHv, S.out[nh & 1][l], (kGPItem - kGPHv) * 4);
+        }
+      }
+      tc::bulk_commit();
+    }
+  };
   if constexpr (!EXACT) {
     const float c1 = (float)cpar[0], c2 = (float)cpar[1];
     GPT<float> q;
-    if (!gauss_point(T, g, S.z[le], S.x[le], S.p[le], q)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
-    float sub[6][9], hyd[9], jgw;
-    iron_point_tensors(q, c1, c2, sub, hyd, jgw);
+    float sub[6][9], hyd[9], jgw = 0.0f;
+    if (live) {
+      if (!gauss_point(T, g, S.z[le], S.x[le], S.p[le], q)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
+      iron_point_tensors(q, c1, c2, sub, hyd, jgw);
+    }
     // blocks to xi space: Dxi = Zi sub Zi^T (Zi = dxi/dz); upper blocks as transposes of the lower
 #pragma unroll
-    for (int mh = 0; mh < 3; ++mh)
+    for (int nh = 0; nh < 3; ++nh) {
+      begin_stage(nh);
+      float* o = stage(nh);
+      if (live) {
 #pragma unroll
-      for (int nh = 0; nh < 3; ++nh) {
-        const int blk = mh == nh ? mh : (mh > nh ? 3 + (mh == 1 ? 0 : (nh == 0 ? 1 : 2))
-                                                 : 3 + (nh == 1 ? 0 : (mh == 0 ? 1 : 2)));
-        const bool tr = mh < nh;
-        float W[3][3];
+        for (int mh = 0; mh < 3; ++mh) {
+          const int blk = mh == nh ? mh : (mh > nh ? 3 + (mh == 1 ? 0 : (nh == 0 ? 1 : 2))
+                                                   : 3 + (nh == 1 ? 0 : (mh == 0 ? 1 : 2)));
+          const bool tr = mh < nh;
+          float W[3][3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+          for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int z = 0; z < 3; ++z) {
-            float s = float(0);
+            for (int z = 0; z < 3; ++z) {
+              float s = float(0);
 #pragma unroll
-            for (int j = 0; j < 3; ++j) s += (tr ? sub[blk][j * 3 + i] : sub[blk][i * 3 + j]) * q.Zi[z][j];
-            W[i][z] = s;  // (sub Zi^T)[i][zeta]
-          }
+              for (int j = 0; j < 3; ++j) s += (tr ? sub[blk][j * 3 + i] : sub[blk][i * 3 + j]) * q.Zi[z][j];
+              W[i][z] = s;  // (sub Zi^T)[i][zeta]
+            }
 #pragma unroll
-        for (int xi = 0; xi < 3; ++xi)
+          for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
-          for (int z = 0; z < 3; ++z)
-            o[(mh * 3 + nh) * 9 + xi * 3 + z] =
-                (float)(q.Zi[xi][0] * W[0][z] + q.Zi[xi][1] * W[1][z] + q.Zi[xi][2] * W[2][z]);
+            for (int z = 0; z < 3; ++z)
+              o[mh * kGPBlock + xi * 3 + z] =
+                  (float)(q.Zi[xi][0] * W[0][z] + q.Zi[xi][1] * W[1][z] + q.Zi[xi][2] * W[2][z]);
+        }
       }
+      end_stage(nh);
+    }
+    begin_stage(3);
+    float* o = stage(3);
+    if (live) {
 #pragma unroll
-    for (int xi = 0; xi < 3; ++xi)
+      for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        o[81 + xi * 3 + m] = (float)(q.Zi[xi][0] * hyd[m * 3 + 0] + q.Zi[xi][1] * hyd[m * 3 + 1] +
-                                  q.Zi[xi][2] * hyd[m * 3 + 2]);
-        o[90 + xi * 3 + m] = (float)(jgw * q.Zi[xi][m]);
-      }
+        for (int m = 0; m < 3; ++m) {
+          o[m * NG * 4 + xi] = (float)(q.Zi[xi][0] * hyd[m * 3 + 0] + q.Zi[xi][1] * hyd[m * 3 + 1] +
+                                       q.Zi[xi][2] * hyd[m * 3 + 2]);
+          o[kGPPv - kGPHv + m * NG * 4 + xi] = (float)(jgw * q.Zi[xi][m]);
+        }
+    }
+    end_stage(3);
   } else {
     const float c1 = (float)cpar[0], c2 = (float)cpar[1];
     GPInT<float> in;
-    gauss_inputs(T, g, S.z[le], S.x[le], S.p[le], in);
     float jz[10];
-    jz_seeds(in.Z, jz);
-    for (int seed = 0; seed < 10; ++seed) {
-      float d[9];
-      point_dP(in, seed, c1, c2, d, jz);
-      if (seed < 9) {
-        const int nh = seed / 3, z = seed % 3;
+    if (live) {
+      gauss_inputs(T, g, S.z[le], S.x[le], S.p[le], in);
+      jz_seeds(in.Z, jz);
+    }
+    for (int nh = 0; nh < 4; ++nh) {
+      begin_stage(nh);
+      float* o = stage(nh);
+      if (live) {
+        for (int z = 0; z < (nh < 3 ? 3 : 1); ++z) {
+          float d[9];
+          point_dP(in, nh * 3 + z, c1, c2, d, jz);
 #pragma unroll
-        for (int xi = 0; xi < 3; ++xi)
+          for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
-          for (int mh = 0; mh < 3; ++mh) o[(mh * 3 + nh) * 9 + xi * 3 + z] = (float)d[xi * 3 + mh];
-      } else {
+            for (int mh = 0; mh < 3; ++mh) {
+              if (nh < 3) o[mh * kGPBlock + xi * 3 + z] = d[xi * 3 + mh];
+              else o[mh * NG * 4 + xi] = d[xi * 3 + mh];
+            }
+        }
+        if (nh == 3) {
+          float Zi[3][3];
+          const float dz = inv3(in.Z, Zi);
+          if (!(dz > float(0)) || !isfinite(dz)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) o[81 + k] = (float)d[k];
-        float Zi[3][3];
-        const float dz = inv3(in.Z, Zi);
-        if (!(dz > float(0)) || !isfinite(dz)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
+          for (int xi = 0; xi < 3; ++xi)
 #pragma unroll
-        for (int xi = 0; xi < 3; ++xi)
-#pragma unroll
-          for (int nh = 0; nh < 3; ++nh) o[90 + xi * 3 + nh] = (float)(in.w * jz[0] * Zi[xi][nh]);
+            for (int m = 0; m < 3; ++m) o[kGPPv - kGPHv + m * NG * 4 + xi] = (float)(in.w * jz[0] * Zi[xi][m]);
+        }
       }
+      end_stage(nh);
     }
   }
+  if (threadIdx.x == 0) tc::bulk_wait_read<0>();  // the stages may be gone once this thread exits
 }
 
 constexpr int kCThreads = 256;
 
 // u-p / p-u coefficients of one element: HvG[g][(mh,ms)] = sum_xi G[(g,xi)][ms] Hv_g[xi][mh] and
-// PvG[g][(nh,ns)] = sum_xi G[(g,xi)][ns] Pv_g[xi][nh] from the Gauss-point blocks Dg[g][99].
-template <typename TS, int GP>
-__device__ __forceinline__ void form_up_coefficients(const TS (*G)[GP], const TS (*Dg)[kGPOut], TS (*HvG)[81],
-                                                     TS (*PvG)[81]) {
+// PvG[g][(nh,ns)] = sum_xi G[(g,xi)][ns] Pv_g[xi][nh] from the element's Gauss-point blocks Dg.
+__device__ __forceinline__ void form_up_coefficients(const float (*G)[28], const float* Dg, float (*HvG)[81],
+                                                     float (*PvG)[81]) {
   for (int t = threadIdx.x; t < NG * 81; t += blockDim.x) {
     const int g = t / 81, c = t % 81, h = c / 27, s = c % 27;
-    const TS g0 = G[g * 3 + 0][s], g1 = G[g * 3 + 1][s], g2 = G[g * 3 + 2][s];
-    HvG[g][c] = g0 * Dg[g][81 + h] + g1 * Dg[g][84 + h] + g2 * Dg[g][87 + h];
-    PvG[g][c] = g0 * Dg[g][90 + h] + g1 * Dg[g][93 + h] + g2 * Dg[g][96 + h];
+    const float g0 = G[g * 3 + 0][s], g1 = G[g * 3 + 1][s], g2 = G[g * 3 + 2][s];
+    const float* H = Dg + kGPHv + (h * NG + g) * 4;
+    const float* P = Dg + kGPPv + (h * NG + g) * 4;
+    HvG[g][c] = g0 * H[0] + g1 * H[1] + g2 * H[2];
+    PvG[g][c] = g0 * P[0] + g1 * P[1] + g2 * P[2];
   }
 }
 
@@ -712,7 +814,7 @@ struct ContractShared {
   float C[2 * kCRows][28]; // C[(mh,nh,ms)][ns]
   float HvG[NG][81];       // sum_xi G[(g,xi)][ms] Hv[xi][mh]  -> [g][(mh,ms)]
   float PvG[NG][81];       // sum_xi G[(g,xi)][ns] Pv[xi][nh]  -> [g][(nh,ns)]
-  float Dg[NG][kGPOut];    // this element's Gauss-point blocks
+  float Dg[kGPItem];       // this element's Gauss-point blocks
   float psi[NG][NL];       // pressure basis at the Gauss points
 };
 static_assert(sizeof(float) * kCRows % 16 == 0 && sizeof(float) * 28 % 16 == 0, "vector rows");
@@ -741,9 +843,9 @@ mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Table
   for (int item = blockIdx.x; item < count; item += gridDim.x) {
     __syncthreads();
     const float* src = gp + (size_t)item * kGPItem;
-    for (int t = tid; t < NG * kGPOut; t += blockDim.x) (&S.Dg[0][0])[t] = src[t];
+    for (int t = tid; t < kGPItem; t += blockDim.x) S.Dg[t] = src[t];
     __syncthreads();
-    form_up_coefficients<float, 28>(S.G, S.Dg, S.HvG, S.PvG);
+    form_up_coefficients(S.G, S.Dg, S.HvG, S.PvG);
     for (int pass = 0; pass < 2; ++pass) {
       // operand rows [pass * kCRows, pass * kCRows + kCRows); rows past 242 are zero
       for (int t = tid; t < 81 * kCRows; t += blockDim.x) {
@@ -751,7 +853,7 @@ mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Table
         float v = 0.0f;
         if (row < 243) {
           const int pair = row / 27, ms = row % 27, g = k / 3, zeta = k % 3;
-          const float* D = &S.Dg[g][pair * 9 + zeta];
+          const float* D = &S.Dg[pair * kGPBlock + g * 9 + zeta];
           v = S.G[g * 3 + 0][ms] * D[0] + S.G[g * 3 + 1][ms] * D[3] + S.G[g * 3 + 2][ms] * D[6];
         }
         S.A[k][rl] = v;
@@ -780,7 +882,7 @@ mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Table
       }
       __syncthreads();  // A is rewritten by the next pass
     }
-    float* Ke = Kel + (size_t)__ldg(elems + item) * ND * ND;
+    float* Ke = Kel + (size_t)__ldg(elems + item) * kKelF;
     write_up_blocks<float, float>(Ke, S.HvG, S.PvG, S.psi);
     write_uu_block<EXACT, float, float, 28>(Ke, S.C);
   }
@@ -792,36 +894,45 @@ mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Table
 // For every (mh, nh) displacement-component pair the u-u block is
 //   K[(ms,mh),(ns,nh)] = sum_{g,zeta} A[(mh,nh,ms)][(g,zeta)] G[(g,zeta)][ns],
 //   A[(mh,nh,ms)][(g,zeta)] = sum_xi G[(g,xi)][ms] D_g[(mh,nh)][xi][zeta],
-// i.e. one 243 x 81 by 81 x 27 product per element.  A is formed on the CUDA cores (FP32) straight
-// into shared memory in the tensor cores' operand layout; the product runs as two M = 128 halves of
-// tcgen05.mma kind::tf32 (N = 32, K = 88 in 11 steps of 8) accumulating in tensor memory.  With
-// SPLIT3 each operand is split into a TF32 head and a TF32 tail and the three products
-// hi*hi + lo*hi + hi*lo recover about FP32 accuracy; without it the contraction is plain TF32
-// (about 1e-3 relative).  u-p / p-u blocks, Iron's lower-triangle mirror and the element-matrix
-// output are as in mr_contract_kernel.
-constexpr int kTCThreads = 1024;               // 32 warps: every phase is latency bound
-constexpr int kTCGroupWarps = kTCThreads / 32 / 16;  // warps sharing one 8-row group of the operand
+// i.e. one 243 x 81 by 81 x 27 product per element, as two M = 128 halves of tcgen05.mma kind::tf32 (N = 32, K = 88
+// in 11 steps of 8).  With SPLIT3 each operand is split into a TF32 head and a TF32 tail and the three products
+// hi*hi + lo*hi + hi*lo recover about FP32 accuracy; without it the contraction is plain TF32 (about 1e-3
+// relative).
+//
+// With A formed in shared memory (one CTA an SM, every phase behind the other) this took 2,073 us for 32^3 elements:
+// 5,600 wavefronts of shared memory an element for forming A, 2,600 cycles for the MMAs' operand reads and a single
+// thread's descriptor arithmetic.  Now (665 us) a thread forms a part of a row of A in registers (D by 16-byte
+// broadcasts, G without bank conflicts) and stores it to tensor memory, from which the MMAs take it; only the constant
+// G^T stays in shared memory, and the finished matrix leaves by one bulk copy.  The MMAs bound it: each takes 48
+// cycles for any N up to 64, 66 of them 3,200 cycles an element, and stores to tensor memory wait while MMAs of
+// either CTA run.  Hence two CTAs an SM that alternate, and large stores.  Slower: forming one K chunk while the
+// other is multiplied (801 us: the stores wait), one CTA that keeps a half of A in registers (952 us).  The head of
+// the split is rounded on the integer pipe (706 us with two conversions an entry).
+constexpr int kTCThreads = 384;
+constexpr int kTCForm = 8, kTCUp = 3;  // warps 0 .. 7 (two a tensor-memory quadrant), 8 .. 10; 11 copies and MMAs
 constexpr int kTK = 88;                        // K = 27 Gauss points x 3, padded to 11 steps of 8
 constexpr int kTKC = kTK / 4;                  // core-matrix columns along K (4 TF32 = 16 bytes)
-constexpr int kTABytes = 16 * kTKC * 128;      // one M = 128 operand tile
 constexpr int kTBBytes = 4 * kTKC * 128;       // the N = 32 operand
 constexpr uint32_t kTLbo = 128, kTSbo = kTKC * 128;
-constexpr int kTKRow = 33;                     // padded row of the staged product (no bank conflicts)
-constexpr uint32_t kTWaitPolls = 1u << 24;     // bounded mbarrier wait
+// tensor memory: a half of A, its K columns as 24 heads, 24 tails, 24 heads, ..., 16 heads, 16 tails; the two halves'
+// products
+constexpr uint32_t kTCols = 256;
+constexpr uint32_t kTAccCol = 2 * kTK;
+__host__ __device__ constexpr uint32_t tc_a_col(int step) { return (uint32_t)(step / 3 * 48 + step % 3 * 8); }
+__host__ __device__ constexpr uint32_t tc_a_tail(int step) { return step < 9 ? 24u : 16u; }
+constexpr long long kTWaitCycles = 2000000000; // bounded waits: about a second
 
 struct __align__(128) TCShared {
-  unsigned char A[2][kTABytes];  // head, tail of the current M half
   unsigned char B[2][kTBBytes];  // G head, tail: B[ns][(g,zeta)]
-  float G[81][28];               // G[(g,xi)][ms]; column 27 zero
-  float psi[NG][NL];
+  float G[84][28];               // G[(g,xi)][ms]; column 27 and rows 81 .. 83 zero
+  alignas(16) float psi[NG][NL];
   alignas(16) float Dg[2][kGPItem];  // Gauss-point blocks of the current and the next element (TMA)
-  float K[256][kTKRow];          // product rows (mh,nh,ms), columns ns
-  float HvG[NG][81];
-  float PvG[NG][81];
-  uint64_t mbar;
-  uint64_t dbar[2];              // completion of the bulk copies into Dg[0], Dg[1]
+  alignas(16) float K[kKelF];    // the element matrix
+  uint64_t afull, acc;           // a half of A formed / multiplied
+  uint64_t dfull[2];             // bulk copies into Dg[0], Dg[1]
+  uint64_t kfull, kempty;        // K written by the other warps / copied out
   uint32_t tmem;
-  int abort;
+  int undrained;
 };
 
 // byte offset of element (row, k) in a no-swizzle K-major operand with kTKC core columns
@@ -829,156 +940,249 @@ __device__ __forceinline__ uint32_t tc_offset(int row, int k) {
   return (uint32_t)((((row >> 3) * kTKC + (k >> 2)) * 8 + (row & 7)) * 16 + (k & 3) * 4);
 }
 
+// Warp: waits for the phase of parity `parity`; false after about a second.
+__device__ __forceinline__ bool tc_wait(uint64_t* mbar, uint32_t parity, unsigned* err) {
+  bool ok = tc::mbar_wait(mbar, parity, 16);
+  if (!ok) {
+    const long long t0 = clock64();
+    while (!(ok = tc::mbar_wait(mbar, parity, 16)) && clock64() - t0 < kTWaitCycles) {
+    }
+  }
+  ok = __all_sync(0xffffffffu, ok);
+  if (!ok) gfe_raise(err, GFE_DEVERR_TIMEOUT);
+  return ok;
+}
+
 template <bool EXACT, bool SPLIT3>
-__global__ void __launch_bounds__(kTCThreads, 1)
+__global__ void __launch_bounds__(kTCThreads, 2)
 mr_contract_tc_kernel(const int32_t* __restrict__ elems, int32_t count, const Tables* __restrict__ Tg,
                       const float* __restrict__ gp, float* __restrict__ Kel, unsigned* err) {
-  static_assert(kTCThreads % (16 * 32) == 0, "whole warps per 8-row group of an M = 128 operand tile");
   extern __shared__ __align__(1024) unsigned char traw[];
   TCShared& S = *reinterpret_cast<TCShared*>(traw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr uint32_t kDgBytes = kGPItem * sizeof(float);
   // constant operands: G (FP32, for forming A) and B = G^T split into TF32 head / tail
-  for (int t = tid; t < 81 * 28; t += blockDim.x) {
+  for (int t = tid; t < 84 * 28; t += kTCThreads) {
     const int k = t / 28, ms = t % 28;
-    S.G[k][ms] = ms < 27 ? (float)Tg->dphi[k / 3][k % 3][ms] : 0.0f;
+    S.G[k][ms] = ms < 27 && k < 81 ? (float)Tg->dphi[k / 3][k % 3][ms] : 0.0f;
   }
-  for (int t = tid; t < NG * NL; t += blockDim.x) S.psi[t / NL][t % NL] = (float)Tg->psi[t / NL][t % NL];
-  for (int t = tid; t < 32 * kTK; t += blockDim.x) {
+  for (int t = tid; t < NG * NL; t += kTCThreads) S.psi[t / NL][t % NL] = (float)Tg->psi[t / NL][t % NL];
+  for (int t = tid; t < 32 * kTK; t += kTCThreads) {
     const int n = t / kTK, k = t % kTK;
     const float v = (n < 27 && k < 81) ? (float)Tg->dphi[k / 3][k % 3][n] : 0.0f;
     const float hi = tc::to_tf32(v);
     *reinterpret_cast<float*>(S.B[0] + tc_offset(n, k)) = hi;
     *reinterpret_cast<float*>(S.B[1] + tc_offset(n, k)) = tc::to_tf32(v - hi);
   }
-  if (warp == 0) tc::tmem_alloc(&S.tmem, 64);
-  constexpr uint32_t kDgBytes = kGPItem * sizeof(float);
+  // the zero p-p block and the padding behind the matrix are never written again
+  for (int t = tid; t < NL * NL; t += kTCThreads) S.K[(81 + t / NL) * ND + 81 + t % NL] = 0.0f;
+  if (tid < kKelF - ND * ND) S.K[ND * ND + tid] = 0.0f;
+  if (warp == 0) tc::tmem_alloc(&S.tmem, kTCols);
   if (tid == 0) {
-    tc::mbar_init(&S.mbar, 1);
-    tc::mbar_init(&S.dbar[0], 1);
-    tc::mbar_init(&S.dbar[1], 1);
-    S.abort = 0;
-    // the first element's Gauss-point blocks: one TMA bulk copy
-    if ((int)blockIdx.x < count) {
-      tc::mbar_arrive_expect_tx(&S.dbar[0], kDgBytes);
-      tc::bulk_copy_g2s(S.Dg[0], gp + (size_t)blockIdx.x * kGPItem, kDgBytes, &S.dbar[0]);
-    }
+    tc::mbar_init(&S.afull, kTCForm);
+    tc::mbar_init(&S.acc, 1);
+    tc::mbar_init(&S.dfull[0], 1);
+    tc::mbar_init(&S.dfull[1], 1);
+    tc::mbar_init(&S.kfull, kTCForm + kTCUp);
+    tc::mbar_init(&S.kempty, 1);
+    S.undrained = 0;
   }
   tc::fence_proxy_async();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = S.tmem;
-  constexpr uint32_t idesc = tc::idesc_tf32(128, 32);
-  const uint32_t a_hi = tc::smem_u32(S.A[0]), a_lo = tc::smem_u32(S.A[1]);
-  const uint32_t b_hi = tc::smem_u32(S.B[0]), b_lo = tc::smem_u32(S.B[1]);
-  uint32_t parity = 0;
-  uint32_t dpar[2] = {0u, 0u};
-  bool pending[2] = {(int)blockIdx.x < count, false};  // (thread 0) copies issued and not yet waited for
-  // operand formation: warp w writes the 8-row group w of the current M = 128 tile, lane l its
-  // row 8 w + l / 4 and the K columns 4 kc + l % 4 (each step one core matrix, 128 bytes)
-  const int r_in = lane >> 2, kq = lane & 3;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem, 0);
 
-  int buf = 0;
-  for (int item = blockIdx.x; item < count; item += gridDim.x, buf ^= 1) {
-    __syncthreads();  // every thread is done with the previous element, whose buffer is Dg[buf ^ 1]
-    const int next = item + (int)gridDim.x;
-    if (tid == 0 && next < count) {
-      // prefetch the next element's blocks while this one is computed
-      tc::fence_proxy_async();
-      tc::mbar_arrive_expect_tx(&S.dbar[buf ^ 1], kDgBytes);
-      tc::bulk_copy_g2s(S.Dg[buf ^ 1], gp + (size_t)next * kGPItem, kDgBytes, &S.dbar[buf ^ 1]);
-      pending[buf ^ 1] = true;
-    }
-    if (!tc::mbar_wait(&S.dbar[buf], dpar[buf], kTWaitPolls)) {
-      gfe_raise(err, GFE_DEVERR_TIMEOUT);
-      tc::mbar_wait(&S.dbar[buf], dpar[buf], kTWaitPolls);
-      atomicMax(&S.abort, 1);
-    }
-    if (tid == 0) pending[buf] = false;
-    dpar[buf] ^= 1u;
-    __syncthreads();
-    if (S.abort) break;
-    const float(*Dg)[kGPOut] = reinterpret_cast<const float(*)[kGPOut]>(S.Dg[buf]);
-    float* Ke = Kel + (size_t)__ldg(elems + item) * ND * ND;
-    // warp w forms the core columns kc = w / 16, w / 16 + kTCGroupWarps, ... of the 8-row group w % 16
-    const int rg = warp & 15, kc0 = warp >> 4;
-    for (int half = 0; half < 2; ++half) {
-      const int row = half * 128 + rg * 8 + r_in;
-      const bool valid = row < 243;
-      const int pair = valid ? row / 27 : 0, ms = valid ? row % 27 : 0;
-      const float* Gm = &S.G[0][ms];
-      const float* Dp = &Dg[0][pair * 9];
-      unsigned char* a0 = S.A[0] + (rg * kTKC) * 128 + lane * 4;
-      unsigned char* a1 = S.A[1] + (rg * kTKC) * 128 + lane * 4;
-#pragma unroll 2
-      for (int kc = kc0; kc < kTKC; kc += kTCGroupWarps) {
-        const int k = kc * 4 + kq;
-        float v = 0.0f;
-        if (valid && k < 81) {
-          const int g = k / 3, zeta = k - 3 * g;
-          const float* D = Dp + g * kGPOut + zeta;
-          const float* Gg = Gm + (g * 3) * 28;
-          v = Gg[0] * D[0] + Gg[28] * D[3] + Gg[56] * D[6];
+  if (warp < kTCForm) {
+    // rows half * 128 + 32 warp + lane of A, formed four Gauss points (12 columns) at a time
+    const uint32_t quad = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const int part = warp >> 2;  // columns 0 .. 47, or 48 .. 87
+    // head and tail of the 12 columns of Gauss points 4 gg .. 4 gg + 3
+    auto form12 = [&](const float4* D4, const float* Gm, int gg, float* hi, float* lo) {
+      float d[36];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const float4 t = D4[gg * 9 + q];
+        d[4 * q] = t.x;
+        d[4 * q + 1] = t.y;
+        d[4 * q + 2] = t.z;
+        d[4 * q + 3] = t.w;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float* Gg = Gm + (gg * 4 + u) * 3 * 28;
+        const float g0 = Gg[0], g1 = Gg[28], g2 = Gg[56];
+#pragma unroll
+        for (int z = 0; z < 3; ++z) {
+          const float v = g0 * d[u * 9 + z] + g1 * d[u * 9 + 3 + z] + g2 * d[u * 9 + 6 + z];
+          hi[u * 3 + z] = SPLIT3 ? tc::to_tf32_number(v) : tc::to_tf32(v);
+          if (SPLIT3) lo[u * 3 + z] = tc::to_tf32(v - hi[u * 3 + z]);
         }
-        const float hi = tc::to_tf32(v);
-        *reinterpret_cast<float*>(a0 + kc * 128) = hi;
-        if (SPLIT3) *reinterpret_cast<float*>(a1 + kc * 128) = tc::to_tf32(v - hi);
+      }
+    };
+    // A store to tensor memory waits for the MMA in flight, so it takes 24 columns (head and tail) at once: with
+    // 12 columns in four stores, forming took twice as long
+    auto form = [&](const float* Dg, int half) {
+      const int row = half * 128 + (warp & 3) * 32 + lane, pair = min(row / 27, 8), ms = row % 27;
+      const float4* D4 = reinterpret_cast<const float4*>(Dg + pair * kGPBlock) + part * 36;
+      const float* Gm = &S.G[part * 48][ms];
+      const uint32_t base = quad + (uint32_t)(part * 96);
+      auto form24 = [&](int h) {
+        float v[48];  // 24 heads, 24 tails
+        form12(D4, Gm, h * 2, v, v + 24);
+        form12(D4, Gm, h * 2 + 1, v + 12, v + 36);
+        if (SPLIT3) {
+          tc::tmem_st_32(base + h * 48, v);
+          tc::tmem_st_16(base + h * 48 + 32, v + 32);
+        } else {
+          tc::tmem_st_16(base + h * 48, v);
+          tc::tmem_st_8(base + h * 48 + 16, v + 16);
+        }
+      };
+      form24(0);
+      if (part == 0) {
+        form24(1);
+      } else {
+        float v[32];  // 12 heads, 4 zeros, 12 tails, 4 zeros
+        form12(D4, Gm, 2, v, v + 16);
+#pragma unroll
+        for (int k = 12; k < 16; ++k) v[k] = v[16 + k] = 0.0f;
+        if (SPLIT3) tc::tmem_st_32(base + 48, v);
+        else tc::tmem_st_16(base + 48, v);
+      }
+      tc::tmem_wait_st();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&S.afull);
+    };
+    // the products of a half into the element matrix
+    auto read_back = [&](int half) {  // columns 0 .. 15, or 16 .. 26
+      float v[16];
+      tc::fence_after_sync();
+      tc::tmem_ld_32x16(quad + kTAccCol + (uint32_t)(half * 32 + part * 16), v);
+      const int row = half * 128 + (warp & 3) * 32 + lane, pair = min(row / 27, 8), ms = row % 27;
+      if (row >= 243) return;
+      const int mh = pair / 3, nh = pair % 3, r = mh * 27 + ms, n0 = part * 16;
+      float* Kr = S.K + r * ND + nh * 27 + n0;
+      float* Kc = S.K + (nh * 27 + n0) * ND + r;
+#pragma unroll
+      for (int n = 0; n < 16; ++n) {
+        if (n >= 11 && part) break;
+        // Iron mirrors the lower triangle into the upper one unless EXACT
+        if (EXACT || r >= nh * 27 + n0 + n) Kr[n] = v[n];
+        if (!EXACT && r >= nh * 27 + n0 + n) Kc[n * ND] = v[n];
+      }
+    };
+    for (int i = 0, item = blockIdx.x; item < count; ++i, item += gridDim.x) {
+      if (!tc_wait(&S.dfull[i & 1], (uint32_t)(i >> 1) & 1u, err)) break;
+      form(S.Dg[i & 1], 0);
+      if (!tc_wait(&S.acc, 0u, err) || (i > 0 && !tc_wait(&S.kempty, (uint32_t)(i - 1) & 1u, err))) break;
+      read_back(0);
+      form(S.Dg[i & 1], 1);
+      if (!tc_wait(&S.acc, 1u, err)) break;
+      read_back(1);
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&S.kfull);
+    }
+  } else if (warp < kTCForm + kTCUp) {
+    // u-p / p-u blocks: warp h has component h, lane ms; both are 27-term sums with the pressure basis
+    const int h = warp - kTCForm, ms = min(lane, 26), r = h * 27 + ms;
+    for (int i = 0, item = blockIdx.x; item < count; ++i, item += gridDim.x) {
+      if (!tc_wait(&S.dfull[i & 1], (uint32_t)(i >> 1) & 1u, err)) break;
+      const float4* H4 = reinterpret_cast<const float4*>(S.Dg[i & 1] + kGPHv) + h * NG;
+      const float4* P4 = reinterpret_cast<const float4*>(S.Dg[i & 1] + kGPPv) + h * NG;
+      float up[NL], pu[NL];
+#pragma unroll
+      for (int b = 0; b < NL; ++b) up[b] = pu[b] = 0.0f;
+#pragma unroll 3
+      for (int g = 0; g < NG; ++g) {
+        const float4 H = H4[g], P = P4[g];
+        const float g0 = S.G[g * 3][ms], g1 = S.G[g * 3 + 1][ms], g2 = S.G[g * 3 + 2][ms];
+        const float hg = g0 * H.x + g1 * H.y + g2 * H.z;
+        const float pg = g0 * P.x + g1 * P.y + g2 * P.z;
+        float psi[NL];
+        load4(&S.psi[g][0], *reinterpret_cast<float(*)[4]>(psi));
+        load4(&S.psi[g][4], *reinterpret_cast<float(*)[4]>(psi + 4));
+#pragma unroll
+        for (int b = 0; b < NL; ++b) {
+          up[b] += hg * psi[b];
+          pu[b] += psi[b] * pg;
+        }
+      }
+      if (i > 0 && !tc_wait(&S.kempty, (uint32_t)(i - 1) & 1u, err)) break;
+      if (lane < 27) {
+#pragma unroll
+        for (int b = 0; b < NL; ++b) {
+          S.K[r * ND + 81 + b] = up[b];
+          S.K[(81 + b) * ND + r] = pu[b];
+        }
       }
       tc::fence_proxy_async();
-      __syncthreads();
-      if (tid == 0) {
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&S.kfull);
+    }
+  } else if (lane == 0) {
+    // the next elements' blocks in, the MMAs as the halves of A come, the matrices out
+    constexpr uint32_t idesc = tc::idesc_tf32(128, 32);
+    const uint64_t b_hi = tc::smem_desc(tc::smem_u32(S.B[0]), kTLbo, kTSbo);
+    const uint64_t b_lo = tc::smem_desc(tc::smem_u32(S.B[1]), kTLbo, kTSbo);
+    auto load = [&](int i, int item) {
+      tc::mbar_arrive_expect_tx(&S.dfull[i & 1], kDgBytes);
+      tc::bulk_copy_g2s(S.Dg[i & 1], gp + (size_t)item * kGPItem, kDgBytes, &S.dfull[i & 1]);
+    };
+    auto wait = [&](uint64_t* mbar, uint32_t parity) {
+      const long long t0 = clock64();
+      while (!tc::mbar_wait(mbar, parity, 16))
+        if (clock64() - t0 > kTWaitCycles) {
+          gfe_raise(err, GFE_DEVERR_TIMEOUT);
+          return false;
+        }
+      return true;
+    };
+    const int step = (int)gridDim.x;
+    for (int k = 0; k < 2; ++k)
+      if ((int)blockIdx.x + k * step < count) load(k, blockIdx.x + k * step);
+    bool ok = true;
+    int i = 0;
+    for (int item = blockIdx.x; item < count; ++i, item += step) {
+      for (int half = 0; half < 2; ++half) {
+        if (!(ok = wait(&S.afull, (uint32_t)half))) break;
         tc::fence_after_sync();
-        const uint32_t d = tmem + (uint32_t)(half * 32);
-#pragma unroll 1
+        const uint32_t d = tmem + kTAccCol + (uint32_t)(half * 32);
+#pragma unroll
         for (int s = 0; s < kTK / 8; ++s) {
-          const uint32_t ko = (uint32_t)(s * 256);
-          tc::mma_tf32(d, tc::smem_desc(a_hi + ko, kTLbo, kTSbo), tc::smem_desc(b_hi + ko, kTLbo, kTSbo), idesc,
-                       s > 0 ? 1u : 0u);
+          const uint32_t a = tmem + tc_a_col(s);
+          tc::mma_tf32_ts(d, a, b_hi + s * 16, idesc, s > 0 ? 1u : 0u);  // a step is 256 bytes: 16 in the descriptor
           if (SPLIT3) {
-            tc::mma_tf32(d, tc::smem_desc(a_lo + ko, kTLbo, kTSbo), tc::smem_desc(b_hi + ko, kTLbo, kTSbo), idesc, 1u);
-            tc::mma_tf32(d, tc::smem_desc(a_hi + ko, kTLbo, kTSbo), tc::smem_desc(b_lo + ko, kTLbo, kTSbo), idesc, 1u);
+            tc::mma_tf32_ts(d, a + tc_a_tail(s), b_hi + s * 16, idesc, 1u);
+            tc::mma_tf32_ts(d, a, b_lo + s * 16, idesc, 1u);
           }
         }
-        tc::commit(&S.mbar);
-        // the A tile is rewritten by the next half: wait (bounded) for this half's products
-        if (!tc::mbar_wait(&S.mbar, parity, kTWaitPolls)) {
-          // the MMAs may still be writing tensor memory: wait once more for their commit before
-          // anything releases it; if that also ends without it, the tensor memory stays
-          // allocated (abort = 2) rather than being freed under the MMAs
-          gfe_raise(err, GFE_DEVERR_TIMEOUT);
-          const bool drained = tc::mbar_wait(&S.mbar, parity, kTWaitPolls);
-          S.abort = drained ? 1 : 2;
-        }
+        tc::commit(&S.acc);
       }
-      // work that needs neither A nor the product runs while the tensor cores multiply
-      if (half == 0) form_up_coefficients<float, 28>(S.G, Dg, S.HvG, S.PvG);
-      else write_up_blocks<float, float>(Ke, S.HvG, S.PvG, S.psi);
-      parity ^= 1u;
-      __syncthreads();
-      tc::fence_after_sync();
-      if (S.abort) break;
+      // every warp is done with this element (and the MMAs are, as their products have been read): its matrix goes
+      // out and its blocks' buffer is free
+      if (!ok || !(ok = wait(&S.kfull, (uint32_t)i & 1u))) break;
+      tc::fence_proxy_async();
+      tc::bulk_copy_s2g(Kel + (size_t)__ldg(elems + item) * kKelF, S.K, kKelF * (uint32_t)sizeof(float));
+      tc::bulk_commit();
+      if (item + 2 * step < count) load(i + 2, item + 2 * step);
+      tc::bulk_wait_read<0>();
+      tc::mbar_arrive(&S.kempty);
     }
-    if (S.abort) break;
-    // tensor memory -> staged product: warp w < 8 reads lanes 32 (w % 4) .. of half w / 4
-    if (warp < 8) {
-      const int half = warp >> 2, q = warp & 3;
-      float v[32];
-      tc::tmem_ld_32x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 32), v);
-      const int row = half * 128 + q * 32 + lane;
-#pragma unroll
-      for (int n = 0; n < 27; ++n) S.K[row][n] = v[n];
+    if (!ok) {
+      // MMAs may still write tensor memory: it stays allocated.  No copy may still be landing in this CTA's shared
+      // memory when it exits
+      S.undrained = 1;
+      for (int k = i; k < i + 2; ++k)
+        if ((int)blockIdx.x + k * step < count) wait(&S.dfull[k & 1], (uint32_t)(k >> 1) & 1u);
     }
-    tc::fence_before_sync();
-    __syncthreads();
-    write_uu_block<EXACT, float, float, kTKRow>(Ke, S.K);
   }
-  // no bulk copy may still be landing in this CTA's shared memory when it exits (bounded)
-  if (tid == 0)
-    for (int b = 0; b < 2; ++b)
-      if (pending[b] && !tc::mbar_wait(&S.dbar[b], dpar[b], kTWaitPolls)) gfe_raise(err, GFE_DEVERR_TIMEOUT);
+  __syncwarp();
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0 && S.abort < 2) tc::tmem_dealloc(tmem, 64);
+  if (warp == 0 && !S.undrained) tc::tmem_dealloc(tmem, kTCols);
 }
 
 int check_mesh(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t nq2, int32_t nlin, const double* xg,
@@ -1046,7 +1250,7 @@ int gather_rows(int32_t n_elem, const int32_t* elems, const int32_t* eq2, const 
   const long long rows = 3ll * nq2 + nlin;
   const int grid = (int)std::min<long long>((rows + kRowWarps - 1) / kRowWarps, 16ll * sms);
   mr_row_gather_kernel<TS><<<grid, kRowWarps * 32, 0, s>>>(nq2, nlin, cnt, list, Kel, slots, row_ptr, values,
-                                                          nullptr, err);
+                                                          err);
   gfe::scratch_free(inc, s);
   return GFE_OK;
 }
@@ -1095,7 +1299,7 @@ int jacobian_f32(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* el
   }
   const int chunk = std::min(n_elem, kElemChunk);
   float* Kel = nullptr;
-  if ((rc = gfe::scratch_alloc((void**)&Kel, sizeof(float) * (size_t)n_elem * ND * ND, s, "element matrices"))) return rc;
+  if ((rc = gfe::scratch_alloc((void**)&Kel, sizeof(float) * (size_t)n_elem * kKelF, s, "element matrices"))) return rc;
   float* gpbuf = nullptr;
   if ((rc = gfe::scratch_alloc((void**)&gpbuf, sizeof(float) * (size_t)chunk * kGPItem + 16, s,
                                "Gauss-point tangent blocks"))) {
@@ -1115,7 +1319,7 @@ int jacobian_f32(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* el
       mr_gp_kernel<true><<<ggrid, kGPThreads, gsm_k, s>>>(elems + c0, cnt, eq2, elin, nq2, xg, dep, cpar, TK, gpbuf, err);
     launches += 2;
     if (tc_mode) {
-      const int tgrid = std::min(cnt, sms);
+      const int tgrid = std::min(cnt, 2 * sms);
       if (mode == 0) {
         if (tc_mode == GFE_TC_TF32X3) launch_contract_tc<false, true>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
         else launch_contract_tc<false, false>(tgrid, s, elems + c0, cnt, T, gpbuf, Kel, err);
