@@ -70,6 +70,32 @@ __device__ __forceinline__ void accum(float& acc, float t) { acc += t; }
 __device__ __forceinline__ void accum_sub(float& acc, float t) { acc -= t; }
 __device__ __forceinline__ void finish(float&) {}
 
+
+// Forms without the final renormalisation (8 operations a sum instead of 11), for chains whose values do not cancel:
+// `lo` then reaches a few ulp(hi), and only products of two such values lose by it (they drop lo lo), so a
+// value is renormalised before it enters a product with another one.
+__device__ __forceinline__ f2 add_raw(f2 a, f2 b) {
+  accum(a, b);
+  return a;
+}
+__device__ __forceinline__ f2 sub_raw(f2 a, f2 b) { return add_raw(a, -b); }
+__device__ __forceinline__ f2 renorm(f2 a) { return fast_two_sum(a.hi, a.lo); }
+__device__ __forceinline__ double add_raw(double a, double b) { return a + b; }
+__device__ __forceinline__ double sub_raw(double a, double b) { return a - b; }
+// a b - c d and a b + c d + e f
+template <typename T>
+__device__ __forceinline__ T minor2(T a, T b, T c, T d) {
+  return a * b - c * d;
+}
+__device__ __forceinline__ f2 minor2(f2 a, f2 b, f2 c, f2 d) { return sub_raw(a * b, c * d); }
+template <typename T>
+__device__ __forceinline__ T dot3(T a, T b, T c, T d, T e, T f) {
+  return a * b + c * d + e * f;
+}
+__device__ __forceinline__ f2 dot3(f2 a, f2 b, f2 c, f2 d, f2 e, f2 f) {
+  return renorm(add_raw(add_raw(a * b, c * d), e * f));
+}
+
 __device__ __forceinline__ f2& operator+=(f2& a, f2 b) { return a = a + b; }
 __device__ __forceinline__ f2& operator-=(f2& a, f2 b) { return a = a - b; }
 __device__ __forceinline__ bool operator>(f2 a, f2 b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
@@ -100,6 +126,21 @@ __device__ __forceinline__ double f32_to_f64_exact(float f) {
   const unsigned long long bits =
       sgn | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(u & 0x7fffffu) << 29);
   return __longlong_as_double((long long)bits);
+}
+
+// hi + lo of a double with integer operations (see f32_to_f64_exact for why): hi is the mantissa's top 24 bits,
+// rounded to nearest, lo the signed rest of up to 29 bits, which one integer conversion rounds to 24.  Numbers whose
+// lo could be subnormal, infinities and NaNs take the conversions.
+__device__ __forceinline__ f2 f2_split(double a) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(a), t = u & 0x7fffffffffffffffull;
+  const int e = (int)(t >> 52) - 1023;
+  if ((unsigned)(e + 64) > 190u && t != 0) return f2_from(a);
+  const unsigned long long r = t + (1ull << 28);
+  const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
+  const unsigned hi = t == 0 ? 0u : (unsigned)(r >> 29) - (896u << 23);
+  const int rest = t == 0 ? 0 : (int)((unsigned)r & 0x1fffffffu) - (1 << 28);
+  const float lo = (float)rest * __uint_as_float((unsigned)(e - 52 + 127) << 23);  // a power of two: exact
+  return {__uint_as_float(hi | sign), sign ? -lo : lo};
 }
 
 // precision-generic helpers used by the element kernels

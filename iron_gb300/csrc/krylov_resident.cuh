@@ -18,7 +18,7 @@
 // (Slots that carry a barrier's number beside the value, read until all are current, save a round trip to the
 // L2 but have every CTA poll every slot: slower, 16 instead of 10 us an iteration.)
 // Measured, launched form -> resident: CG on the 64^3 Laplace system, FP32 matrix, 40 -> 16.6 us an iteration (the
-// sliced-ELL copy 47 MB, of which 32 MB are held on chip), FP64 58 -> 31 us; MINRES on the 8^3 Mooney-Rivlin
+// sliced-ELL copy 47 MB, of which 32 MB are held on chip), FP64 52 -> 31 us; MINRES on the 8^3 Mooney-Rivlin
 // tangent, FP32, 24 -> 9.4 us an iteration.  MINRES chains two FP64 sums and two barriers behind 2 us of product.
 // A wait is bounded; when it runs out every CTA leaves and the solve returns GFE_ERR_TIMEOUT.
 #pragma once

@@ -103,6 +103,19 @@ __device__ __forceinline__ bool hex8_metrics(const T (&x)[3][8], T kappa, T p, T
           Jt[c][a][0][g2] = fma(q, d, E[0][g2]);
           Jt[c][a][1][g2] = fma(p, d, E[0][g2]);
         }
+      } else if constexpr (std::is_same<T, f2>::value) {
+        // (not in scaled 1D values: that would move the sizes at which det overflows)
+        f2 E[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          E[i][0] = add_raw(D[i][0] * p, D[i][1] * q);
+          E[i][1] = add_raw(D[i][0] * q, D[i][1] * p);
+        }
+#pragma unroll
+        for (int g2 = 0; g2 < 2; ++g2) {
+          Jt[c][a][0][g2] = renorm(add_raw(E[0][g2] * p, E[1][g2] * q));
+          Jt[c][a][1][g2] = renorm(add_raw(E[0][g2] * q, E[1][g2] * p));
+        }
       } else {
 #pragma unroll
         for (int g2 = 0; g2 < 2; ++g2) {
@@ -128,19 +141,19 @@ __device__ __forceinline__ bool hex8_metrics(const T (&x)[3][8], T kappa, T p, T
         const int d1 = a == 0 ? 1 : 0, d2 = a == 2 ? 1 : 2;
         J[c][a] = Jt[c][a][gb[d1]][gb[d2]];
       }
-    T G00 = J[0][0] * J[0][0] + J[1][0] * J[1][0] + J[2][0] * J[2][0];
-    T G11 = J[0][1] * J[0][1] + J[1][1] * J[1][1] + J[2][1] * J[2][1];
-    T G22 = J[0][2] * J[0][2] + J[1][2] * J[1][2] + J[2][2] * J[2][2];
-    T G01 = J[0][0] * J[0][1] + J[1][0] * J[1][1] + J[2][0] * J[2][1];
-    T G02 = J[0][0] * J[0][2] + J[1][0] * J[1][2] + J[2][0] * J[2][2];
-    T G12 = J[0][1] * J[0][2] + J[1][1] * J[1][2] + J[2][1] * J[2][2];
-    T A00 = G11 * G22 - G12 * G12;
-    T A11 = G00 * G22 - G02 * G02;
-    T A22 = G00 * G11 - G01 * G01;
-    T A01 = G02 * G12 - G01 * G22;
-    T A02 = G01 * G12 - G02 * G11;
-    T A12 = G01 * G02 - G00 * G12;
-    T det = G00 * A00 + G01 * A01 + G02 * A02;
+    const T G00 = dot3(J[0][0], J[0][0], J[1][0], J[1][0], J[2][0], J[2][0]);
+    const T G11 = dot3(J[0][1], J[0][1], J[1][1], J[1][1], J[2][1], J[2][1]);
+    const T G22 = dot3(J[0][2], J[0][2], J[1][2], J[1][2], J[2][2], J[2][2]);
+    const T G01 = dot3(J[0][0], J[0][1], J[1][0], J[1][1], J[2][0], J[2][1]);
+    const T G02 = dot3(J[0][0], J[0][2], J[1][0], J[1][2], J[2][0], J[2][2]);
+    const T G12 = dot3(J[0][1], J[0][2], J[1][1], J[1][2], J[2][1], J[2][2]);
+    const T A00 = minor2(G11, G22, G12, G12);
+    const T A11 = minor2(G00, G22, G02, G02);
+    const T A22 = minor2(G00, G11, G01, G01);
+    const T A01 = minor2(G02, G12, G01, G22);
+    const T A02 = minor2(G01, G12, G02, G11);
+    const T A12 = minor2(G01, G02, G00, G12);
+    const T det = dot3(G00, A00, G01, A01, G02, A02);
     ok = ok && (det > zero);
     // GU * sqrt(det) * w = adj / det * sqrt(det) * w = adj * w * rsqrt(det); w = 1/8
     T sc = eighth * rsqrt(det);
@@ -240,13 +253,13 @@ __device__ __forceinline__ void hex8_contract_at(MetricAt Mg, T p, T q, T (&K)[3
 
 // a x + y
 __device__ __forceinline__ double axpy(double a, double x, double y) { return fma(a, x, y); }
-__device__ __forceinline__ f2 axpy(f2 a, f2 x, f2 y) { return a * x + y; }
+__device__ __forceinline__ f2 axpy(f2 a, f2 x, f2 y) { return add_raw(a * x, y); }
 
 // o[k] = sum over the two points of products of the scaled 1D values keyed by k = m + n: s0 (p/q)^2 + s1,
 // (s0 + s1) p/q, s0 + s1 (p/q)^2
 template <typename T>
 __device__ __forceinline__ void pair_sums(T s0, T s1, T r, T pp1, T (&o)[3]) {
-  const T s = s0 + s1;
+  const T s = add_raw(s0, s1);
   o[0] = axpy(pp1, s0, s);
   o[1] = r * s;
   o[2] = axpy(pp1, s1, s);
@@ -255,7 +268,8 @@ __device__ __forceinline__ void pair_sums(T s0, T s1, T r, T pp1, T (&o)[3]) {
 // hex8_contract_at in FP64 and float-float with fewer operations (about 390 instead of 590): scaled 1D
 // values (metric_scale), the symmetric part of each entry formed once per distinct triple of pairs (27 of
 // the 36 entries) and the two orders of each off-diagonal term added before they meet the entries.
-// 128^3 float-float assembly 1.27 -> 1.22 ms.
+// Float-float sums stay unnormalised (df.cuh): the kernel is bound by its FP32 instructions and their fetch.  128^3:
+// metrics 405 -> 376 us, contraction 431 -> 382 (fewer operations) -> 328 us, assembly 1.27 -> 1.13 ms.
 template <typename T, typename MetricAt>
 __device__ __forceinline__ void hex8_contract_scaled(MetricAt Mg, T (&K)[36]) {
   const T r = from_double<T>(kPoverQ), pp1 = from_double<T>(kPP1);
@@ -268,7 +282,7 @@ __device__ __forceinline__ void hex8_contract_scaled(MetricAt Mg, T (&K)[36]) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int g0 = j << d2, g1 = g0 | (1 << d1);
-      pair_sums(Mg(g0, a) + Mg(g0 | (1 << a), a), Mg(g1, a) + Mg(g1 | (1 << a), a), r, pp1, Tt[j]);
+      pair_sums(add_raw(Mg(g0, a), Mg(g0 | (1 << a), a)), add_raw(Mg(g1, a), Mg(g1 | (1 << a), a)), r, pp1, Tt[j]);
     }
 #pragma unroll
     for (int k1 = 0; k1 < 3; ++k1) {
@@ -330,7 +344,7 @@ __device__ __forceinline__ void hex8_contract_scaled(MetricAt Mg, T (&K)[36]) {
               if (ma * 2 + mb > na * 2 + nb) continue;  // the other order of the same sum
               const bool sa = ma == nb, sb = na == mb;
               const T t1 = W[na][mb][k], t2 = W[ma][nb][k];
-              const T x = sa == sb ? t1 + t2 : (sa ? t1 - t2 : t2 - t1);
+              const T x = sa == sb ? add_raw(t1, t2) : (sa ? sub_raw(t1, t2) : sub_raw(t2, t1));
               // the entries with these (a, b) indices, in either order, and pair k in direction c
 #pragma unroll
               for (int mc = 0; mc < 2; ++mc)
@@ -383,9 +397,16 @@ __device__ __forceinline__ void load_element(int e, const int32_t* __restrict__ 
   nd[0] = a.x; nd[1] = a.y; nd[2] = a.z; nd[3] = a.w;
   nd[4] = b.x; nd[5] = b.y; nd[6] = b.z; nd[7] = b.w;
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+  for (int c = 0; c < 3; ++c) {
+    const double* xc = coords + (size_t)c * n_nodes;
+    // float-float: relative to the element's first node, so that the split loses only the element's size
+    [[maybe_unused]] const double x0 = __ldg(xc + nd[0]);
 #pragma unroll
-    for (int m = 0; m < 8; ++m) x[c][m] = from_double<T>(__ldg(coords + (size_t)c * n_nodes + nd[m]));
+    for (int m = 0; m < 8; ++m) {
+      if constexpr (std::is_same<T, f2>::value) x[c][m] = f2_split(__ldg(xc + nd[m]) - x0);
+      else x[c][m] = from_double<T>(__ldg(xc + nd[m]));
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -525,11 +546,32 @@ __device__ __forceinline__ f2 acc_add(f2 a, f2 b) {
 }
 
 // Coordinates are read in the element arithmetic type: the FP32-pipe precisions take them from a
-// copy split once per node (float or float-float), so no element converts FP64 values itself.
+// copy split once per node (float or float-float), so no element converts FP64 values itself.  The float-float copy
+// is relative to the middle node (elements use differences only), which halves what the split to 48 bits loses on a
+// mesh at the origin and keeps a mesh far from it; it is formed with integer operations (129^3 nodes: 51 us by
+// conversions).
 template <typename T>
-__global__ void split_coords(long long n, const double* __restrict__ in, T* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = from_double<T>(in[i]);
+struct CoordSplit {
+  __device__ __forceinline__ CoordSplit(const double*, long long) {}
+  __device__ __forceinline__ T operator()(double x) const { return from_double<T>(x); }
+};
+template <>
+struct CoordSplit<f2> {
+  double r;
+  __device__ __forceinline__ CoordSplit(const double* xc, long long n) : r(__ldg(xc + n / 2)) {
+    if (!isfinite(r)) r = 0.0;
+  }
+  __device__ __forceinline__ f2 operator()(double x) const { return f2_split(x - r); }
+};
+// nodes [a, b) of n, three components
+template <typename T>
+__global__ void split_coords(long long n, long long a, long long b, const double* __restrict__ in, T* __restrict__ out) {
+  for (int c = 0; c < 3; ++c) {
+    const CoordSplit<T> split(in + c * n, n);
+#pragma unroll 4
+    for (long long i = a + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < b; i += (long long)gridDim.x * blockDim.x)
+      out[c * n + i] = split(__ldg(in + c * n + i));
+  }
 }
 
 template <typename P>
@@ -1083,6 +1125,8 @@ size_t regular_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, int precision
   return cb + (regular_metric_entries(nx, ny, nz) + 36ull * nx * ny * nz) * sizeof(f2);
 }
 
+// (Slower: block-wide barriers between the kernels' stages, so that warps share fetched instructions, 430 and 367 us;
+// 4 blocks an SM for the metrics, 429 us; edges formed in FP64 in the metric kernel, 553 us.)
 constexpr int kSplitThreads = 128;
 constexpr int kContractThreads = 128;
 
@@ -1132,13 +1176,13 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
                    unsigned* err, void* ws, int32_t l0, int32_t l1, bool split) {
   constexpr bool DF = std::is_same<T, f2>::value;
   const int prec = DF ? GFE_MIXED_DF : GFE_MIXED;
-  const long long n3 = 3ll * (nx + 1) * (ny + 1) * (nz + 1);
+  const long long n_nodes = (nx + 1ll) * (ny + 1) * (nz + 1);
   char* base = static_cast<char*>(ws);
   if (!base)
     if (int rc = gfe::scratch_alloc((void**)&base, regular_workspace_bytes(nx, ny, nz, prec), s, "split coordinates"))
       return rc;
   T* ct = reinterpret_cast<T*>(base);
-  if (split || !ws) split_coords<T><<<4 * gfe::sm_count(), 256, 0, s>>>(n3, coords, ct);
+  if (split || !ws) split_coords<T><<<4 * gfe::sm_count(), 256, 0, s>>>(n_nodes, 0, n_nodes, coords, ct);
   if constexpr (DF) {
     launch_elements_f2(s, nx, ny, nz, ct, kappa, base, std::max(l0 - 1, 0), std::min(l1, nz), err);
     launch_gather<f2>(s, nx, ny, nz, element_matrices_f2(base, nx, ny, nz), rp, values, values32, rhs, l0, l1);
@@ -1276,9 +1320,9 @@ extern "C" int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32
     // an empty range only converts the coordinates into the workspace
     if (!workspace || !convert_coords)
       return gfe::set_error(GFE_ERR_ARG, "%s: an empty layer range needs a workspace and convert_coords", fn);
-    const long long n3 = 3ll * (nx + 1) * (ny + 1) * (nz + 1);
-    if (precision == GFE_MIXED) split_coords<float><<<4 * gfe::sm_count(), 256, 0, s>>>(n3, coords, (float*)workspace);
-    else if (precision == GFE_MIXED_DF) split_coords<f2><<<4 * gfe::sm_count(), 256, 0, s>>>(n3, coords, (f2*)workspace);
+    const long long n = (nx + 1ll) * (ny + 1) * (nz + 1);
+    if (precision == GFE_MIXED) split_coords<float><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (float*)workspace);
+    else if (precision == GFE_MIXED_DF) split_coords<f2><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (f2*)workspace);
     GFE_LAUNCH_CHECK(fn);
     return GFE_OK;
   }
@@ -1303,18 +1347,6 @@ extern "C" int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32
 }
 
 namespace {
-
-// Node layers [a, a + n) of each coordinate component (component-major [3][NXY * NZ], layers
-// contiguous) converted into the workspace: the slab-wise form of split_coords.
-template <typename T>
-__global__ void split_coords_layers(long long per_comp, long long a, long long n, const double* __restrict__ in,
-                                    T* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 3 * n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long j = (i / n) * per_comp + a + i % n;
-    out[j] = from_double<T>(in[j]);
-  }
-}
 
 // CSR entries in the rows of node layers [0, L) of the regular mesh: every row holds its clipped
 // 27-point stencil, so the count factorises into (3 NX - 2)(3 NY - 2) times the clipped widths
@@ -1392,6 +1424,11 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
   // every pipeline stream starts after the work already on `stream`
   GFE_CUDA_TRY(cudaEventRecord(ev[0], s));
   for (cudaStream_t t : {hp->in, hp->comp[0], hp->comp[1], hp->out}) GFE_CUDA_TRY(cudaStreamWaitEvent(t, ev[0], 0));
+  // the middle node's coordinates, which the others are split relative to, ahead of their layer
+  if (coords_host && precision == GFE_MIXED_DF)
+    for (int c = 0; c < 3; ++c)
+      GFE_CUDA_TRY(cudaMemcpyAsync(coords + c * N + N / 2, coords_host + c * N + N / 2, sizeof(double),
+                                   cudaMemcpyHostToDevice, hp->in));
   long long node_hi = 0, elem_hi = 0;  // node / element layers uploaded so far
   const int cvt_grid = 2 * gfe::sm_count();
   for (int i = 0; i < n_slabs; ++i) {
@@ -1407,11 +1444,10 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
                                        cudaMemcpyHostToDevice, hp->in));
         }
       if (precision == GFE_MIXED)
-        split_coords_layers<float><<<cvt_grid, 256, 0, hp->in>>>(N, node_hi * NXY, (nh - node_hi) * NXY, coords,
-                                                                 static_cast<float*>(workspace));
+        split_coords<float><<<cvt_grid, 256, 0, hp->in>>>(N, node_hi * NXY, nh * NXY, coords,
+                                                          static_cast<float*>(workspace));
       else if (precision == GFE_MIXED_DF)
-        split_coords_layers<f2><<<cvt_grid, 256, 0, hp->in>>>(N, node_hi * NXY, (nh - node_hi) * NXY, coords,
-                                                              static_cast<f2*>(workspace));
+        split_coords<f2><<<cvt_grid, 256, 0, hp->in>>>(N, node_hi * NXY, nh * NXY, coords, static_cast<f2*>(workspace));
       node_hi = nh;
     }
     if (kappa_host && eh > elem_hi) {

@@ -88,3 +88,19 @@ def test_fp64_regular_mesh_forms(gfe_cuda, ne, with_kappa):
         rp, ci = oracle.csr_structure(m.elem_nodes, m.n_nodes)
         ov, _ = oracle.laplace_assemble(3, [1, 1, 1], [2, 2, 2], m.elem_nodes, m.coords, kap, rp, ci)
         assert np.abs(v.cpu().numpy() - ov).max() <= 1e-13 * np.abs(ov).max()
+
+
+@pytest.mark.parametrize("scale", [1.0, 3e-4, 7e5])
+def test_float_float_element_chain(gfe_cuda, scale):
+    """Float-float assembly with sums that are renormalised only before products, on a sheared, distorted mesh off the
+    origin and over several sizes, against FP64.  Bound: coordinates split to 2^-48 of their magnitude, 8 elements
+    and offsets of about one mesh length a side give differences to 2^-48 * 16, cubed ratios and cancelling sums a
+    factor of about 100 on top: 1e-11 of max|K|."""
+    A = LaplaceAssembly.from_regular_mesh(RegularMesh((7, 8, 5)))
+    g = torch.Generator().manual_seed(5)
+    x = A.coords.cpu()
+    x = x + 0.3 * x.roll(1, 0) + 0.02 * torch.rand(x.shape, generator=g, dtype=torch.float64) + 0.7
+    A.coords.copy_(x * scale)
+    ref = A.assemble("fp64").clone()
+    got = A.assemble("mixed_df")
+    assert (got - ref).abs().max().item() <= 1e-11 * ref.abs().max().item()
