@@ -272,11 +272,12 @@ int gfe_laplace_assemble_regular(int32_t nx, int32_t ny, int32_t nz, const doubl
 
 /* The same assembly with a caller-owned device workspace (16-byte aligned) of
  * gfe_laplace_regular_workspace_bytes(nx, ny, nz, precision) bytes, so that nothing is allocated:
- * the form to capture into a CUDA graph.  The workspace holds the converted coordinates and, for
- * GFE_MIXED_DF, every element's Gauss-point metrics and element matrix (float-float, 672 bytes an
- * element): the float-float element work runs as a metric kernel and a contraction kernel, each
- * element once, and the rows are then gathered from the element matrices.  workspace may be NULL
- * (then it is allocated and freed on `stream`, as gfe_laplace_assemble_regular does). */
+ * the form to capture into a CUDA graph.  The element matrices are formed once and the rows gathered from
+ * them.  The workspace holds them (288 bytes an element for GFE_FP64, 144 for GFE_MIXED), for the FP32-pipe
+ * precisions also room for converted coordinates and, for GFE_MIXED_DF, every element's Gauss-point metrics
+ * (float-float, 672 bytes an element in all).  workspace may be NULL: GFE_FP64 then runs a kernel that
+ * needs none, the others allocate and free it on `stream`, as gfe_laplace_assemble_regular does (GFE_MIXED,
+ * without memory for it, runs on the converted coordinates alone). */
 int64_t gfe_laplace_regular_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, int32_t precision);
 int gfe_laplace_assemble_regular_ws(int32_t nx, int32_t ny, int32_t nz, const double* coords, const double* kappa,
                                     const int32_t* row_ptr, double* values, float* values32, double* rhs,
@@ -304,8 +305,8 @@ int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, cons
  * stream while later slabs compute.  coords [3][N] / kappa [n_elem] are the device copies the
  * uploads fill (coords_host / kappa_host NULL: the device copy is already current; kappa NULL:
  * unit conductivity); values [nnz] is the device CSR value array.  Host buffers should be pinned
- * for the copies to overlap.  The FP32-pipe precisions need a 16-byte aligned workspace of
- * gfe_laplace_regular_workspace_bytes bytes; nothing is allocated.  Asynchronous: the pipeline's
+ * for the copies to overlap.  The FP32-pipe precisions need a 16-byte aligned workspace: GFE_MIXED_DF of
+ * gfe_laplace_regular_workspace_bytes bytes, GFE_MIXED of 12 bytes a node; nothing is allocated.  Asynchronous: the pipeline's
  * own streams start after the work already on `stream`, and `stream` waits for all of them, so
  * values_host is complete once `stream` has reached this point.  Slab boundaries come from the
  * closed-form entry count of the clipped 27-point stencil, so row_ptr must be the structure of the

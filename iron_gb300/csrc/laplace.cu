@@ -792,30 +792,30 @@ laplace_contract_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict_
   }
 }
 
-// FP64 element matrices of every element into Kel[36][E], metrics and contraction in one kernel (the code
-// fits the instruction cache): a thread an element.  Bound by the FP64 pipe: about 960 operations an
-// element.
+// FP64 or FP32 element matrices of every element into Kel[36][E], metrics and contraction in one kernel (the code
+// fits the instruction cache): a thread an element.  FP64: bound by its pipe, about 960 operations an element.
+template <typename T>
 __global__ void __launch_bounds__(128)
-laplace_element64_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __restrict__ coords,
-                         const double* __restrict__ kappa, double* __restrict__ Kel, unsigned* err) {
+laplace_matrix_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __restrict__ coords,
+                      const double* __restrict__ kappa, T* __restrict__ Kel, unsigned* err) {
   const long long EXY = (long long)nx * ny, E = EXY * nz;
   const long long NX = nx + 1, NXY = NX * (ny + 1), N = NXY * (nz + 1);
-  double p, q;
+  T p, q;
   gauss_pq(p, q);
   bool bad = false, nonfinite = false;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E; e += (long long)gridDim.x * blockDim.x) {
     const long long ex = e % nx, ey = (e / nx) % ny, ez = e / EXY;
-    double x[3][8];
+    T x[3][8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const long long n = (ex + (m & 1)) + (ey + ((m >> 1) & 1)) * NX + (ez + (m >> 2)) * NXY;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c][m] = __ldg(coords + c * N + n);
+      for (int c = 0; c < 3; ++c) x[c][m] = from_double<T>(__ldg(coords + c * N + n));
     }
     const double kd = kappa ? __ldg(kappa + e) : 1.0;
     if (!isfinite(kd)) nonfinite = true;
-    double K[36];
-    if (!laplace_hex8<double>(x, kd, p, q, K)) bad = true;
+    T K[36];
+    if (!laplace_hex8<T>(x, from_double<T>(kd), p, q, K)) bad = true;
 #pragma unroll
     for (int k = 0; k < 36; ++k) Kel[k * E + e] = K[k];
   }
@@ -823,7 +823,7 @@ laplace_element64_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __res
   if (nonfinite) gfe_raise(err, GFE_DEVERR_NONFINITE);
 }
 
-// The same for meshes too small to give every SM sub-partition a warp of elements: eight lanes an element,
+// FP64 for meshes too small to give every SM sub-partition a warp of elements: eight lanes an element,
 // a Gauss point each for the metrics, then the 63 directional sums of the contraction and the 36 entries
 // spread over the lanes.  On an idle GPU a kernel's time is its longest chain at one FP64 instruction in
 // 64 cycles: about 270 instructions here, 960 for a thread an element.
@@ -1108,8 +1108,8 @@ int check_device_errors(cudaStream_t s, const char* fn, bool sync) {
 }
 
 // Workspace: for FP64 the element matrices (36 numbers an element); for the FP32-pipe precisions the
-// converted coordinates and, for float-float, behind them at a 256-byte boundary the Gauss-point metrics
-// (48 float-float numbers an element) and the element matrices (36) of every element.
+// converted coordinates and, behind them at a 256-byte boundary, for float-float the Gauss-point metrics
+// (48 float-float numbers an element) and the element matrices (36) of every element, for FP32 the latter.
 size_t regular_coords_bytes(int32_t nx, int32_t ny, int32_t nz, int precision) {
   const size_t n3 = 3ull * (nx + 1) * (ny + 1) * (nz + 1);
   if (precision == GFE_FP64) return 0;
@@ -1121,7 +1121,7 @@ size_t regular_metric_entries(int32_t nx, int32_t ny, int32_t nz) {  // 48 per e
 size_t regular_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, int precision) {
   if (precision == GFE_FP64) return 36ull * nx * ny * nz * sizeof(double);
   const size_t cb = regular_coords_bytes(nx, ny, nz, precision);
-  if (precision != GFE_MIXED_DF) return cb;
+  if (precision == GFE_MIXED) return cb + 36ull * nx * ny * nz * sizeof(float);
   return cb + (regular_metric_entries(nx, ny, nz) + 36ull * nx * ny * nz) * sizeof(f2);
 }
 
@@ -1154,7 +1154,7 @@ void launch_gather(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const T* 
   const long long rows = (long long)(l1 - l0) * (nx + 1) * (ny + 1);
   const int grid = (int)std::min<long long>((rows + kGatherWarps * 32 - 1) / (kGatherWarps * 32),
                                             8ll * gfe::sm_count());
-  const size_t smem = (size_t)kGatherWarps * kGatherStage * sizeof(T);
+  const size_t smem = (size_t)kGatherWarps * kGatherStage * sizeof(typename AccOf<T>::type);
   cudaFuncSetAttribute((const void*)laplace_gather_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   laplace_gather_kernel<T><<<grid, kGatherWarps * 32, smem, s>>>(nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
 }
@@ -1173,14 +1173,36 @@ const f2* element_matrices_f2(const void* ws, int32_t nx, int32_t ny, int32_t nz
 template <typename T>
 int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const double* coords,
                    const double* kappa, const int32_t* rp, double* values, float* values32, double* rhs,
-                   unsigned* err, void* ws, int32_t l0, int32_t l1, bool split) {
+                   unsigned* err, void* ws, int32_t l0, int32_t l1, bool split, bool keep) {
   constexpr bool DF = std::is_same<T, f2>::value;
   const int prec = DF ? GFE_MIXED_DF : GFE_MIXED;
   const long long n_nodes = (nx + 1ll) * (ny + 1) * (nz + 1);
+  const size_t cb = regular_coords_bytes(nx, ny, nz, prec);
   char* base = static_cast<char*>(ws);
-  if (!base)
-    if (int rc = gfe::scratch_alloc((void**)&base, regular_workspace_bytes(nx, ny, nz, prec), s, "split coordinates"))
-      return rc;
+  // FP32, whole mesh: the element matrices once, then the row gather, as in FP64 (45 x 33 x 51 elements 75 -> 28 us,
+  // 4^3 32 -> 17 us, 128^3 1,064 -> 430 us: the tiled kernel forms a third of the elements twice and has few CTAs on
+  // a small mesh).  Slabs, and a mesh without memory for 144 bytes an element, take the tiled kernel.
+  bool gather = !DF && !keep && l0 == 0 && l1 == nz + 1;
+  if (!base) {
+    int rc = gfe::scratch_alloc((void**)&base, gather || DF ? regular_workspace_bytes(nx, ny, nz, prec) : cb, s,
+                                "regular-mesh workspace");
+    if (rc && gather) {
+      gather = false;
+      rc = gfe::scratch_alloc((void**)&base, cb, s, "split coordinates");
+    }
+    if (rc) return rc;
+  }
+  if constexpr (!DF) {
+    if (gather) {
+      const long long E = (long long)nx * ny * nz;
+      T* Kel = reinterpret_cast<T*>(base + cb);
+      laplace_matrix_kernel<T><<<(int)std::min<long long>((E + 127) / 128, 1 << 20), 128, 0, s>>>(nx, ny, nz, coords, kappa,
+                                                                                                  Kel, err);
+      launch_gather<T>(s, nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
+      if (!ws) gfe::scratch_free(base, s);
+      return GFE_OK;
+    }
+  }
   T* ct = reinterpret_cast<T*>(base);
   if (split || !ws) split_coords<T><<<4 * gfe::sm_count(), 256, 0, s>>>(n_nodes, 0, n_nodes, coords, ct);
   if constexpr (DF) {
@@ -1207,15 +1229,15 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
 template <>
 int launch_regular<double>(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const double* coords,
                            const double* kappa, const int32_t* rp, double* values, float* values32, double* rhs,
-                           unsigned* err, void* ws, int32_t l0, int32_t l1, bool) {
+                           unsigned* err, void* ws, int32_t l0, int32_t l1, bool, bool) {
   if (ws && l0 == 0 && l1 == nz + 1) {
     double* Kel = static_cast<double*>(ws);
     const long long E = (long long)nx * ny * nz;
     if (E <= 64ll * gfe::sm_count())
       laplace_element64_small_kernel<<<(int)((E + 15) / 16), 128, 0, s>>>(nx, ny, nz, coords, kappa, Kel, err);
     else
-      laplace_element64_kernel<<<(int)std::min<long long>((E + 127) / 128, 1 << 20), 128, 0, s>>>(nx, ny, nz, coords,
-                                                                                               kappa, Kel, err);
+      laplace_matrix_kernel<double><<<(int)std::min<long long>((E + 127) / 128, 1 << 20), 128, 0, s>>>(nx, ny, nz, coords,
+                                                                                                     kappa, Kel, err);
     launch_gather<double>(s, nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
     return GFE_OK;
   }
@@ -1291,19 +1313,14 @@ extern "C" int gfe_laplace_assemble_regular(int32_t nx, int32_t ny, int32_t nz, 
                                          nullptr, stream);
 }
 
-extern "C" int gfe_laplace_assemble_regular_ws(int32_t nx, int32_t ny, int32_t nz, const double* coords,
-                                               const double* kappa, const int32_t* row_ptr, double* values,
-                                               float* values32, double* rhs, int32_t precision, void* workspace,
-                                               void* stream) {
-  return gfe_laplace_assemble_regular_layers(nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, precision,
-                                             workspace, 0, nz + 1, 1, stream);
-}
+namespace {
 
-extern "C" int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* coords,
-                                                   const double* kappa, const int32_t* row_ptr, double* values,
-                                                   float* values32, double* rhs, int32_t precision, void* workspace,
-                                                   int32_t layer_begin, int32_t layer_end, int32_t convert_coords,
-                                                   void* stream) {
+// keep: the workspace keeps the converted coordinates for later layer calls
+int assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* coords,
+                            const double* kappa, const int32_t* row_ptr, double* values,
+                            float* values32, double* rhs, int32_t precision, void* workspace,
+                            int32_t layer_begin, int32_t layer_end, int32_t convert_coords,
+                            bool keep, void* stream) {
   const char* fn = "gfe_laplace_assemble_regular";
   if (nx <= 0 || ny <= 0 || nz <= 0 || !coords || !row_ptr || !values)
     return gfe::set_error(GFE_ERR_ARG, "%s: invalid arguments", fn);
@@ -1333,17 +1350,37 @@ extern "C" int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32
   const bool cv = convert_coords != 0;
   if (precision == GFE_FP64)
     rc = launch_regular<double>(s, nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, err, workspace,
-                                l0, l1, cv);
+                                l0, l1, cv, keep);
   else if (precision == GFE_MIXED)
     rc = launch_regular<float>(s, nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, err, workspace,
-                               l0, l1, cv);
+                               l0, l1, cv, keep);
   else
     rc = launch_regular<f2>(s, nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, err, workspace, l0,
-                            l1, cv);
-  gfe::stage_end(GFE_STAGE_LAPLACE_ELEMENTS, prof, s, precision == GFE_MIXED_DF ? 3 : 1);
+                            l1, cv, keep);
+  gfe::stage_end(GFE_STAGE_LAPLACE_ELEMENTS, prof, s,
+                 precision == GFE_MIXED_DF ? 3 : (l0 == 0 && l1 == nz + 1 && (workspace || precision == GFE_MIXED) ? 2 : 1));
   if (rc) return rc;
   GFE_LAUNCH_CHECK(fn);
   return GFE_OK;
+}
+
+}  // namespace
+
+extern "C" int gfe_laplace_assemble_regular_ws(int32_t nx, int32_t ny, int32_t nz, const double* coords,
+                                               const double* kappa, const int32_t* row_ptr, double* values,
+                                               float* values32, double* rhs, int32_t precision, void* workspace,
+                                               void* stream) {
+  return assemble_regular_layers(nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, precision, workspace, 0,
+                                 nz + 1, 1, false, stream);
+}
+
+extern "C" int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* coords,
+                                                   const double* kappa, const int32_t* row_ptr, double* values,
+                                                   float* values32, double* rhs, int32_t precision, void* workspace,
+                                                   int32_t layer_begin, int32_t layer_end, int32_t convert_coords,
+                                                   void* stream) {
+  return assemble_regular_layers(nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, precision, workspace,
+                                 layer_begin, layer_end, convert_coords, true, stream);
 }
 
 namespace {
@@ -1467,10 +1504,10 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
     int rc;
     if (precision == GFE_FP64)
       rc = launch_regular<double>(cs, nx, ny, nz, coords, kappa, row_ptr, values, nullptr, rhs, err, nullptr,
-                                  l0, l1, false);
+                                  l0, l1, false, true);
     else if (precision == GFE_MIXED)
       rc = launch_regular<float>(cs, nx, ny, nz, coords, kappa, row_ptr, values, nullptr, rhs, err, workspace,
-                                 l0, l1, false);
+                                 l0, l1, false, true);
     else {
       launch_gather<f2>(cs, nx, ny, nz, element_matrices_f2(workspace, nx, ny, nz), row_ptr, values, nullptr, rhs, l0, l1);
       rc = GFE_OK;

@@ -200,7 +200,12 @@ class LaplaceAssembly:
         if path == "regular":
             nx, ny, nz = self.regular
             if prec != GFE_FP64:
-                ws = self._regular_workspace(prec)
+                try:
+                    ws = self._regular_workspace(prec)
+                except torch.OutOfMemoryError:
+                    # FP32 runs without room for the element matrices (144 bytes an element), on a smaller scratch
+                    if prec != GFE_MIXED:
+                        raise
             _lib.call("gfe_laplace_assemble_regular_ws", nx, ny, nz, _lib.ptr(self.coords), _lib.ptr(self.kappa),
                       _lib.ptr(self.row_ptr), _lib.ptr(self.values), _lib.ptr(v32), _lib.ptr(self.rhs), prec,
                       _lib.ptr(ws), _lib.stream_handle(stream))
@@ -264,7 +269,16 @@ class LaplaceAssembly:
         L = _lib.load()
         nx, ny, nz = self.regular
         prec = PRECISIONS[precision]
-        ws = self._regular_workspace(prec)
+        # the slabs of FP64 need no workspace, those of FP32 the rounded coordinates alone
+        if prec == GFE_FP64:
+            ws = None
+        elif prec == GFE_MIXED:
+            ws = self.__dict__.setdefault("_ws_cache", {}).get("coords32")
+            if ws is None:
+                ws = self._ws_cache["coords32"] = torch.empty(12 * self.n_nodes + 256, dtype=torch.uint8,
+                                                              device=self.device)
+        else:
+            ws = self._regular_workspace(prec)
         _lib.call("gfe_laplace_assemble_regular_host", nx, ny, nz, _lib.host_ptr(coords_host),
                   _lib.host_ptr(kappa_host), _lib.ptr(self.coords), _lib.ptr(self.kappa), _lib.ptr(self.row_ptr),
                   _lib.ptr(self.values), _lib.host_ptr(values_host), _lib.ptr(self.rhs), prec, _lib.ptr(ws),
@@ -273,8 +287,8 @@ class LaplaceAssembly:
 
     def _regular_workspace(self, prec: int) -> torch.Tensor:
         """Device workspace of the regular-mesh kernels for precision code `prec`, allocated once per
-        precision and kept (FP64: every element's matrix, 288 bytes an element; float-float: also its
-        Gauss-point metrics, 672 bytes)."""
+        precision and kept (every element's matrix, 288 bytes an element in FP64 and 144 in FP32; float-float:
+        also its Gauss-point metrics, 672 bytes)."""
         cache = self.__dict__.setdefault("_ws_cache", {})
         if prec not in cache:
             nx, ny, nz = self.regular

@@ -104,3 +104,28 @@ def test_float_float_element_chain(gfe_cuda, scale):
     ref = A.assemble("fp64").clone()
     got = A.assemble("mixed_df")
     assert (got - ref).abs().max().item() <= 1e-11 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("ne", [(1, 1, 1), (2, 1, 1), (7, 5, 3), (33, 9, 17), (24, 31, 19)])
+def test_fp32_gather_equals_tiled_rows(gfe_cuda, ne):
+    """FP32 on the regular mesh: the whole assembly through element matrices, with a workspace, with scratch and in
+    layer slabs (the tiled kernel, which sums a row's eight contributions in the same order), gives the same bits."""
+    from iron_gb300 import _lib
+    A = LaplaceAssembly.from_regular_mesh(RegularMesh(ne))
+    g = torch.Generator().manual_seed(11)
+    x = A.coords.cpu() + 0.1 / max(ne) * torch.rand(A.coords.shape, generator=g, dtype=torch.float64)
+    A.coords.copy_(x)
+    got = A.assemble("mixed").clone()
+    nx, ny, nz = ne
+    ws = torch.empty(int(_lib.load().gfe_laplace_regular_workspace_bytes(nx, ny, nz, 1)), dtype=torch.uint8, device="cuda")
+    for mode in ("scratch", "slabs"):
+        A.values.fill_(-7.0)
+        args = (nx, ny, nz, _lib.ptr(A.coords), _lib.ptr(A.kappa), _lib.ptr(A.row_ptr), _lib.ptr(A.values), None, None, 1)
+        if mode == "scratch":
+            _lib.call("gfe_laplace_assemble_regular_ws", *args, None, _lib.stream_handle(None))
+        else:
+            for l0 in range(0, nz + 1, 8):
+                _lib.call("gfe_laplace_assemble_regular_layers", *args, _lib.ptr(ws), l0, min(l0 + 8, nz + 1),
+                          int(l0 == 0), _lib.stream_handle(None))
+        torch.cuda.synchronize()
+        assert torch.equal(A.values, got), mode
