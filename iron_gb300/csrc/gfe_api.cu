@@ -133,7 +133,8 @@ namespace {
 
 // The error word is taken by one kernel into pinned host memory: a copy to pageable memory, a memset and a
 // synchronisation took 21 us of a checked call on an idle stream, this 15 us (4^3 FP64 elements assembled and
-// checked: 61 -> 48 us, 45 x 33 x 51 FP32 59 -> 48 us).  64 words, one a call in progress, are allocated once; a call that finds none free (or no
+// checked: 61 -> 48 us, 45 x 33 x 51 FP32 59 -> 48 us).  64 words, one a call in progress, are allocated once; a
+// call that finds none free (or no
 // pinned memory) copies as before.
 constexpr int kTakeWords = 64, kTakeStride = 32;  // a cache line each
 std::mutex g_take_mu;

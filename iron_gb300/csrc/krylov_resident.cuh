@@ -17,20 +17,24 @@
 //    with the next Lanczos update.
 // (Slots that carry a barrier's number beside the value, read until all are current, save a round trip to the
 // L2 but have every CTA poll every slot: slower, 16 instead of 10 us an iteration.)
-// Measured, launched form -> resident: CG on the 64^3 Laplace system, FP32 matrix, 40 -> 16.6 us an iteration (the
-// sliced-ELL copy 47 MB, of which 32 MB are held on chip), FP64 52 -> 31 us; MINRES on the 8^3 Mooney-Rivlin
+// Measured, launched form -> resident: CG on the 64^3 Laplace system, FP32 matrix, 42 -> 12.3 us an iteration (the
+// sliced-ELL copy 47 MB, of which 32 MB are held on chip), FP64 52 -> 29 us (bound by the FP64 pipe); MINRES on the 8^3 Mooney-Rivlin
 // tangent, FP32, 24 -> 9.4 us an iteration.  MINRES chains two FP64 sums and two barriers behind 2 us of product.
 // A wait is bounded; when it runs out every CTA leaves and the solve returns GFE_ERR_TIMEOUT.
 #pragma once
 
 namespace {
 
-constexpr int kCgThreads = 1024;     // more warps hide the product's loads: 16.6 us an iteration at 64^3, 768 threads 20
+constexpr int kCgThreads = 1024;     // more warps hide the product's loads: at 768 threads an iteration at 64^3 took a fifth longer
 constexpr int kMinresThreads = 768;  // 80 registers a thread, no spills: the waits invalidate the L1, so that a spill
                                      // costs an L2 round trip an iteration
 constexpr int kResPolls = 1 << 21;  // about a second
 constexpr int kResMaxGrid = 160;    // CTAs at most
 constexpr int kResSmem = 212 << 10; // shared memory for the matrix
+constexpr int kCgSmem = 224 << 10;     // of the CG kernel
+template <int R>
+constexpr int kCgAt = (R * (kCgThreads / 32 - 1) + 1 + 3) / 4 * 4;  // slice bounds of a CTA
+constexpr int kCgRows = kCgThreads - 32;
 constexpr int kCgWorkers = kCgThreads / 32 - 1;      // worker warps of the CG kernel, then the barrier warp
 constexpr int kMinresWorkers = kMinresThreads / 32 - 2;  // of MINRES, then the rotation and the barrier warp
 
@@ -130,9 +134,12 @@ __global__ void __launch_bounds__(kCgThreads, 1)
 cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, const TV* __restrict__ dinv,
             const uint8_t* __restrict__ fixed, Scalars* sc, ResBarrier* bar, int iters, bool fresh) {
   extern __shared__ __align__(16) unsigned char res_smem[];
-  constexpr int kCap = kResSmem / (sizeof(TM) + sizeof(IT));
-  TM* s_val = reinterpret_cast<TM*>(res_smem);
-  IT* s_col = reinterpret_cast<IT*>(s_val + kCap);
+  TV* const s_x = reinterpret_cast<TV*>(res_smem);  // [R][kCgRows] each
+  TV* const s_d = s_x + R * kCgRows;
+  int* const s_at = reinterpret_cast<int*>(s_d + R * kCgRows);  // first entry of each slice, and the end
+  TM* const s_val = reinterpret_cast<TM*>(s_at + kCgAt<R>);
+  const int cap = (int)(res_smem + kCgSmem - reinterpret_cast<unsigned char*>(s_val)) / (int)(sizeof(TM) + sizeof(IT));
+  IT* s_col = reinterpret_cast<IT*>(s_val + cap);
   __shared__ TV part[2][32];
   __shared__ TV beta_v, alpha_v;
   __shared__ int done, aborted;
@@ -157,39 +164,35 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
   const int slices = (n + kSell - 1) / kSell;
   const int s0 = (int)((long long)slices * blockIdx.x / gridDim.x), s1 = (int)((long long)slices * (blockIdx.x + 1) / gridDim.x);
   const long long e0 = s0 < s1 ? __ldg(A.sptr + s0) : 0;
-  const int held = s0 < s1 ? (int)min((long long)kCap, __ldg(A.sptr + s1 - 1) + __ldg(A.slen + s1 - 1) - e0) : 0;
+  const int held = s0 < s1 ? (int)min((long long)cap, __ldg(A.sptr + s1 - 1) + __ldg(A.slen + s1 - 1) - e0) : 0;
   for (int i = threadIdx.x; i < held; i += kCgThreads) {
     s_val[i] = __ldg(A.val + e0 + i);
     s_col[i] = __ldg(A.col + e0 + i);
   }
-  // the rows of this thread: bounds of their slices, vector entries
-  int at[R], len[R], row[R];  // offsets within the CTA's share
-
-  TV xv[R], rv[R], zv[R], pv[R], qv[R], wv[R], dv[R];
-  unsigned off = 0;  // bit u: row u is fixed
+  // a thread's rows: slices s0 + u kCgWorkers + warp.  Their bounds, x and 1 / diagonal stay in shared memory, z is
+  // formed again from r, so that 64 registers hold the rest: the waits invalidate the L1, and with spilled values an
+  // iteration at 64^3 took 16.6 us instead of 12.3.  (Copying the part of z that the CTA's rows read to shared memory
+  // first: 15.2 us, for the matrix then has less of it.)
+  for (int i = threadIdx.x; i <= s1 - s0; i += kCgThreads)
+    s_at[i] = (int)((s0 + i < slices ? __ldg(A.sptr + s0 + i) : __ldg(A.sptr + slices - 1) + __ldg(A.slen + slices - 1)) - e0);
+  TV rv[R], pv[R], qv[R], wv[R];
+  unsigned off = 0, own = 0;  // bit u: row u is fixed, row u exists
 #pragma unroll
   for (int u = 0; u < R; ++u) {
-    const int sl = s0 + u * kCgWorkers + warp;
-    row[u] = n;
-    at[u] = 0;
-    len[u] = 0;
-    xv[u] = rv[u] = zv[u] = pv[u] = qv[u] = wv[u] = dv[u] = TV(0);
-    if (worker && sl < s1) {
-      at[u] = (int)(__ldg(A.sptr + sl) - e0) + lane;
-      len[u] = __ldg(A.slen + sl) / kSell;
-      const int i = sl * kSell + lane;
-      if (i < n) {
-        row[u] = i;
-        xv[u] = x[i];
-        rv[u] = r[i];
-        zv[u] = z[i];
-        dv[u] = dinv[i];
-        if (!fresh) {
-          pv[u] = p[i];
-          qv[u] = q[i];
-        }
-        if (fixed && fixed[i]) off |= 1u << u;
+    const int sl = s0 + u * kCgWorkers + warp, i = sl * kSell + lane;
+    rv[u] = pv[u] = qv[u] = wv[u] = TV(0);
+    if (!worker) continue;
+    s_x[u * kCgRows + threadIdx.x] = s_d[u * kCgRows + threadIdx.x] = TV(0);
+    if (sl < s1 && i < n) {
+      own |= 1u << u;
+      s_x[u * kCgRows + threadIdx.x] = x[i];
+      s_d[u * kCgRows + threadIdx.x] = dinv[i];
+      rv[u] = r[i];
+      if (!fresh) {
+        pv[u] = p[i];
+        qv[u] = q[i];
       }
+      if (fixed && fixed[i]) off |= 1u << u;
     }
   }
   cta_sync();
@@ -201,16 +204,17 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
 #pragma unroll
         for (int u = 0; u < R; ++u) {
           TV acc = TV(0);
-          const bool in_smem = at[u] - lane + len[u] * kSell <= held;  // uniform over the warp
-          const int self = (s0 + u * kCgWorkers + warp) * kSell + lane;
-          const TM* va = in_smem ? s_val + at[u] : A.val + e0 + at[u];
-          const IT* ca = in_smem ? s_col + at[u] : A.col + e0 + at[u];
-          for (int k0 = 0; k0 < len[u]; k0 += kSellUnroll) {
+          const int sl = u * kCgWorkers + warp, self = (s0 + sl) * kSell + lane;
+          const int at = sl < s1 - s0 ? s_at[sl] : 0, len = sl < s1 - s0 ? (s_at[sl + 1] - at) / kSell : 0;
+          const bool in_smem = at + len * kSell <= held;  // uniform over the warp
+          const TM* va = (in_smem ? s_val + at : A.val + e0 + at) + lane;
+          const IT* ca = (in_smem ? s_col + at : A.col + e0 + at) + lane;
+          for (int k0 = 0; k0 < len; k0 += kSellUnroll) {
             TM v[kSellUnroll];
             IT cc[kSellUnroll];
 #pragma unroll
             for (int k = 0; k < kSellUnroll; ++k) {
-              const bool in = k0 + k < len[u];
+              const bool in = k0 + k < len;
               v[k] = in ? va[(k0 + k) * kSell] : TM(0);
               cc[k] = in ? ca[(k0 + k) * kSell] : SellIndex<IT>::pad;
             }
@@ -242,9 +246,10 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
       TV dot = TV(0);
 #pragma unroll
       for (int u = 0; u < R; ++u) {
-        pv[u] = start ? zv[u] : zv[u] + b * pv[u];
+        const TV zv = s_d[u * kCgRows + threadIdx.x] * rv[u];
+        pv[u] = start ? zv : zv + b * pv[u];
         qv[u] = start ? wv[u] : wv[u] + b * qv[u];
-        if (row[u] < n) dot += pv[u] * qv[u];
+        if ((own >> u) & 1) dot += pv[u] * qv[u];
       }
       dot = warp_sum_down(dot);
       if (lane == 0) part[0][warp] = dot;
@@ -268,12 +273,12 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
       TV sz = TV(0), sr = TV(0);
 #pragma unroll
       for (int u = 0; u < R; ++u) {
-        xv[u] += a * pv[u];
+        s_x[u * kCgRows + threadIdx.x] += a * pv[u];
         rv[u] -= a * qv[u];
-        zv[u] = dv[u] * rv[u];
-        if (row[u] < n) {
-          z[row[u]] = zv[u];
-          sz += rv[u] * zv[u];
+        const TV zv = s_d[u * kCgRows + threadIdx.x] * rv[u];
+        if ((own >> u) & 1) {
+          z[(s0 + u * kCgWorkers + warp) * kSell + lane] = zv;
+          sz += rv[u] * zv;
           sr += rv[u] * rv[u];
         }
       }
@@ -294,11 +299,12 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
   }
 #pragma unroll
   for (int u = 0; u < R; ++u)
-    if (row[u] < n) {
-      x[row[u]] = xv[u];
-      r[row[u]] = rv[u];
-      p[row[u]] = pv[u];
-      q[row[u]] = qv[u];
+    if ((own >> u) & 1) {
+      const int i = (s0 + u * kCgWorkers + warp) * kSell + lane;
+      x[i] = s_x[u * kCgRows + threadIdx.x];
+      r[i] = rv[u];
+      p[i] = pv[u];
+      q[i] = qv[u];
     }
   if (blockIdx.x == 0 && !worker && lane == 0) {
     sc->beta = beta;
@@ -606,13 +612,13 @@ minres_resident(int n, int n_node, const int32_t* __restrict__ rp, const int32_t
 // Cooperative launch of a resident kernel; false when the device cannot hold its grid at once (the caller
 // then runs the launched form).
 template <typename... Params, typename... Args>
-bool launch_resident(void (*kernel)(Params...), int grid, int threads, cudaStream_t s, Args... args) {
-  if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem) != cudaSuccess) {
+bool launch_resident(void (*kernel)(Params...), int grid, int threads, int smem, cudaStream_t s, Args... args) {
+  if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.dynamicSmemBytes = kResSmem;
+  cfg.dynamicSmemBytes = smem;
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
   cfg.stream = s;

@@ -629,9 +629,9 @@ int run_cg_resident(cudaStream_t s, int n, const SellCopy<TM>& A, const uint8_t*
     GFE_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(ResBarrier), s));
     void* prof = gfe::stage_begin(GFE_STAGE_SPMV, s);
 #define GFE_CG_RESIDENT(R)                                                                                            \
-  (A.is_near ? launch_resident(cg_resident<TM, TV, int16_t, R>, grid, kCgThreads, s, n, A.near, x, r, z, p, q, dinv, fixed, \
+  (A.is_near ? launch_resident(cg_resident<TM, TV, int16_t, R>, grid, kCgThreads, kCgSmem, s, n, A.near, x, r, z, p, q, dinv, fixed, \
                                sc, bar, k, fresh)                                                                     \
-             : launch_resident(cg_resident<TM, TV, int32_t, R>, grid, kCgThreads, s, n, A.far, x, r, z, p, q, dinv, fixed, \
+             : launch_resident(cg_resident<TM, TV, int32_t, R>, grid, kCgThreads, kCgSmem, s, n, A.far, x, r, z, p, q, dinv, fixed, \
                                sc, bar, k, fresh))
     const bool ok = rounds == 1 ? GFE_CG_RESIDENT(1) : (rounds == 2 ? GFE_CG_RESIDENT(2) : (rounds == 3 && GFE_CG_RESIDENT(3)));
 #undef GFE_CG_RESIDENT
@@ -1342,7 +1342,7 @@ int run_minres_resident(cudaStream_t s, int n, const int32_t* rp, const int32_t*
     void* prof = gfe::stage_begin(GFE_STAGE_SPMV, s);
     bool ok;
 #define GFE_MINRES_RESIDENT(L, C)                                                                                     \
-  launch_resident(minres_resident<TM, TV, TX, L, C>, grid, kMinresThreads, s, n, n_node, rp, ci, val, fixed, minv, x, \
+  launch_resident(minres_resident<TM, TV, TX, L, C>, grid, kMinresThreads, kResSmem, s, n, n_node, rp, ci, val, fixed, minv, x, \
                   V[0], V[1], Z[0], Z[1], W[0], W[1], sc, bar, j, k)
     if constexpr (std::is_same<TV, double>::value) ok = GFE_MINRES_RESIDENT(8, 1);
     else if (nodes) ok = lpr == 16 ? GFE_MINRES_RESIDENT(16, 3) : GFE_MINRES_RESIDENT(32, 3);
