@@ -320,17 +320,32 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
 
 // ---- MINRES -----------------------------------------------------------------------------------------
 
-// First group of CTA b of `grid`: equal shares, where a single row behind the nodes counts twice (a pressure row
-// of the Q2/Q1 tangent has about twice the columns of an average displacement node's).
-__host__ __device__ inline int minres_share(int n_groups, int n_node, int b, int grid) {
-  const long long units = n_node + 2ll * (n_groups - n_node), u = units * b / grid;
-  return u <= n_node ? (int)u : n_node + (int)((u - n_node) / 2);
+// First group of CTA b: shares of equal cost, a group costing its entries plus c0.  With equal numbers of groups the
+// CTAs with the longest rows (a triquadratic node has 89 to 402 entries, by lines of the mesh) held the others up at
+// the first barrier: an FP64 Newton solve at 8^3, bound by the FP64 pipe, takes 45.6 instead of 51.0 ms.  An FP32
+// group costs its latency more than its entries: with 32 entries' worth as in FP64 an iteration took 10.4 us, with
+// 256 it takes the 9.4 of equal numbers.  `nodes` groups of NC rows, then single rows; e0, total: entries of the nodes'
+// rows of one component, and the cost of all groups.
+template <int NC>
+__device__ int minres_share(const int32_t* __restrict__ rp, int nodes, int n_groups, long long e0, long long c0,
+                            long long total, int b, int grid) {
+  const long long want = total * b / grid;
+  int lo = 0, hi = n_groups;  // the first group with cost(g) >= want
+  while (lo < hi) {
+    const int g = lo + (hi - lo) / 2;
+    const long long e = g <= nodes ? __ldg(rp + g) - 1ll
+                                   : e0 + __ldg(rp + g + (NC - 1) * nodes) - __ldg(rp + NC * nodes);
+    if (e + c0 * g < want) lo = g + 1;
+    else hi = g;
+  }
+  return lo;
 }
 
 // At most `iters` iterations of the preconditioned MINRES from z = Z[j0 & 1] and the scalars of *sc
 // (nothing pending); vectors rotate with the iteration number as in the launched form.  NC rows a group:
 // the NC components of a node (minres_spmv_nodal), or 1.  A CTA takes a contiguous share of the groups, at
-// most kMinresWorkers * 32 rows, and LPR lanes a group in the product.
+// most kMinresWorkers * 32 rows (the host sees to n_groups / grid + 4 <= kMinresWorkers * 32 / NC), and LPR lanes a
+// group in the product.
 template <typename TM, typename TV, typename TX, int LPR, int NC>
 __global__ void __launch_bounds__(kMinresThreads, 1)
 minres_resident(int n, int n_node, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
@@ -359,8 +374,17 @@ minres_resident(int n, int n_node, const int32_t* __restrict__ rp, const int32_t
   // groups [g_begin, g_end) of this CTA: nn nodes, then single rows; their rows are local 0 .. rows - 1,
   // component by component
   const int n_groups = n - (NC - 1) * n_node;
-  const int g_begin = minres_share(n_groups, NC > 1 ? n_node : n_groups, blockIdx.x, gridDim.x);
-  const int g_end = minres_share(n_groups, NC > 1 ? n_node : n_groups, blockIdx.x + 1, gridDim.x);
+  // c0: as minres_share says, and enough for a share's rows to have a thread each
+  __shared__ int g_cut[2];
+  if (threadIdx.x < 2) {
+    const int nodes = NC > 1 ? n_node : n_groups, grid = (int)gridDim.x;
+    const long long e0 = __ldg(rp + nodes) - 1ll, E = e0 + (NC > 1 ? __ldg(rp + n) - __ldg(rp + NC * n_node) : 0);
+    const int room = kMinresWorkers * 32 / NC - n_groups / grid - 3;
+    const long long c0 = max(sizeof(TV) == 8 ? 32ll : 256ll, (E / grid + 1) / room + 1);
+    g_cut[threadIdx.x] = minres_share<NC>(rp, nodes, n_groups, e0, c0, E + c0 * n_groups, blockIdx.x + threadIdx.x, grid);
+  }
+  __syncthreads();
+  const int g_begin = g_cut[0], g_end = g_cut[1];
   const int nn = NC > 1 ? min(max(n_node - g_begin, 0), g_end - g_begin) : 0;
   const int rows = nn * NC + (g_end - g_begin - nn);
   // entries: the nodes' rows are NC contiguous ranges of the CSR, the single rows another one; held in

@@ -1330,10 +1330,9 @@ int run_minres_resident(cudaStream_t s, int n, const int32_t* rp, const int32_t*
   // lanes a group: FP64 8 (the shuffle sums run on the FP64 pipe); FP32 a warp, or half a warp where that lets
   // one pass of a CTA cover its groups.  At least eight groups a CTA: below that the barriers cost more
   const int grid = std::min({sms, kResMaxGrid, (groups + 7) / 8});
-  const long long units = nodes ? n_node + 2ll * (groups - n_node) : groups;
-  const int share = (int)((units + grid - 1) / grid);  // groups a CTA at most
+  const int share = (groups + grid - 1) / grid;  // groups a CTA on average
   const int lpr = std::is_same<TV, double>::value ? 8 : (share > kMinresWorkers && share <= 2 * kMinresWorkers ? 16 : 32);
-  *ran = share * (nodes ? 3 : 1) <= kMinresWorkers * 32;  // a thread a row
+  *ran = groups / grid + 4 <= kMinresWorkers * 32 / (nodes ? 3 : 1);  // a thread a row
   if (!*ran) return GFE_OK;
   int j = 1;
   while (j <= max_iters) {
