@@ -343,7 +343,9 @@ int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t nz, const 
  * hexahedral bases, GFE_TC_TF32X3: the contraction K(m,n) = sum_g dphi_m^T M_g dphi_n as an
  * M = 128 tcgen05 product (FP32 metrics, TF32 head / tail operands, FP32 accumulation in tensor
  * memory; about FP32 accuracy).  The matrix and rhs are zeroed first; each pair of element nodes
- * is added through Iron's CSR search.
+ * is added through Iron's CSR search.  Quadratic and cubic hexahedra in FP64 and float-float with as many
+ * Gauss points as functions a direction form all element matrices in scratch on `stream` first when they
+ * fit 256 MB (not while `stream` is being captured) and add them colour by colour, the same sums.
  * Asynchronous; device-side failures are reported through gfe_device_errors(). */
 int gfe_laplace_assemble_tp(const int32_t* order, const int32_t* n_gauss, int32_t n_elem, int32_t n_nodes,
                             const int32_t* elem_nodes, const double* coords, const double* scale, const double* kappa,
@@ -384,7 +386,8 @@ int gfe_laplace_element_matrices(int32_t n_elem, int32_t n_nodes, const int32_t*
  * is [batch][2]).  Replaces the element loop of EquationsSet_ResidualEvaluateStaticFEM
  * (src/equations_set_routines.F90:5164-5286) around the MOONEY_RIVLIN_SUBTYPE branch of
  * FiniteElasticity_FiniteElementResidualEvaluate (src/finite_elasticity_routines.F90:1669-1756).
- * Colouring as in gfe_laplace_assemble.  R is zeroed first. */
+ * Colouring as in gfe_laplace_assemble.  R is zeroed first.  Element vectors go through scratch on `stream`
+ * when they fit 256 MB, else straight into R colour by colour: the same sums. */
 int gfe_mr_residual(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t n_q2, int32_t n_lin,
                     const double* xg, const int32_t* color_elems, const int32_t* color_ptr_host, int32_t n_colors,
                     int32_t batch, const double* dep, const double* cpar, double* R, void* stream);
@@ -433,7 +436,8 @@ int gfe_mr_tangent(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int3
  * `step` is Iron's jacobianFiniteDifferenceStepSize (default 1e-6, set by
  * cmfe_Equations_JacobianFiniteDifferenceStepSizeSet, src/opencmiss_iron.F90:25271-25348).  Outputs
  * as gfe_mr_jacobian, assembled colour by colour through the slot map (values zeroed first).
- * Allocates and frees a small norm scratch on `stream`. */
+ * Allocates and frees on `stream` a small norm scratch and, for up to 4,096 elements without K_out, the
+ * element matrices (without memory for them the columns are added as they are formed). */
 int gfe_mr_jacobian_fd(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t n_q2, int32_t n_lin,
                        const double* xg, const int32_t* color_elems, const int32_t* color_ptr_host, int32_t n_colors,
                        const double* dep, const double* cpar, double step, const int32_t* slots, double* values,
@@ -465,6 +469,8 @@ int gfe_csr_spmv(int32_t n_rows, const int32_t* row_ptr, const int32_t* col_idx,
  *             FP32 one after each 1e3-fold reduction; the FP32 search direction is kept)
  *  rtol       relative residual target ||f - K x|| / ||f - K x0||
  *  iters_host out: total (inner) iterations;  rel_host out: final relative FP64 residual
+ * Short rows (32 entries on average at most) and a matrix of at most 100 MB: the iterations run in
+ * cooperative kernels of one CTA an SM; GFE_ERR_TIMEOUT when a wait between their CTAs runs out.
  * Synchronises `stream`.  Allocates and frees its scratch on `stream`. */
 int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* col_idx, const double* values,
                  const float* values32, const double* f, const uint8_t* fixed, double* x, double rtol,
@@ -524,6 +530,7 @@ int gfe_cg_status(int32_t n, void* workspace, gfe_cg_state* state_host, void* st
  *             minimises, PETSc's default for KSPMINRES), x0 = Dirichlet values with zeros
  *             elsewhere; rel_host returns that ratio for the final FP64 residual.  Other arguments
  *             as gfe_cg_solve (GFE_MIXED: FP64-residual refinement around FP32 MINRES on values32).
+ * Long rows (48 entries on average at least) and a matrix of at most 100 MB: cooperative kernels, as there.
  * Synchronises `stream`.  Allocates and frees its scratch on `stream`. */
 int gfe_minres_solve(int32_t n, const int32_t* row_ptr, const int32_t* col_idx, const double* values,
                      const float* values32, const double* minv, const double* f, const uint8_t* fixed, double* x,
