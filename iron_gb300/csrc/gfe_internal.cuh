@@ -52,6 +52,28 @@ void stage_end(int stage, void* token, cudaStream_t s, int launches);
       return gfe::set_error(GFE_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e__)); \
   } while (0)
 
+// Chains of small kernels, each adding one colour's entries: with `overlap` a launch may start once every CTA of the
+// kernel before it has called chain_release (or has ended), so its launch and first loads run under that kernel's end;
+// what the kernels before it wrote may be read (past the L1: __ldcg) or written after chain_wait only.  A kernel calls chain_wait before
+// chain_release: what precedes the whole chain is then complete when the next one starts.
+namespace gfe {
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(bool overlap, void (*kernel)(Params...), int grid, int block, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+}  // namespace gfe
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Device-side error reporting: kernels never trap; they set bits in the error word.
 __device__ __forceinline__ void gfe_raise(unsigned* err, unsigned bit) {
   if (err) atomicOr(err, bit);

@@ -289,24 +289,34 @@ laplace_tp_sf_kernel(const int32_t* __restrict__ ce, int32_t cnt, int32_t n_node
   if (nonfinite) gfe_raise(err, GFE_DEVERR_NONFINITE);
 }
 
-// values += the packed element matrices Kel[item][pair] of one colour's elements (no two share a row)
+// values += the packed element matrices Kel[item][pair] of one colour's elements (no two share a row).  The colours'
+// launches overlap (launch_chained): 36 x 31 x 33 quadratic elements 731 -> 712 us a call.
 __global__ void tp_add_element_matrices(const int32_t* __restrict__ ce, int32_t cnt, int32_t nns, int32_t npairs,
                                         const int32_t* __restrict__ en, const SFPair* __restrict__ pairs,
                                         const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                         const int32_t* __restrict__ slots, const double* __restrict__ Kel,
                                         double* __restrict__ values, unsigned* err) {
   const long long total = (long long)cnt * npairs;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, pmn = -2, pnm = -2;
+  double v = 0.0;
+  auto load = [&] {
     const int item = (int)(t / npairs), p = (int)(t - (long long)item * npairs);
     const int e = __ldg(ce + item), mn = __ldg(&pairs[p].mn), m = mn & 0xffff, n = mn >> 16;
-    const double v = __ldcs(Kel + t);
+    v = __ldcs(Kel + t);
     const int rm = __ldg(en + (size_t)e * nns + m), rn = __ldg(en + (size_t)e * nns + n);
-    const long long pmn = entry_pos(slots, e, nns, m, n, rp, ci, rm, rn + 1);
-    const long long pnm = m == n ? -2 : entry_pos(slots, e, nns, n, m, rp, ci, rn, rm + 1);
-    const double o0 = pmn >= 0 ? values[pmn] : 0.0, o1 = pnm >= 0 ? values[pnm] : 0.0;
+    pmn = entry_pos(slots, e, nns, m, n, rp, ci, rm, rn + 1);
+    pnm = m == n ? -2 : entry_pos(slots, e, nns, n, m, rp, ci, rn, rm + 1);
+  };
+  if (t < total) load();
+  chain_wait();
+  chain_release();
+  while (t < total) {
+    const double o0 = pmn >= 0 ? __ldcg(values + pmn) : 0.0, o1 = pnm >= 0 ? __ldcg(values + pnm) : 0.0;
     if (pmn >= 0) values[pmn] = o0 + v;
     if (pnm >= 0) values[pnm] = o1 + v;
     if (pmn < 0 || pnm == -1) gfe_raise(err, GFE_DEVERR_SLOT);
+    t += (long long)gridDim.x * blockDim.x;
+    if (t < total) load();
   }
 }
 
@@ -436,6 +446,7 @@ int launch_tp_sf(const int32_t* order, const int32_t* ngauss, int32_t n_nodes, c
     ++*launches;
   };
   if (Kel) launch(0, n_elem);
+  bool first = true;
   for (int c = 0; c < n_colors; ++c) {
     const int c0 = color_ptr_host[c], cnt = color_ptr_host[c + 1] - c0;
     if (cnt <= 0) continue;
@@ -444,8 +455,9 @@ int launch_tp_sf(const int32_t* order, const int32_t* ngauss, int32_t n_nodes, c
       continue;
     }
     const int grid = (int)std::min<long long>(((long long)cnt * Sh::NP + 255) / 256, 16ll * gfe::sm_count());
-    tp_add_element_matrices<<<grid, 256, 0, s>>>(color_elems + c0, cnt, Sh::NF, Sh::NP, en, sf->pairs, rp, ci, slots,
-                                                 Kel + (size_t)c0 * Sh::NP, values, err);
+    gfe::launch_chained(!first, tp_add_element_matrices, grid, 256, s, color_elems + c0, cnt, Sh::NF, Sh::NP, en,
+                        sf->pairs, rp, ci, slots, Kel + (size_t)c0 * Sh::NP, values, err);
+    first = false;
     ++*launches;
   }
   gfe::scratch_free(Kel, s);

@@ -171,7 +171,7 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
       if (Ke) Ke[(size_t)r * ND + c] = v;
       if (sl && !(r >= 81 && c >= 81)) {
         const int pos = __ldg(sl + (size_t)r * ND + c);
-        if (pos >= 0) values[pos] += v;
+        if (pos >= 0) values[pos] = __ldcg(values + pos) + v;
         else gfe_raise(err, GFE_DEVERR_SLOT);
       }
     }
@@ -257,13 +257,25 @@ __global__ void mr_add_element_matrices(const int32_t* __restrict__ elems, int32
                                         double* __restrict__ values, unsigned* err) {
   constexpr int kEntries = ND * ND;
   const long long n = (long long)count * kEntries;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int pos = -2;  // nothing to add
+  double v = 0.0;
+  auto load = [&] {
     const int item = (int)(t / kEntries), k = (int)(t % kEntries);
-    if (k >= 81 * ND && k % ND >= 81) continue;
+    pos = -2;
+    if (k >= 81 * ND && k % ND >= 81) return;
     const size_t at = (size_t)__ldg(elems + item) * kEntries + k;
-    const int pos = __ldg(slots + at);
-    if (pos >= 0) values[pos] += __ldg(K + at);
-    else gfe_raise(err, GFE_DEVERR_SLOT);
+    pos = __ldg(slots + at);
+    v = __ldg(K + at);
+  };
+  if (t < n) load();
+  chain_wait();  // the colours' launches overlap: 9 x 8 x 7 elements 713 -> 680 us a call
+  chain_release();
+  while (t < n) {
+    if (pos >= 0) values[pos] = __ldcg(values + pos) + v;
+    else if (pos != -2) gfe_raise(err, GFE_DEVERR_SLOT);
+    t += (long long)gridDim.x * blockDim.x;
+    if (t < n) load();
   }
 }
 
@@ -328,11 +340,16 @@ extern "C" int gfe_mr_jacobian_fd(int32_t n_elem, const int32_t* eq2, const int3
   };
   if (K && n_elem > 0) {
     launch(0, n_elem, nullptr, nullptr);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool chained = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    bool first = true;
     for (int c = 0; add && c < n_colors; ++c) {
       const int c0 = color_ptr_host[c], cnt = color_ptr_host[c + 1] - c0;
       if (cnt <= 0) continue;
       const int grid = (int)std::min<long long>(((long long)cnt * ND * ND + 255) / 256, 16ll * gfe::sm_count());
-      mr_add_element_matrices<<<grid, 256, 0, s>>>(color_elems + c0, cnt, K, slots, values, err);
+      gfe::launch_chained(!first && chained, mr_add_element_matrices, grid, 256, s, color_elems + c0, cnt, K, slots, values,
+                          err);
+      first = false;
       ++launches;
     }
   } else {

@@ -306,14 +306,26 @@ __global__ void mr_add_element_vectors(const int32_t* __restrict__ elems, int32_
                                        const int32_t* __restrict__ eq2, const int32_t* __restrict__ elin, int32_t nq2,
                                        int64_t ndof, const double* __restrict__ vec, double* __restrict__ R) {
   const long long n = (long long)count * batch * ND;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t at = 0;
+  double v = 0.0;
+  auto load = [&] {
     const int r = (int)(t % ND);
     const long long ib = t / ND;
     const int item = (int)(ib / batch), b = (int)(ib % batch);
     const int e = __ldg(elems + item);
     const int64_t dof = r < 81 ? (int64_t)(r / NQ) * nq2 + __ldg(eq2 + (size_t)e * NQ + r % NQ)
                                : 3ll * nq2 + __ldg(elin + (size_t)e * NL + r - 81);
-    R[b * ndof + dof] += __ldcs(vec + ((size_t)item0 * batch) * ND + t);
+    at = b * ndof + dof;
+    v = __ldcs(vec + ((size_t)item0 * batch) * ND + t);
+  };
+  if (t < n) load();
+  chain_wait();  // the colours' launches overlap
+  chain_release();
+  while (t < n) {
+    R[at] = __ldcg(R + at) + v;
+    t += (long long)gridDim.x * blockDim.x;
+    if (t < n) load();
   }
 }
 
@@ -368,6 +380,7 @@ int run_batch(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t n
     ++*launches;
   };
   if (vec) launch(0, n_elem);
+  bool first = true;
   for (int c = 0; c < n_colors; ++c) {
     const int c0 = color_ptr_host[c], cnt = color_ptr_host[c + 1] - c0;
     if (cnt <= 0) continue;
@@ -376,7 +389,9 @@ int run_batch(int32_t n_elem, const int32_t* eq2, const int32_t* elin, int32_t n
       continue;
     }
     const int grid = (int)std::min<long long>(((long long)cnt * batch * ND + 255) / 256, 16ll * gfe::sm_count());
-    mr_add_element_vectors<<<grid, 256, 0, s>>>(color_elems + c0, c0, cnt, batch, eq2, elin, nq2, ndof, vec, R);
+    gfe::launch_chained(!first, mr_add_element_vectors, grid, 256, s, color_elems + c0, c0, cnt, batch, eq2, elin, nq2, ndof,
+                        vec, R);
+    first = false;
     ++*launches;
   }
   gfe::scratch_free(vec, s);
