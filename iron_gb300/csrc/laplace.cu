@@ -728,12 +728,12 @@ laplace_regular_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__
 // ---------------------------------------------------------------------------------------------
 // Float-float on Iron's regular mesh: element work in two kernels, then a row gather
 // ---------------------------------------------------------------------------------------------
-// The float-float element routine is ~13.6 k instructions of straight-line code per element; inside
+// The float-float element routine is about 9 k instructions of straight-line code per element; inside
 // the row-owning kernel its instruction stream does not fit the SM's instruction cache and warps
 // stall on instruction fetch.  Split, each kernel's code fits: the metric kernel forms the 8
 // Gauss-point metrics of every element once, the contraction kernel turns them into the 36 element
 // matrix entries, and the gather kernel sums each CSR row from the matrices of the elements around
-// its node, in the fixed order of the row-owning kernel (the values are bit-identical to it).
+// its node, in the fixed order of the row-owning kernel.
 
 // Gauss-point metrics of element layers [ez0, ez1) into metrics, tiled by 32 elements (entry k of
 // Gauss point g of element e at (48 (e / 32) + 8 k + g) 32 + e % 32).
@@ -1165,8 +1165,9 @@ const f2* element_matrices_f2(const void* ws, int32_t nx, int32_t ny, int32_t nz
 }
 
 // Node layers [l0, l1) (l0 a multiple of kRZ).  ws: caller workspace of regular_workspace_bytes(),
-// or NULL to allocate it on the stream; split: convert the coordinates into it first (the later
-// layer calls of one assembly reuse the converted array).  FP32: the row-owning tiled kernel.
+// or NULL to allocate it on the stream; split: convert the coordinates into it first; keep: the later
+// layer calls of one assembly reuse the converted array.  FP32: element matrices and the row gather, or
+// the row-owning tiled kernel.
 // Float-float: the element work of the element layers the rows read ([l0 - 1, l1) within the mesh;
 // a neighbouring slab on another stream may write the matrices of the layer between them at the
 // same time, with identical values), then the row gather.
