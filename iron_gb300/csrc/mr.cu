@@ -732,160 +732,136 @@ mr_gp_kernel(const int32_t* __restrict__ elems, int32_t count, const int32_t* __
   if (threadIdx.x == 0) tc::bulk_wait_read<0>();  // the stages may be gone once this thread exits
 }
 
-constexpr int kCThreads = 256;
-
-// u-p / p-u coefficients of one element: HvG[g][(mh,ms)] = sum_xi G[(g,xi)][ms] Hv_g[xi][mh] and
-// PvG[g][(nh,ns)] = sum_xi G[(g,xi)][ns] Pv_g[xi][nh] from the element's Gauss-point blocks Dg.
-__device__ __forceinline__ void form_up_coefficients(const float (*G)[28], const float* Dg, float (*HvG)[81],
-                                                     float (*PvG)[81]) {
-  for (int t = threadIdx.x; t < NG * 81; t += blockDim.x) {
-    const int g = t / 81, c = t % 81, h = c / 27, s = c % 27;
-    const float g0 = G[g * 3 + 0][s], g1 = G[g * 3 + 1][s], g2 = G[g * 3 + 2][s];
-    const float* H = Dg + kGPHv + (h * NG + g) * 4;
-    const float* P = Dg + kGPPv + (h * NG + g) * 4;
-    HvG[g][c] = g0 * H[0] + g1 * H[1] + g2 * H[2];
-    PvG[g][c] = g0 * P[0] + g1 * P[1] + g2 * P[2];
-  }
-}
-
-// The u-u block of one element's 89 x 89 matrix (row-major at Ke) from the staged product
-// C[(mh*3+nh)*27+ms][ns]; Iron mirrors its lower triangle into the upper one unless EXACT.  One
-// warp writes each row (consecutive lanes, consecutive entries).
-template <bool EXACT, typename KT, typename CT, int P>
-__device__ __forceinline__ void write_uu_block(KT* __restrict__ Ke, const CT (*C)[P]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int cq[3], cr[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    cq[j] = (lane + 32 * j) / 27;
-    cr[j] = (lane + 32 * j) % 27;
-  }
-  for (int r = warp; r < 81; r += nw) {
-    const int rq = r / 27, rr = r % 27;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int c = lane + 32 * j;
-      if (c < 81) {
-        const CT v = (EXACT || r >= c) ? C[(rq * 3 + cq[j]) * 27 + rr][cr[j]] : C[(cq[j] * 3 + rq) * 27 + cr[j]][rr];
-        Ke[r * ND + c] = (KT)v;
-      }
-    }
-  }
-}
-
-// The u-p and p-u blocks of one element's matrix as 27-term sums of HvG / PvG with the pressure
-// basis psi, and the zero p-p block.
-template <typename KT, typename CT>
-__device__ __forceinline__ void write_up_blocks(KT* __restrict__ Ke, const CT (*HvG)[81], const CT (*PvG)[81],
-                                                const CT (*psi)[NL]) {
-  for (int t = threadIdx.x; t < 2 * 81 * NL + NL * NL; t += blockDim.x) {
-    if (t < 81 * NL) {  // u rows, p columns
-      const int r = t / NL, b = t % NL;
-      CT s = CT(0);
-      for (int g = 0; g < NG; ++g) s += HvG[g][r] * psi[g][b];
-      Ke[r * ND + 81 + b] = (KT)s;
-    } else if (t < 2 * 81 * NL) {  // p rows, u columns
-      const int b = (t - 81 * NL) / 81, c = (t - 81 * NL) % 81;
-      CT s = CT(0);
-      for (int g = 0; g < NG; ++g) s += psi[g][b] * PvG[g][c];
-      Ke[(81 + b) * ND + c] = (KT)s;
-    } else {
-      const int q = t - 2 * 81 * NL;
-      Ke[(81 + q / NL) * ND + 81 + q % NL] = KT(0);
-    }
-  }
-}
-
-// Per element the u-u block is one product, as in the tensor-core kernel below:
-//   C[(mh,nh,ms)][ns] = sum_{(g,zeta)} A[(mh,nh,ms)][(g,zeta)] G[(g,zeta)][ns],
-//   A[(mh,nh,ms)][(g,zeta)] = sum_xi G[(g,xi)][ms] D_g[(mh,nh)][xi][zeta],
-// 243 x 81 by 81 x 27.  A is formed in two passes of kCRows rows ([k][row] in shared memory, so a
-// thread's four rows are one vector load), and each thread of the product accumulates a 4 x 4 tile
-// of C in registers: two vector loads per 16 FMAs.  u-p / p-u blocks and Iron's lower-triangle
-// mirror are formed from C, HvG and PvG while the element matrix is written.
-constexpr int kCRows = 128;                   // rows of A per pass
-constexpr int kCTileRows = kCRows / 4;        // 32 row groups of 4
-constexpr int kCTileCols = 7;                 // 7 column groups of 4 (27 columns, padded to 28)
-
-// The arrays read with vector loads (A, G) come first: their rows are multiples of 16 bytes.
-struct ContractShared {
-  float A[81][kCRows];     // A[(g,zeta)][row] of the current pass
-  float G[81][28];         // G[(g,xi)][ms]; column 27 zero
-  float C[2 * kCRows][28]; // C[(mh,nh,ms)][ns]
-  float HvG[NG][81];       // sum_xi G[(g,xi)][ms] Hv[xi][mh]  -> [g][(mh,ms)]
-  float PvG[NG][81];       // sum_xi G[(g,xi)][ns] Pv[xi][nh]  -> [g][(nh,ns)]
-  float Dg[kGPItem];       // this element's Gauss-point blocks
-  float psi[NG][NL];       // pressure basis at the Gauss points
-};
-static_assert(sizeof(float) * kCRows % 16 == 0 && sizeof(float) * 28 % 16 == 0, "vector rows");
-static_assert(sizeof(float) * 81 * kCRows % 16 == 0, "G follows A on a 16-byte boundary");
-
-__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+__device__ __forceinline__ void load4(const float* p, float* v) {
   const float4 q = *reinterpret_cast<const float4*>(p);
   v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
 
-// Element matrices of `count` elements into Kel[e][89][89] (element number e = elems[item]).
+// u-p / p-u blocks of one element into its matrix K: a warp has component h, its lanes ms; both are 27-term sums with
+// the pressure basis.
+template <typename Wait>
+__device__ __forceinline__ void up_blocks(int h, const float* Dg, const float (*G)[28], const float (*psi)[NL], float* K,
+                                          Wait wait) {
+  const int lane = threadIdx.x & 31, ms = min(lane, 26), r = h * 27 + ms;
+  const float4* H4 = reinterpret_cast<const float4*>(Dg + kGPHv) + h * NG;
+  const float4* P4 = reinterpret_cast<const float4*>(Dg + kGPPv) + h * NG;
+  float up[NL], pu[NL];
+#pragma unroll
+  for (int b = 0; b < NL; ++b) up[b] = pu[b] = 0.0f;
+#pragma unroll 3
+  for (int g = 0; g < NG; ++g) {
+    const float4 H = H4[g], P = P4[g];
+    const float g0 = G[g * 3][ms], g1 = G[g * 3 + 1][ms], g2 = G[g * 3 + 2][ms];
+    const float hg = g0 * H.x + g1 * H.y + g2 * H.z;
+    const float pg = g0 * P.x + g1 * P.y + g2 * P.z;
+    float q[NL];
+    load4(&psi[g][0], q);
+    load4(&psi[g][4], q + 4);
+#pragma unroll
+    for (int b = 0; b < NL; ++b) {
+      up[b] += hg * q[b];
+      pu[b] += q[b] * pg;
+    }
+  }
+  if (!wait()) return;
+  if (lane < 27) {
+#pragma unroll
+    for (int b = 0; b < NL; ++b) {
+      K[r * ND + 81 + b] = up[b];
+      K[(81 + b) * ND + r] = pu[b];
+    }
+  }
+}
+
+// CUDA-core form of the product of the tensor-core kernel below,
+//   C[(mh,nh,ms)][ns] = sum_{(g,zeta)} A[(mh,nh,ms)][(g,zeta)] G[(g,zeta)][ns],
+//   A[(mh,nh,ms)][(g,zeta)] = sum_xi G[(g,xi)][ms] D_g[(mh,nh)][xi][zeta],
+// 243 x 81 by 81 x 27.  A thread owns a row of C for two elements: it forms A's entries in registers as it goes and
+// takes a row of G, the same for all threads, by 16-byte broadcasts, 54 FMAs for seven.  Bound by the issue of the FMAs
+// (about 6,100 cycles an element and SM).  With A in shared memory and a 4 x 4 tile a thread, two vector loads for
+// 16 FMAs, 32^3 elements took 2,869 us, now 1,240.
+constexpr int kCThreads = 256;
+
+struct ContractShared {
+  alignas(16) float G[81][28];          // G[(g,xi)][ms]; column 27 zero
+  alignas(16) float psi[NG][NL];        // pressure basis at the Gauss points
+  alignas(16) float Dg[2][kGPItem];     // the two elements' Gauss-point blocks
+  alignas(16) float K[2][kKelF];        // and matrices
+};
+
+// Element matrices of `count` elements into Kel[e * kKelF] (element number e = elems[item]).
 template <bool EXACT>
-__global__ void __launch_bounds__(kCThreads)
+__global__ void __launch_bounds__(kCThreads, 2)
 mr_contract_kernel(const int32_t* __restrict__ elems, int32_t count, const Tables* __restrict__ Tg,
                    const float* __restrict__ gp, float* __restrict__ Kel) {
   extern __shared__ __align__(16) unsigned char craw[];
   ContractShared& S = *reinterpret_cast<ContractShared*>(craw);
-  const int tid = threadIdx.x;
-  for (int t = tid; t < 81 * 28; t += blockDim.x) {
+  const int tid = threadIdx.x, warp = tid >> 5;
+  for (int t = tid; t < 81 * 28; t += kCThreads) {
     const int k = t / 28, ms = t % 28;
     S.G[k][ms] = ms < 27 ? (float)Tg->dphi[k / 3][k % 3][ms] : 0.0f;
   }
-  for (int t = tid; t < NG * NL; t += blockDim.x) S.psi[t / NL][t % NL] = (float)Tg->psi[t / NL][t % NL];
-  const int rq = tid / kCTileCols, cq = tid % kCTileCols;  // product tile of this thread
-  const bool in_product = tid < kCTileRows * kCTileCols;
-  for (int item = blockIdx.x; item < count; item += gridDim.x) {
+  for (int t = tid; t < NG * NL; t += kCThreads) S.psi[t / NL][t % NL] = (float)Tg->psi[t / NL][t % NL];
+  // the zero p-p blocks and the padding behind the matrices are never written again
+  for (int t = tid; t < 2 * NL * NL; t += kCThreads) S.K[t / 64][(81 + t % 64 / NL) * ND + 81 + t % NL] = 0.0f;
+  if (tid < 2 * (kKelF - ND * ND)) S.K[tid & 1][ND * ND + (tid >> 1)] = 0.0f;
+  const int row = tid, pair = min(row / 27, 8), ms = row % 27, mh = pair / 3, nh = pair % 3, r = mh * 27 + ms;
+  for (int item = blockIdx.x * 2; item < count; item += gridDim.x * 2) {
+    const int n_live = min(2, count - item);
+    if (tid == 0) tc::bulk_wait_read<0>();  // the matrices of the round before have been read
     __syncthreads();
-    const float* src = gp + (size_t)item * kGPItem;
-    for (int t = tid; t < kGPItem; t += blockDim.x) S.Dg[t] = src[t];
+    const float4* src = reinterpret_cast<const float4*>(gp + (size_t)item * kGPItem);
+    float4* dst = reinterpret_cast<float4*>(&S.Dg[0][0]);
+    for (int t = tid; t < n_live * kGPItem / 4; t += kCThreads) dst[t] = __ldg(src + t);
     __syncthreads();
-    form_up_coefficients(S.G, S.Dg, S.HvG, S.PvG);
-    for (int pass = 0; pass < 2; ++pass) {
-      // operand rows [pass * kCRows, pass * kCRows + kCRows); rows past 242 are zero
-      for (int t = tid; t < 81 * kCRows; t += blockDim.x) {
-        const int k = t / kCRows, rl = t % kCRows, row = pass * kCRows + rl;
-        float v = 0.0f;
-        if (row < 243) {
-          const int pair = row / 27, ms = row % 27, g = k / 3, zeta = k % 3;
-          const float* D = &S.Dg[pair * kGPBlock + g * 9 + zeta];
-          v = S.G[g * 3 + 0][ms] * D[0] + S.G[g * 3 + 1][ms] * D[3] + S.G[g * 3 + 2][ms] * D[6];
-        }
-        S.A[k][rl] = v;
-      }
-      __syncthreads();
-      if (in_product) {
-        float acc[4][4];
+    if (row < 243) {
+      float acc[2][27];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+      for (int n = 0; n < 27; ++n) acc[0][n] = acc[1][n] = 0.0f;
+#pragma unroll 1
+      for (int g = 0; g < NG; ++g) {
+        const float g0 = S.G[g * 3][ms], g1 = S.G[g * 3 + 1][ms], g2 = S.G[g * 3 + 2][ms];
+        float a[2][3];
 #pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = 0.0f;
-#pragma unroll 3
-        for (int k = 0; k < 81; ++k) {
-          float av[4], bv[4];
-          load4(&S.A[k][rq * 4], av);
-          load4(&S.G[k][cq * 4], bv);
+        for (int l = 0; l < 2; ++l) {
+          const float* D = S.Dg[l] + pair * kGPBlock + g * 9;
 #pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
+          for (int z = 0; z < 3; ++z) a[l][z] = g0 * D[z] + g1 * D[3 + z] + g2 * D[6 + z];
         }
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int z = 0; z < 3; ++z) {
+          float b[28];
 #pragma unroll
-          for (int b = 0; b < 4; ++b) S.C[pass * kCRows + rq * 4 + a][cq * 4 + b] = acc[a][b];
+          for (int q = 0; q < 7; ++q) load4(&S.G[g * 3 + z][4 * q], b + 4 * q);
+#pragma unroll
+          for (int n = 0; n < 27; ++n) {
+            acc[0][n] += a[0][z] * b[n];
+            acc[1][n] += a[1][z] * b[n];
+          }
+        }
       }
-      __syncthreads();  // A is rewritten by the next pass
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        float* Kr = S.K[l] + r * ND + nh * 27;
+        float* Kc = S.K[l] + nh * 27 * ND + r;
+#pragma unroll
+        for (int n = 0; n < 27; ++n) {
+          // Iron mirrors the lower triangle into the upper one unless EXACT
+          if (EXACT || r >= nh * 27 + n) Kr[n] = acc[l][n];
+          if (!EXACT && r >= nh * 27 + n) Kc[n * ND] = acc[l][n];
+        }
+      }
     }
-    float* Ke = Kel + (size_t)__ldg(elems + item) * kKelF;
-    write_up_blocks<float, float>(Ke, S.HvG, S.PvG, S.psi);
-    write_uu_block<EXACT, float, float, 28>(Ke, S.C);
+    if (warp < 6) up_blocks(warp % 3, S.Dg[warp / 3], S.G, S.psi, S.K[warp / 3], [] { return true; });
+    tc::fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      for (int l = 0; l < n_live; ++l)
+        tc::bulk_copy_s2g(Kel + (size_t)__ldg(elems + item + l) * kKelF, S.K[l], kKelF * (uint32_t)sizeof(float));
+      tc::bulk_commit();
+    }
   }
+  if (tid == 0) tc::bulk_wait_read<0>();  // shared memory may be gone once this thread exits
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1086,38 +1062,13 @@ mr_contract_tc_kernel(const int32_t* __restrict__ elems, int32_t count, const Ta
       if (lane == 0) tc::mbar_arrive(&S.kfull);
     }
   } else if (warp < kTCForm + kTCUp) {
-    // u-p / p-u blocks: warp h has component h, lane ms; both are 27-term sums with the pressure basis
-    const int h = warp - kTCForm, ms = min(lane, 26), r = h * 27 + ms;
+    // u-p / p-u blocks
     for (int i = 0, item = blockIdx.x; item < count; ++i, item += gridDim.x) {
       if (!tc_wait(&S.dfull[i & 1], (uint32_t)(i >> 1) & 1u, err)) break;
-      const float4* H4 = reinterpret_cast<const float4*>(S.Dg[i & 1] + kGPHv) + h * NG;
-      const float4* P4 = reinterpret_cast<const float4*>(S.Dg[i & 1] + kGPPv) + h * NG;
-      float up[NL], pu[NL];
-#pragma unroll
-      for (int b = 0; b < NL; ++b) up[b] = pu[b] = 0.0f;
-#pragma unroll 3
-      for (int g = 0; g < NG; ++g) {
-        const float4 H = H4[g], P = P4[g];
-        const float g0 = S.G[g * 3][ms], g1 = S.G[g * 3 + 1][ms], g2 = S.G[g * 3 + 2][ms];
-        const float hg = g0 * H.x + g1 * H.y + g2 * H.z;
-        const float pg = g0 * P.x + g1 * P.y + g2 * P.z;
-        float psi[NL];
-        load4(&S.psi[g][0], *reinterpret_cast<float(*)[4]>(psi));
-        load4(&S.psi[g][4], *reinterpret_cast<float(*)[4]>(psi + 4));
-#pragma unroll
-        for (int b = 0; b < NL; ++b) {
-          up[b] += hg * psi[b];
-          pu[b] += psi[b] * pg;
-        }
-      }
-      if (i > 0 && !tc_wait(&S.kempty, (uint32_t)(i - 1) & 1u, err)) break;
-      if (lane < 27) {
-#pragma unroll
-        for (int b = 0; b < NL; ++b) {
-          S.K[r * ND + 81 + b] = up[b];
-          S.K[(81 + b) * ND + r] = pu[b];
-        }
-      }
+      bool ok = true;
+      up_blocks(warp - kTCForm, S.Dg[i & 1], S.G, S.psi, S.K,
+                [&] { return ok = i == 0 || tc_wait(&S.kempty, (uint32_t)(i - 1) & 1u, err); });
+      if (!ok) break;
       tc::fence_proxy_async();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&S.kfull);
@@ -1329,7 +1280,7 @@ int jacobian_f32(int mode, int32_t n_elem, const int32_t* eq2, const int32_t* el
       }
       continue;
     }
-    const int cgrid = std::min(cnt, 8 * sms);
+    const int cgrid = std::min((cnt + 1) / 2, 2 * sms);
     if (mode == 0)
       mr_contract_kernel<false><<<cgrid, kCThreads, csm, s>>>(elems + c0, cnt, T, gpbuf, Kel);
     else
