@@ -8,7 +8,7 @@
 //
 // The kernel is bound by the FP64 pipe.  Raising one displacement parameter changes one row of the
 // deformed gradient Z at each Gauss point by a multiple of the node's basis gradient, so a column
-// takes the point's stored state (Z, Z H, two rows of cofactors, the other entries of Z H Z^T), the
+// takes the point's stored state (Z, V = Z U^-1, two rows of cofactors, the other entries of Z H Z^T), the
 // changed row's products and the stress (about 150 operations a point), the difference of P to its
 // unperturbed value, and one sum-factorised transpose (mr_sf.cuh), instead of a whole residual with
 // dense tables and the reference metrics again (about 1,650 warp instructions a column; here 220).
@@ -52,8 +52,8 @@ struct FDShared {
   double node[2][81];        // reference and deformed nodes, [c * 27 + n]
   double p[NL];
   double X[243], Z[243];     // gradients [(c * 3 + k) * 27 + g]
-  double W[243], cof[243];   // Z H and cofactors of Z, same layout
-  double H[6][NQ], b[6][NQ]; // H and Z H Z^T (packed)
+  double V[243], cof[243];   // Z U^-1 and cofactors of Z, same layout
+  double h[6][NQ], b[6][NQ]; // factor of the reference metric, and Z H Z^T (packed)
   double P0[243];            // unperturbed P / delta, [(k * 3 + c) * 27 + g]
   double iJx[NQ], det[NQ], pg[NQ];
   double A[kSlots][243], B[kSlots][243];  // point differences, transposed stage by stage
@@ -104,7 +104,7 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
 
   // the unperturbed state of each point
   if (slot == 0) {
-    double X[3][3], Z[3][3], H[6], cof[3][3], W[3][3], b[6];
+    double X[3][3], Z[3][3], h[6], cof[3][3], V[3][3], Y[3][3], b[6];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -112,17 +112,10 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
         X[c][k] = S.X[(c * 3 + k) * NQ + g];
         Z[c][k] = S.Z[(c * 3 + k) * NQ + g];
       }
-    const double Jx = mr_sf::geometry(X, H), iJx = 1.0 / Jx;
+    const double Jx = mr_sf::geometry(X, h), iJx = 1.0 / Jx;
     const double det = mr_sf::cofactors(Z, cof);
     if (!(det > 0.0 && Jx > 0.0 && isfinite(det))) gfe_raise(err, GFE_DEVERR_JACOBIAN);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) mr_sf::row_h(Z[c], H, W[c]);
-    b[0] = mr_sf::dot3(W[0], Z[0]);
-    b[1] = mr_sf::dot3(W[1], Z[1]);
-    b[2] = mr_sf::dot3(W[2], Z[2]);
-    b[3] = mr_sf::dot3(W[0], Z[1]);
-    b[4] = mr_sf::dot3(W[0], Z[2]);
-    b[5] = mr_sf::dot3(W[1], Z[2]);
+    mr_sf::left_metric(Z, h, V, Y, b);
     const double p = mr_sf::point_pressure(g, S.p);
     double sg[6];
     mr_sf::stress(b, fabs(det) * iJx, p, c1, c2, (det > 0.0 ? 1.0 : -1.0) * mr_sf::point_weight(g) * idelta, sg);
@@ -132,13 +125,13 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         S.P0[(k * 3 + c) * NQ + g] = cof[0][k] * s0 + cof[1][k] * s1 + cof[2][k] * s2;
-        S.W[(c * 3 + k) * NQ + g] = W[c][k];
+        S.V[(c * 3 + k) * NQ + g] = V[c][k];
         S.cof[(c * 3 + k) * NQ + g] = cof[c][k];
       }
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      S.H[i][g] = H[i];
+      S.h[i][g] = h[i];
       S.b[i][g] = b[i];
     }
     S.iJx[g] = iJx;
@@ -184,7 +177,7 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
       const int c = slot % 3, ns = round * 3 + slot / 3, ca = c == 2 ? 0 : c + 1, cb = c == 0 ? 2 : c - 1;
       const int a1 = ns % 3, a2 = (ns / 3) % 3, a3 = ns / 9, g1 = g % 3, g2 = (g / 3) % 3, g3 = g / 9;
       const double z0 = S.node[1][c * NQ + ns], d = (z0 + delta) - z0;  // the step as it is taken
-      double zc[3], za[3], zb[3], wc[3], H[6];
+      double zc[3], za[3], zb[3], h[6];
       {
         const double v1 = S.v1[a1][g1] * d, v2 = S.v1[a2][g2], v3 = S.v1[a3][g3];
         const double v23 = v2 * v3;
@@ -193,8 +186,7 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
         zc[2] = fma(v1 * v2, S.d1[a3][g3], S.Z[(c * 3 + 2) * NQ + g]);
       }
 #pragma unroll
-      for (int i = 0; i < 6; ++i) H[i] = S.H[i][g];
-      mr_sf::row_h(zc, H, wc);
+      for (int i = 0; i < 6; ++i) h[i] = S.h[i][g];
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         za[k] = S.Z[(ca * 3 + k) * NQ + g];
@@ -212,11 +204,21 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
       const double det = mr_sf::dot3(zc, cof[0]);
       if (!(det > 0.0 && isfinite(det))) gfe_raise(err, GFE_DEVERR_JACOBIAN);
       double b[6];
-      b[0] = mr_sf::dot3(wc, zc);
+      {
+        double vc[3], yc[3], va[3], vb[3];
+        mr_sf::row_v(zc, h, vc);
+        mr_sf::row_e(vc, h, yc);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          va[k] = S.V[(ca * 3 + k) * NQ + g];
+          vb[k] = S.V[(cb * 3 + k) * NQ + g];
+        }
+        b[0] = mr_sf::dot3(yc, vc);
+        b[3] = mr_sf::dot3(yc, va);
+        b[4] = mr_sf::dot3(yc, vb);
+      }
       b[1] = S.b[ca][g];
       b[2] = S.b[cb][g];
-      b[3] = mr_sf::dot3(wc, za);
-      b[4] = mr_sf::dot3(wc, zb);
       b[5] = S.b[c == 0 ? 5 : (c == 1 ? 4 : 3)][g];
       const double wd = mr_sf::point_weight(g) * idelta, sgn = det > 0.0 ? 1.0 : -1.0;
       double sg[6];

@@ -52,22 +52,17 @@ struct PointShared {
 // Bz_m = sum_i B_im z_i, BB = sum_i z_i Bz_i^T, SS = sum_ij S_ij z_i z_j^T.
 __device__ __forceinline__ void exact_blocks(const double (&Z)[3][3], const double (&X)[3][3], double p, double w,
                                              double c1, double c2, double* __restrict__ o, unsigned* err) {
-  double H[6], z[3][3], B[6];
-  const double Jx = mr_sf::geometry(X, H);
+  double h[6], z[3][3], B[6];
+  const double Jx = mr_sf::geometry(X, h);
   const double det = mr_sf::cofactors(Z, z);
   if (!(det > 0.0) || !isfinite(det)) gfe_raise(err, GFE_DEVERR_JACOBIAN);
   const double J = fabs(det) / Jx;
   const double r = rcbrt(J), r2 = r * r, iJ = r2 * r;
   {
-    double W[3][3];
+    double V[3][3], Y[3][3];
+    mr_sf::left_metric(Z, h, V, Y, B);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) mr_sf::row_h(Z[c], H, W[c]);
-    B[0] = r2 * mr_sf::dot3(W[0], Z[0]);
-    B[1] = r2 * mr_sf::dot3(W[1], Z[1]);
-    B[2] = r2 * mr_sf::dot3(W[2], Z[2]);
-    B[3] = r2 * mr_sf::dot3(W[0], Z[1]);
-    B[4] = r2 * mr_sf::dot3(W[0], Z[2]);
-    B[5] = r2 * mr_sf::dot3(W[1], Z[2]);
+    for (int i = 0; i < 6; ++i) B[i] *= r2;
   }
   const double I1 = B[0] + B[1] + B[2];
   const double a1 = -2.0 * c2 * iJ, a2 = 2.0 * fma(I1, c2, c1) * iJ;

@@ -8,7 +8,7 @@
 // Both kernels are bound by the FP64 pipe.  A CTA takes eight elements, a thread a Gauss point (216
 // threads, 96 % of seven warps): gradients and their transposes are sum-factorised (mr_sf.cuh), the
 // point formulas work on Z H Z^T and cofactors (no square root, no division but one), and the
-// reference metrics H, J_x are formed once an element and kept in registers over the parameter sets
+// reference metric (a factor of H, J_x) is formed once an element and kept in registers over the parameter sets
 // of the CTA's share of the batch.  About 310 FP64 operations a point and parameter set for the
 // residual (1,650 warp instructions an element before, with dense tables, pow and divisions) and 520
 // for the adjoint.
@@ -43,21 +43,21 @@ struct ElemShared {
 //   Bbar = a1 (T B + B T) + a2 T + 2 c2 t2bar I,  t2bar = (T : B) / J,
 //   Jbar = -(2/3 Bbar : B + T : S) / J,  detbar = sign (Jbar / J_x + w Vp),
 //   Zbar = 2 J^(-2/3) Bbar Z H + detbar cof + the cofactors' cross products.
-__device__ __forceinline__ void point_vjp(const double (&Z)[3][3], const double (&H)[6], double iJx, double p, double w,
+__device__ __forceinline__ void point_vjp(const double (&Z)[3][3], const double (&h)[6], double iJx, double p, double w,
                                           double c1, double c2, const double (&V)[3][3], double Vp, double (&Zb)[3][3],
                                           double& pb, double& c1b, double& c2b) {
   double cof[3][3], W[3][3], B[6];
   const double det = mr_sf::cofactors(Z, cof);
   const double sgn = det > 0.0 ? 1.0 : -1.0, J = fabs(det) * iJx;
   const double r = rcbrt(J), r2 = r * r, iJ = r2 * r;
+  {
+    double Vz[3][3], Y[3][3];
+    mr_sf::left_metric(Z, h, Vz, Y, B);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) mr_sf::row_h(Z[c], H, W[c]);
-  B[0] = r2 * mr_sf::dot3(W[0], Z[0]);
-  B[1] = r2 * mr_sf::dot3(W[1], Z[1]);
-  B[2] = r2 * mr_sf::dot3(W[2], Z[2]);
-  B[3] = r2 * mr_sf::dot3(W[0], Z[1]);
-  B[4] = r2 * mr_sf::dot3(W[0], Z[2]);
-  B[5] = r2 * mr_sf::dot3(W[1], Z[2]);
+    for (int i = 0; i < 6; ++i) B[i] *= r2;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) mr_sf::row_zh(Y[c], h, W[c]);
+  }
   const double I1 = B[0] + B[1] + B[2];
   const double a1 = -2.0 * c2 * iJ, a2 = 2.0 * fma(I1, c2, c1) * iJ;
   const double ws = sgn * w;
@@ -204,14 +204,14 @@ mr_residual_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t bat
   }
   fetch(dep, b0);
   sync();
-  double H[6], Jx, iJx;
+  double h[6], Jx, iJx;
   {
     double X[3][3];
     mr_sf::field_gradients(g, on, S.u, S.A, S.B, S.grad, sync);
     sync();
 #pragma unroll
     for (int i = 0; i < 9; ++i) X[i / 3][i % 3] = S.grad[i * NQ + g];
-    Jx = mr_sf::geometry(X, H);
+    Jx = mr_sf::geometry(X, h);
     iJx = 1.0 / Jx;
   }
   const double w = mr_sf::point_weight(g);
@@ -229,17 +229,10 @@ mr_residual_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t bat
     const double p = mr_sf::point_pressure(g, S.p);
     const double c1 = __ldg(cpar + 2 * b), c2 = __ldg(cpar + 2 * b + 1);
     if constexpr (!ADJOINT) {
-      double cof[3][3], W[3][3], bq[6], sg[6];
+      double cof[3][3], V[3][3], Y[3][3], bq[6], sg[6];
       const double det = mr_sf::cofactors(Z, cof);
       if (on && !(det > 0.0 && Jx > 0.0 && isfinite(det))) bad = true;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) mr_sf::row_h(Z[c], H, W[c]);
-      bq[0] = mr_sf::dot3(W[0], Z[0]);
-      bq[1] = mr_sf::dot3(W[1], Z[1]);
-      bq[2] = mr_sf::dot3(W[2], Z[2]);
-      bq[3] = mr_sf::dot3(W[0], Z[1]);
-      bq[4] = mr_sf::dot3(W[0], Z[2]);
-      bq[5] = mr_sf::dot3(W[1], Z[2]);
+      mr_sf::left_metric(Z, h, V, Y, bq);
       mr_sf::stress(bq, fabs(det) * iJx, p, c1, c2, det > 0.0 ? w : -w, sg);
       sync();  // grad has been read
 #pragma unroll
@@ -260,7 +253,7 @@ mr_residual_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t bat
 #pragma unroll
       for (int i = 0; i < 9; ++i) V[i % 3][i / 3] = S.grad[i * NQ + g];
       const double Vp = mr_sf::point_pressure(g, S.p);
-      point_vjp(Z, H, iJx, p, w, c1, c2, V, Vp, Zb, pb, c1b, c2b);
+      point_vjp(Z, h, iJx, p, w, c1, c2, V, Vp, Zb, pb, c1b, c2b);
       sync();
 #pragma unroll
       for (int k = 0; k < 3; ++k)

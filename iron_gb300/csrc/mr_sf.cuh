@@ -220,7 +220,7 @@ __device__ __forceinline__ double point_pressure(int g, const double* p) {
 // With Z = dz/dxi, X = dx/dxi and Iron's fibre-free material frame A = (N^T X)^-1, N the columns of X
 // normalised (src/coordinate_routines.F90:3841-3947), the residual's Cauchy stress
 // (src/finite_elasticity_routines.F90:6985-7061) depends on F = Z A only through F F^T = Z H Z^T with
-// H = A A^T = (G D^-1 G)^-1, G = X^T X, D = diag(G): no square root, six numbers a point.  With
+// H = A A^T: six numbers a point (geometry below).  With
 // J = J_z / J_x, r = J^(-1/3) and B = r^2 Z H Z^T,
 //   sigma = dev((t1 B^2 + t2 B) / J) + p I,  t1 = -2 c2,  t2 = 2 (c1 + tr(B) c2),
 // and the first Piola form of the residual is P[xi][m] = w J_z (Z^-1 sigma)[xi][m] =
@@ -241,11 +241,17 @@ __device__ __forceinline__ double cofactors(const double (&Z)[3][3], double (&co
   return Z[0][0] * cof[0][0] + Z[0][1] * cof[0][1] + Z[0][2] * cof[0][2];
 }
 
-// H (packed) and J_x of a reference gradient matrix.  H = (G D^-1 G)^-1 with D = diag(G): the
-// diagonal of K = G D^-1 G is G_ii plus small terms, so H's entries differ by the rounding of one or
-// two products; rounding common to all of them only scales B, which the deviator does not amplify
-// (near the undeformed state it amplifies differences between B's diagonal entries).
-__device__ __forceinline__ double geometry(const double (&X)[3][3], double (&H)[6]) {
+// Factor of the reference metric and J_x of a reference gradient matrix X.  H = A A^T with A = (N^T X)^-1 and
+// N^T X = D^-1/2 G (G = X^T X, D = diag G), so K = H^-1 = G D^-1 G is the Gram matrix of G's columns in the weights
+// 1/D: orthogonalising them gives K = U^T diag(d) U with U unit upper triangular, and
+//   Z H Z^T = V diag(e) V^T,  V = Z U^-1,  e = 1 / d,      h = u01 u02 u12 e0 e1 e2,
+// without a square root.  V is found by substitution and never multiplies out H: K has the fourth power of X's
+// condition, and inverting it, or forming Z H Z^T from any H, cancels that many digits.  Relative error of the stress
+// term P at a point of an element sheared by 3 (10) in two planes: 3e-14 (3e-12), as with Iron's own order of
+// operations; with H = (G D^-1 G)^-1 5e-12 (6e-8), with H = G^-1 D G^-1 1e-12 (1e-8).  On a box U is the identity and
+// e0, e1, e2 differ by the rounding of a product or two: near the undeformed state the deviator amplifies differences
+// between B's diagonal entries, so the diagonal is formed as G_kk r^2 plus small terms.
+__device__ __forceinline__ double geometry(const double (&X)[3][3], double (&h)[6]) {
   double G[6];
 #pragma unroll
   for (int i = 0; i < 3; ++i) G[i] = X[0][i] * X[0][i] + X[1][i] * X[1][i] + X[2][i] * X[2][i];
@@ -254,35 +260,59 @@ __device__ __forceinline__ double geometry(const double (&X)[3][3], double (&H)[
   G[5] = X[0][1] * X[0][2] + X[1][1] * X[1][2] + X[2][1] * X[2][2];
   const double g01 = G[0] * G[1], d = 1.0 / (g01 * G[2]);
   const double i0 = G[1] * G[2] * d, i1 = G[0] * G[2] * d, i2 = g01 * d;  // 1 / G_kk
-  const double a3 = G[3] * i1, a4 = G[4] * i2, b3 = G[3] * i0, b5 = G[5] * i2, c4 = G[4] * i0, c5 = G[5] * i1;
-  double K[6];
-  K[0] = G[0] + fma(G[3], a3, G[4] * a4);
-  K[1] = G[1] + fma(G[3], b3, G[5] * b5);
-  K[2] = G[2] + fma(G[4], c4, G[5] * c5);
-  K[3] = fma(2.0, G[3], G[5] * a4);
-  K[4] = fma(2.0, G[4], G[5] * a3);
-  K[5] = fma(2.0, G[5], G[4] * b3);
-  H[0] = K[1] * K[2] - K[5] * K[5];
-  H[1] = K[0] * K[2] - K[4] * K[4];
-  H[2] = K[0] * K[1] - K[3] * K[3];
-  H[3] = K[4] * K[5] - K[3] * K[2];
-  H[4] = K[3] * K[5] - K[4] * K[1];
-  H[5] = K[3] * K[4] - K[5] * K[0];
-  const double q = 1.0 / (K[0] * H[0] + K[3] * H[3] + K[4] * H[4]);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) H[i] *= q;
+  // first column (G00, G01, G02), weighted (1, w1, w2)
+  const double w1 = G[3] * i1, w2 = G[4] * i2;
+  h[3] = 1.0 / (G[0] + fma(G[3], w1, G[4] * w2));
+  h[0] = fma(2.0, G[3], w2 * G[5]) * h[3];
+  h[1] = fma(2.0, G[4], w1 * G[5]) * h[3];
+  // the others less their part along it: (a0, G11 ra, a2), (b0, b1, G22 rb)
+  const double a0 = fma(-h[0], G[0], G[3]), ra = fma(-h[0], w1, 1.0), a2 = fma(-h[0], G[4], G[5]);
+  const double b0 = fma(-h[1], G[0], G[4]), b1 = fma(-h[1], G[3], G[5]), rb = fma(-h[1], w2, 1.0);
+  const double a0i = a0 * i0, a2i = a2 * i2;
+  h[4] = 1.0 / fma(G[1] * ra, ra, fma(a0, a0i, a2 * a2i));
+  h[2] = fma(a0i, b0, fma(ra, b1, a2 * rb)) * h[4];
+  // the third less its part along the second: (c0, c1, G22 rc)
+  const double c0 = fma(-h[2], a0, b0), c1 = fma(-h[2], G[1] * ra, b1), rc = fma(-h[2], a2i, rb);
+  h[5] = 1.0 / fma(G[2] * rc, rc, fma(c0 * i0, c0, c1 * i1 * c1));
   return fabs(X[0][0] * (X[1][1] * X[2][2] - X[1][2] * X[2][1]) + X[0][1] * (X[1][2] * X[2][0] - X[1][0] * X[2][2]) +
               X[0][2] * (X[1][0] * X[2][1] - X[1][1] * X[2][0]));
 }
 
-// row of Z times H
-__device__ __forceinline__ void row_h(const double (&z)[3], const double (&H)[6], double (&w)[3]) {
-  w[0] = z[0] * H[0] + z[1] * H[3] + z[2] * H[4];
-  w[1] = z[0] * H[3] + z[1] * H[1] + z[2] * H[5];
-  w[2] = z[0] * H[4] + z[1] * H[5] + z[2] * H[2];
+// row of V = Z U^-1
+__device__ __forceinline__ void row_v(const double (&z)[3], const double (&h)[6], double (&v)[3]) {
+  v[0] = z[0];
+  v[1] = fma(-v[0], h[0], z[1]);
+  v[2] = fma(-v[0], h[1], fma(-v[1], h[2], z[2]));
+}
+// row of V diag(e)
+__device__ __forceinline__ void row_e(const double (&v)[3], const double (&h)[6], double (&y)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) y[k] = v[k] * h[3 + k];
+}
+// row of Z H = V diag(e) U^-T from the row of V diag(e)
+__device__ __forceinline__ void row_zh(const double (&y)[3], const double (&h)[6], double (&w)[3]) {
+  w[2] = y[2];
+  w[1] = fma(-h[2], w[2], y[1]);
+  w[0] = fma(-h[0], w[1], fma(-h[1], w[2], y[0]));
 }
 __device__ __forceinline__ double dot3(const double (&a)[3], const double (&b)[3]) {
   return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+}
+
+// Z H Z^T (packed) from Z and the metric's factor, with V and Y = V diag(e)
+__device__ __forceinline__ void left_metric(const double (&Z)[3][3], const double (&h)[6], double (&V)[3][3],
+                                            double (&Y)[3][3], double (&b)[6]) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    row_v(Z[c], h, V[c]);
+    row_e(V[c], h, Y[c]);
+  }
+  b[0] = dot3(Y[0], V[0]);
+  b[1] = dot3(Y[1], V[1]);
+  b[2] = dot3(Y[2], V[2]);
+  b[3] = dot3(Y[0], V[1]);
+  b[4] = dot3(Y[0], V[2]);
+  b[5] = dot3(Y[1], V[2]);
 }
 
 // scale * (dev((t1 B^2 + t2 B) / J) + p I) from b = Z H Z^T (packed) and J
