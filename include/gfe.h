@@ -275,7 +275,9 @@ int gfe_laplace_assemble_regular(int32_t nx, int32_t ny, int32_t nz, const doubl
  * the form to capture into a CUDA graph.  The element matrices are formed once and the rows gathered from
  * them.  The workspace holds them (288 bytes an element for GFE_FP64, 144 for GFE_MIXED), for the FP32-pipe
  * precisions also room for converted coordinates and, for GFE_MIXED_DF, every element's Gauss-point metrics
- * (float-float, 672 bytes an element in all).  workspace may be NULL: GFE_FP64 then runs a kernel that
+ * (float-float, 672 bytes an element in all).  All of it is written; before version 200 GFE_FP64 wrote nothing
+ * and GFE_MIXED 12 bytes a node, so a buffer must be sized by the function for the precision it is used with.
+ * workspace may be NULL: GFE_FP64 then runs a kernel that
  * needs none, the others allocate and free it on `stream`, as gfe_laplace_assemble_regular does (GFE_MIXED,
  * without memory for it, runs on the converted coordinates alone). */
 int64_t gfe_laplace_regular_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, int32_t precision);
@@ -289,7 +291,9 @@ int gfe_laplace_assemble_regular_ws(int32_t nx, int32_t ny, int32_t nz, const do
  * convert_coords: convert the coordinates into the workspace first (needed in the first call of an
  * assembly; later calls of the same assembly pass 0 and reuse it; requires a workspace).  An empty
  * range (layer_begin == layer_end) with convert_coords only converts, so that slab calls on
- * several streams can all start once the conversion is done. */
+ * several streams can all start once the conversion is done.
+ * The workspace is written as far as 12 bytes a node for GFE_MIXED, gfe_laplace_regular_workspace_bytes for
+ * GFE_MIXED_DF and not at all for GFE_FP64, also when the range is the whole mesh. */
 int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* coords, const double* kappa,
                                         const int32_t* row_ptr, double* values, float* values32, double* rhs,
                                         int32_t precision, void* workspace, int32_t layer_begin, int32_t layer_end,

@@ -98,7 +98,7 @@ int sm_count() {
 
 }  // namespace gfe
 
-extern "C" int gfe_version(void) { return 100; }
+extern "C" int gfe_version(void) { return 200; }
 
 extern "C" int gfe_clear_stale_error(void) { return (int)cudaGetLastError(); }
 

@@ -1224,14 +1224,15 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
 
 // FP64 with a workspace, whole mesh: the element matrices once (the tiled kernel forms a third of them
 // twice in its halo), then the row gather: 90 x 77 x 101 elements 2.56 ms (colour kernel on general
-// connectivity) -> 1.27 ms, 4 x 4 x 4 0.71 -> 0.06 ms (eight colours, each one chain of 90 us).  Without a workspace, or for a slab, the row-owning tiled kernel, which needs no memory.
+// connectivity) -> 1.27 ms, 4 x 4 x 4 0.71 -> 0.05 ms (eight colours, each one chain of 90 us).  Without a workspace,
+// and for layer calls (keep), whose FP64 form has never used one, the row-owning tiled kernel, which needs no memory.
 // Below 64 elements an SM (two warps of four elements to each SM sub-partition, 8 lanes an element) the
 // kernel with eight lanes an element has the shorter chain.
 template <>
 int launch_regular<double>(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const double* coords,
                            const double* kappa, const int32_t* rp, double* values, float* values32, double* rhs,
-                           unsigned* err, void* ws, int32_t l0, int32_t l1, bool, bool) {
-  if (ws && l0 == 0 && l1 == nz + 1) {
+                           unsigned* err, void* ws, int32_t l0, int32_t l1, bool, bool keep) {
+  if (ws && !keep && l0 == 0 && l1 == nz + 1) {
     double* Kel = static_cast<double*>(ws);
     const long long E = (long long)nx * ny * nz;
     if (E <= 64ll * gfe::sm_count())
@@ -1359,7 +1360,7 @@ int assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* co
     rc = launch_regular<f2>(s, nx, ny, nz, coords, kappa, row_ptr, values, values32, rhs, err, workspace, l0,
                             l1, cv, keep);
   gfe::stage_end(GFE_STAGE_LAPLACE_ELEMENTS, prof, s,
-                 precision == GFE_MIXED_DF ? 3 : (l0 == 0 && l1 == nz + 1 && (workspace || precision == GFE_MIXED) ? 2 : 1));
+                 precision == GFE_MIXED_DF ? 3 : (!keep && (workspace || precision == GFE_MIXED) ? 2 : 1));
   if (rc) return rc;
   GFE_LAUNCH_CHECK(fn);
   return GFE_OK;
