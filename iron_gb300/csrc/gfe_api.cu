@@ -231,6 +231,12 @@ void* stage_begin(int stage, cudaStream_t s) {
 void stage_end(int stage, void* token, cudaStream_t s, int launches) {
   if (!token) return;
   auto* pr = static_cast<std::pair<cudaEvent_t, cudaEvent_t>*>(token);
+  if (launches <= 0) {  // nothing ran
+    cudaEventDestroy(pr->first);
+    cudaEventDestroy(pr->second);
+    delete pr;
+    return;
+  }
   cudaEventRecord(pr->second, s);
   std::lock_guard<std::mutex> lk(g_prof_mu);
   for (int i = 0; i < launches; ++i) {

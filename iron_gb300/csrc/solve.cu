@@ -351,7 +351,7 @@ __global__ void norm2_kernel(int n, const double* __restrict__ v, double* red, S
 }
 
 // Sliced-ELL copy of a CSR matrix with short rows, for the CG products: slices of 32 consecutive
-// rows, each stored column-major and padded to its longest row (column 0 marks padding), so entry
+// rows, each stored column-major and padded to its longest row (SellIndex<IT>::pad marks padding), so entry
 // k of row r sits at sptr[r / 32] + 32 k + r % 32.  A lane per row then reads one contiguous
 // 128-byte line per warp and entry, and no row waits on its bounds; the per-row CSR forms wait on
 // the row bounds, then on the entries, then on the gathers.  Built inside each solve call from the
@@ -482,6 +482,8 @@ struct MinresScalars {
 
 constexpr int kNodalBatch = 8;  // entries a lane loads at once in the MINRES products
 
+constexpr long long kResidentBytes = 100ll << 20;  // matrix of a resident solve: within the 129 MB L2
+
 }  // namespace
 
 #include "krylov_resident.cuh"
@@ -489,10 +491,12 @@ constexpr int kNodalBatch = 8;  // entries a lane loads at once in the MINRES pr
 namespace {
 
 // Builds the sliced-ELL copy of (rp, ci, val) in two scratch allocations bufs[0], bufs[1] (the
-// caller frees both with scratch_free).  Synchronises the stream once (the copy's size).
+// caller frees both with scratch_free).  Synchronises the stream once (the copy's size).  *resident is cleared when
+// the copy, with its padding, is larger than kResidentBytes; when only the resident kernels would use it
+// (resident_only), none is made then.
 template <typename TM>
 int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaStream_t s, void* bufs[2],
-               SellCopy<TM>* out) {
+               SellCopy<TM>* out, bool* resident, bool resident_only) {
   using namespace gfe;
   bufs[0] = bufs[1] = nullptr;
   const long long n_slices = (n + kSell - 1) / kSell;
@@ -516,6 +520,11 @@ int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaS
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) { scratch_free(head, s); return set_error(GFE_ERR_CUDA, "sliced-ELL size: %s", cudaGetErrorString(e)); }
   out->is_near = size.reach <= 32767;
+  if (size.total * (long long)(sizeof(TM) + (out->is_near ? 2 : 4)) > kResidentBytes) *resident = false;
+  if (resident_only && !*resident) {
+    scratch_free(head, s);
+    return GFE_OK;
+  }
   const size_t val_bytes = (sizeof(TM) * (size_t)size.total + 255) & ~size_t(255);
   char* body = nullptr;
   if ((rc = scratch_alloc((void**)&body, val_bytes + (out->is_near ? 2 : 4) * (size_t)size.total + 256, s, "sliced-ELL copy"))) {
@@ -543,7 +552,6 @@ int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaS
 // slower); FP64 with 2 lanes a row, 14 entries a lane and two rows a group (152 us, 216 us for one
 // thread a row with the per-row loop; the shuffle of the 2-lane sum is one FP64 add a row).
 // Longer FP32 rows keep the per-row loop with 16 or 32 lanes; longer FP64 rows one thread a row.
-constexpr long long kResidentBytes = 100ll << 20;  // matrix of a resident solve: within the 129 MB L2
 constexpr int kSpmvShort32 = -1;
 constexpr int kSpmvShort64 = -2;
 
@@ -615,14 +623,23 @@ int run_cg(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, const TM
 // CG iterations in resident kernels of at most kResidentIters each, until convergence; *ran is false when
 // the first launch was not possible.
 constexpr int kResidentIters = 200;
+constexpr int kCgRounds = 3;  // slices a warp at most
+
+int cg_resident_grid(int n) {
+  return std::min({gfe::sm_count(), kResMaxGrid, ((n + kSell - 1) / kSell + kCgWorkers - 1) / kCgWorkers});
+}
+// slices a warp for n rows: up to kCgRounds (452,000 rows on 152 SMs) the resident kernels take them
+int cg_resident_rounds(int n) {
+  const int slices = (n + kSell - 1) / kSell, grid = cg_resident_grid(n);
+  return ((slices + grid - 1) / grid + kCgWorkers - 1) / kCgWorkers;
+}
 
 template <typename TM, typename TV>
 int run_cg_resident(cudaStream_t s, int n, const SellCopy<TM>& A, const uint8_t* fixed, const TV* dinv, TV* x, TV* r,
                     TV* z, TV* p, TV* q, Scalars* sc, Scalars* sc_host, ResBarrier* bar, int max_iters, bool fresh,
                     bool* ran) {
-  const int slices = (n + kSell - 1) / kSell;
-  const int grid = std::min({gfe::sm_count(), kResMaxGrid, (slices + kCgWorkers - 1) / kCgWorkers});
-  const int rounds = ((slices + grid - 1) / grid + kCgWorkers - 1) / kCgWorkers;  // slices a warp
+  const int grid = cg_resident_grid(n), rounds = cg_resident_rounds(n);
+  static_assert(kCgRounds == 3, "the instances below");
   *ran = true;
   for (int done = 0; done < max_iters;) {
     const int k = std::min(kResidentIters, max_iters - done);
@@ -635,7 +652,7 @@ int run_cg_resident(cudaStream_t s, int n, const SellCopy<TM>& A, const uint8_t*
                                sc, bar, k, fresh))
     const bool ok = rounds == 1 ? GFE_CG_RESIDENT(1) : (rounds == 2 ? GFE_CG_RESIDENT(2) : (rounds == 3 && GFE_CG_RESIDENT(3)));
 #undef GFE_CG_RESIDENT
-    gfe::stage_end(GFE_STAGE_SPMV, prof, s, 1);
+    gfe::stage_end(GFE_STAGE_SPMV, prof, s, ok ? 1 : 0);
     if (!ok) {
       *ran = done > 0;
       return done > 0 ? gfe::set_error(GFE_ERR_CUDA, "launch of the resident CG kernel failed") : GFE_OK;
@@ -695,13 +712,14 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
   const int chunk = 50;
   const bool short_rows = (double)(nnz1 - 1) / n <= 32.0;
   // short rows: the FP32 iterations of the mixed solve run on a sliced-ELL copy of values32 (128^3
-  // Laplace: 104 -> 91 us a product, 103 -> 93 ms a solve); the FP64 product, bound by FP64 work
+  // Laplace: 104 -> 91 us a product, 103 -> 93 ms a solve); the launched FP64 product, bound by FP64 work
   // as much as by its loads, gained nothing from it and keeps the batched CSR form
   const bool use_sell = precision == GFE_MIXED && (double)(nnz1 - 1) / n <= 32.0 && n >= 4 * kSell;
   // short rows and a matrix that stays in L2: the iterations run in resident kernels on the sliced-ELL copy
-  // (64^3, 59 MB in FP32: a solve takes 6.5 ms instead of 16.4; 128^3, 460 MB, is bound by HBM, where the launched
-  // form already runs at the bandwidth)
-  bool resident = short_rows && (long long)(nnz1 - 1) * (precision == GFE_FP64 ? 12 : 8) <= kResidentBytes;
+  // (64^3, 59 MB in FP32: a solve takes 5.0 ms instead of 16.4; 128^3, 460 MB, is bound by HBM, where the launched
+  // form already runs at the bandwidth).  The rule is settled before a copy is made for it, but for the padding
+  bool resident = short_rows && cg_resident_rounds(n) <= kCgRounds &&
+                  (long long)(nnz1 - 1) * (precision == GFE_FP64 ? 12 : 8) <= kResidentBytes;
   void* sell_bufs[2] = {nullptr, nullptr};
 
   // scratch: dinv, r64, then vector set (FP64 or FP32) and an FP32 copy of dinv
@@ -755,7 +773,7 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
     // and continues along the same search direction (a reliable update).
     double r2_start = b2;
     SellCopy<double> sell{};
-    if (resident && build_sell<double>(n, row_ptr, col_idx, values, s, sell_bufs, &sell)) resident = false;
+    if (resident && build_sell<double>(n, row_ptr, col_idx, values, s, sell_bufs, &sell, &resident, true)) resident = false;
     for (int round = 0; round < 4 && rc == GFE_OK; ++round) {
       cg_start<double, double><<<grid, kThreads, 0, s>>>(n, r64, dinv, r, z, p, x, false, round > 0, red, red2, sc,
                                                          0.25 * rtol * rtol * b2 / r2_start);
@@ -790,7 +808,13 @@ extern "C" int gfe_cg_solve(int32_t n, const int32_t* row_ptr, const int32_t* co
     // all take 727-742 iterations; 1e-3 needs the fewest updates.
     const double inner_rtol = 1e-3;
     SellCopy<float> sell{};
-    if (use_sell || resident) rc = build_sell<float>(n, row_ptr, col_idx, values32, s, sell_bufs, &sell);
+    if (use_sell || resident) {
+      rc = build_sell<float>(n, row_ptr, col_idx, values32, s, sell_bufs, &sell, &resident, !use_sell);
+      if (rc && !use_sell) {  // the launched form needs no copy
+        resident = false;
+        rc = GFE_OK;
+      }
+    }
     for (int outer = 0; outer < 200 && rc == GFE_OK; ++outer) {
       if (outer > 0) {
         residual64(short_rows, grid, s, n, row_ptr, col_idx, values, f, fixed, x, r64);
@@ -1347,7 +1371,7 @@ int run_minres_resident(cudaStream_t s, int n, const int32_t* rp, const int32_t*
     else if (nodes) ok = lpr == 16 ? GFE_MINRES_RESIDENT(16, 3) : GFE_MINRES_RESIDENT(32, 3);
     else ok = lpr == 16 ? GFE_MINRES_RESIDENT(16, 1) : GFE_MINRES_RESIDENT(32, 1);
 #undef GFE_MINRES_RESIDENT
-    gfe::stage_end(GFE_STAGE_SPMV, prof, s, 1);
+    gfe::stage_end(GFE_STAGE_SPMV, prof, s, ok ? 1 : 0);
     if (!ok) {
       *ran = j > 1;
       return j > 1 ? gfe::set_error(GFE_ERR_CUDA, "launch of the resident MINRES kernel failed") : GFE_OK;
