@@ -48,6 +48,41 @@ class SolveInfo:
     precision: str
 
 
+_ASK_FOR_ROOM = 2 << 30
+
+
+def _capturing(stream) -> bool:
+    """Whether `stream` is being captured into a graph."""
+    with torch.cuda.stream(stream):
+        return torch.cuda.is_current_stream_capturing()
+
+
+class _Workspace:
+    """A device buffer that an assembly keeps, with the stream of its last use.  It is allocated as memory of the
+    stream that uses it first; another stream waits for that use to end and is recorded with the allocator, so that
+    neither a later use nor its release overlaps one in flight."""
+
+    def __init__(self, buf, stream):
+        self.buf = buf  # None: there is no room for it
+        self.handle = stream.cuda_stream
+        self.done = None  # event after the last use, None once the host has waited for it
+
+    def take(self, stream) -> None:
+        """Before a use on another stream than the last."""
+        if self.buf is None or _capturing(stream):
+            return
+        if self.done is not None:
+            stream.wait_event(self.done)
+        self.buf.record_stream(stream)
+        self.handle = stream.cuda_stream
+
+    def mark(self, stream) -> None:
+        """After a use that the host does not wait for."""
+        if not _capturing(stream):
+            self.done = torch.cuda.Event()
+            self.done.record(stream)
+
+
 class LaplaceAssembly:
     """Device-resident Laplace problem on a hexahedral mesh of tensor-product Lagrange elements.
 
@@ -187,37 +222,44 @@ class LaplaceAssembly:
             return self.values
         if path == "regular" and self.regular is None:
             raise GfeError(-1, "the regular-mesh kernel needs Iron's regular generated mesh")
+        st = stream if stream is not None else torch.cuda.current_stream()
         ws = None
         if path == "auto":
             path = "general" if self.regular is None else "regular"
             if path == "regular" and prec == GFE_FP64:
                 # element matrices in a workspace, then a row gather; without room for it (288 bytes an
                 # element) the colour kernel, which computes each element once as well
-                try:
-                    ws = self._regular_workspace(prec)
-                except torch.OutOfMemoryError:
-                    path = "general"
+                ws = self._regular_workspace(prec, st, stream is None)
+                if ws.buf is None:
+                    path, ws = "general", None
         if path == "regular":
             nx, ny, nz = self.regular
             if prec != GFE_FP64:
-                try:
-                    ws = self._regular_workspace(prec)
-                except torch.OutOfMemoryError:
-                    # FP32 runs without room for the element matrices (144 bytes an element), on a smaller scratch
-                    if prec != GFE_MIXED:
-                        raise
-            _lib.call("gfe_laplace_assemble_regular_ws", nx, ny, nz, _lib.ptr(self.coords), _lib.ptr(self.kappa),
-                      _lib.ptr(self.row_ptr), _lib.ptr(self.values), _lib.ptr(v32), _lib.ptr(self.rhs), prec,
-                      _lib.ptr(ws), _lib.stream_handle(stream))
+                ws = self._regular_workspace(prec, st, stream is None)
+            if ws is None or ws.buf is not None:
+                _lib.call("gfe_laplace_assemble_regular_ws", nx, ny, nz, _lib.ptr(self.coords), _lib.ptr(self.kappa),
+                          _lib.ptr(self.row_ptr), _lib.ptr(self.values), _lib.ptr(v32), _lib.ptr(self.rhs), prec,
+                          None if ws is None else _lib.ptr(ws.buf), _lib.stream_handle(st))
+            else:
+                # FP32 without room for the element matrices (144 bytes an element): the layer form, over all
+                # layers, which takes the rounded coordinates alone
+                ws = self._regular_workspace("coords32", st, stream is None)
+                _lib.call("gfe_laplace_assemble_regular_layers", nx, ny, nz, _lib.ptr(self.coords),
+                          _lib.ptr(self.kappa), _lib.ptr(self.row_ptr), _lib.ptr(self.values), _lib.ptr(v32),
+                          _lib.ptr(self.rhs), prec, _lib.ptr(ws.buf), 0, nz + 1, 1, _lib.stream_handle(st))
         else:
             cp = self.colour_ptr
             _lib.call("gfe_laplace_assemble", self.n_elements, self.n_nodes, _lib.ptr(self.elem_nodes),
                       _lib.ptr(self.coords), _lib.ptr(self.kappa), _lib.ptr(self.colour_elems),
                       cp.ctypes.data_as(C.c_void_p), len(cp) - 1, _lib.ptr(self.row_ptr), _lib.ptr(self.col_idx),
                       self.nnz, _lib.ptr(self.values), _lib.ptr(v32), _lib.ptr(self.rhs), prec,
-                      _lib.stream_handle(stream))
+                      _lib.stream_handle(st))
         if check:
-            _lib.raise_device_errors("gfe_laplace_assemble", stream)
+            if ws is not None:
+                ws.done = None  # the check waits for the stream
+            _lib.raise_device_errors("gfe_laplace_assemble", st)
+        elif ws is not None:
+            ws.mark(st)
         return self.values
 
     def assemble_generalised(self, conductivity, fibre=None, stream=None, check: bool = True) -> torch.Tensor:
@@ -270,31 +312,54 @@ class LaplaceAssembly:
         nx, ny, nz = self.regular
         prec = PRECISIONS[precision]
         # the slabs of FP64 need no workspace, those of FP32 the rounded coordinates alone
-        if prec == GFE_FP64:
-            ws = None
-        elif prec == GFE_MIXED:
-            ws = self.__dict__.setdefault("_ws_cache", {}).get("coords32")
-            if ws is None:
-                ws = self._ws_cache["coords32"] = torch.empty(12 * self.n_nodes + 256, dtype=torch.uint8,
-                                                              device=self.device)
-        else:
-            ws = self._regular_workspace(prec)
+        ws = None if prec == GFE_FP64 else self._regular_workspace("coords32" if prec == GFE_MIXED else prec, st, False)
         _lib.call("gfe_laplace_assemble_regular_host", nx, ny, nz, _lib.host_ptr(coords_host),
                   _lib.host_ptr(kappa_host), _lib.ptr(self.coords), _lib.ptr(self.kappa), _lib.ptr(self.row_ptr),
-                  _lib.ptr(self.values), _lib.host_ptr(values_host), _lib.ptr(self.rhs), prec, _lib.ptr(ws),
-                  int(slab_layers), _lib.stream_handle(st))
+                  _lib.ptr(self.values), _lib.host_ptr(values_host), _lib.ptr(self.rhs), prec,
+                  _lib.ptr(ws.buf if ws is not None else None), int(slab_layers), _lib.stream_handle(st))
+        if ws is not None:
+            ws.mark(st)
         return values_host
 
-    def _regular_workspace(self, prec: int) -> torch.Tensor:
-        """Device workspace of the regular-mesh kernels for precision code `prec`, allocated once per
-        precision and kept (every element's matrix, 288 bytes an element in FP64 and 144 in FP32; float-float:
-        also its Gauss-point metrics, 672 bytes)."""
-        cache = self.__dict__.setdefault("_ws_cache", {})
-        if prec not in cache:
-            nx, ny, nz = self.regular
-            wb = int(_lib.load().gfe_laplace_regular_workspace_bytes(nx, ny, nz, prec))
-            cache[prec] = torch.empty(max(wb, 16), dtype=torch.uint8, device=self.device)
-        return cache[prec]
+    def __getstate__(self):
+        # a copy has workspaces of its own: two assemblies may run on different streams at the same time
+        return {k: v for k, v in self.__dict__.items() if k != "_ws_cache"}
+
+    def _regular_workspace(self, key, stream, current: bool) -> _Workspace:
+        """Device workspace of the regular-mesh kernels for use on `stream` (current: torch's current one),
+        allocated once and kept; key: a precision code (every element's matrix, 288 bytes an element in FP64 and
+        144 in FP32; float-float: also its Gauss-point metrics, 672 bytes) or "coords32" (the rounded coordinates).
+        FP64 and FP32 run without their element matrices, so there those may take up a quarter of the free memory
+        at most (asked for beyond _ASK_FOR_ROOM bytes, as it takes 100 us; fewer have to be there) and `buf` is None
+        otherwise; that is settled at the first call, so that later ones neither ask again nor change their bits."""
+        cache = self.__dict__.get("_ws_cache")
+        if cache is None:
+            cache = self._ws_cache = {}
+        ws = cache.get(key)
+        if ws is not None:
+            if ws.handle != stream.cuda_stream:
+                ws.take(stream)
+            return ws
+        optional = key in (GFE_FP64, GFE_MIXED)
+        if key == GFE_FP64 and (torch.cuda.is_current_stream_capturing() if current else _capturing(stream)):
+            return _Workspace(None, stream)  # nothing is allocated for FP64 while a graph is captured
+        if key == "coords32":
+            nbytes = 12 * self.n_nodes + 256
+        else:
+            nbytes = max(int(_lib.load().gfe_laplace_regular_workspace_bytes(*self.regular, key)), 16)
+        buf = None
+        if not (optional and nbytes > _ASK_FOR_ROOM and nbytes > torch.cuda.mem_get_info(self.device)[0] // 4):
+            try:
+                if current:
+                    buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+                else:
+                    with torch.cuda.stream(stream):
+                        buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            except torch.OutOfMemoryError:
+                if not optional:
+                    raise
+        cache[key] = ws = _Workspace(buf, stream)
+        return ws
 
     def element_matrices(self, precision: str = "fp64", stream=None) -> torch.Tensor:
         if self.tensor_product:
