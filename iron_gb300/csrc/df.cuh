@@ -73,7 +73,8 @@ __device__ __forceinline__ void finish(float&) {}
 
 // Forms without the final renormalisation (8 operations a sum instead of 11), for chains whose values do not cancel:
 // `lo` then reaches a few ulp(hi), and only products of two such values lose by it (they drop lo lo), so a
-// value is renormalised before it enters a product with another one.
+// value is renormalised before it enters a product with another one.  Sums that cancel on sheared or flat elements (the
+// Gram products and their minors) are normalised: left raw, they cost 7 and 8 % in the error of an element sheared by 10.
 __device__ __forceinline__ f2 add_raw(f2 a, f2 b) {
   accum(a, b);
   return a;
@@ -87,15 +88,11 @@ template <typename T>
 __device__ __forceinline__ T minor2(T a, T b, T c, T d) {
   return a * b - c * d;
 }
-__device__ __forceinline__ f2 minor2(f2 a, f2 b, f2 c, f2 d) { return sub_raw(a * b, c * d); }
+__device__ __forceinline__ f2 minor2(f2 a, f2 b, f2 c, f2 d) { return renorm(sub_raw(a * b, c * d)); }
 template <typename T>
 __device__ __forceinline__ T dot3(T a, T b, T c, T d, T e, T f) {
   return a * b + c * d + e * f;
 }
-__device__ __forceinline__ f2 dot3(f2 a, f2 b, f2 c, f2 d, f2 e, f2 f) {
-  return renorm(add_raw(add_raw(a * b, c * d), e * f));
-}
-
 __device__ __forceinline__ f2& operator+=(f2& a, f2 b) { return a = a + b; }
 __device__ __forceinline__ f2& operator-=(f2& a, f2 b) { return a = a - b; }
 __device__ __forceinline__ bool operator>(f2 a, f2 b) { return a.hi > b.hi || (a.hi == b.hi && a.lo > b.lo); }
@@ -141,6 +138,29 @@ __device__ __forceinline__ f2 f2_split(double a) {
   const int rest = t == 0 ? 0 : (int)((unsigned)r & 0x1fffffffu) - (1 << 28);
   const float lo = (float)rest * __uint_as_float((unsigned)(e - 52 + 127) << 23);  // a power of two: exact
   return {__uint_as_float(hi | sign), sign ? -lo : lo};
+}
+
+// A double as three floats h + a + b without loss: the leading 24, the next 22 and the last 7 bits of the mantissa,
+// cut off with integer operations (see f32_to_f64_exact).  Magnitudes up to 2^-80 become zero (or less than 2^-102),
+// those of 2^128 and more, infinities and NaNs something not finite.
+struct f3 {
+  float h, a, b;
+};
+__device__ __forceinline__ f3 f3_exact(double x) {
+  constexpr unsigned kLeast = (1023u - 80u) << 20, kInf = (1023u + 128u) << 20;
+  const unsigned w1 = (unsigned)__double2hiint(x), w0 = (unsigned)__double2loint(x);
+  const unsigned t = min(max(w1 & 0x7fffffffu, kLeast), kInf);
+  const unsigned h = (__funnelshift_l(w0, t, 3) - (896u << 23)) | (w1 & 0x80000000u);
+  const unsigned ea = (h & 0xff800000u) - (23u << 23), eb = ea - (22u << 23);  // signed powers of two
+  const float a = __uint_as_float(ea | ((w0 >> 6) & 0x7ffffeu)), b = __uint_as_float(eb | ((w0 & 0x7fu) << 16));
+  return {t > kLeast ? __uint_as_float(h) : 0.0f, __fsub_rn(a, __uint_as_float(ea)), __fsub_rn(b, __uint_as_float(eb))};
+}
+// Their difference: exact up to the rounding of its last part, so an edge keeps its digits however far from the
+// origin it lies and whatever the size of the others.
+__device__ __forceinline__ f2 edge(f3 y, f3 x) {
+  const f2 h = two_sum(y.h, -x.h);
+  const f2 s = fast_two_sum(h.hi, __fsub_rn(y.a, x.a));
+  return {s.hi, __fadd_rn(__fadd_rn(s.lo, h.lo), __fsub_rn(y.b, x.b))};
 }
 
 // precision-generic helpers used by the element kernels

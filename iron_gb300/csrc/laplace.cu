@@ -69,13 +69,31 @@ __device__ __forceinline__ constexpr double metric_scale() {
 // Metrics of one trilinear hexahedron at its 8 Gauss points: M[g] = GU Jacobian w kappa (times
 // metric_scale) as the six entries 00 11 22 01 02 12 of the symmetric 3x3 matrix.  x[c][m]: coordinates of local node m
 // (m = m1 + 2 m2 + 4 m3, Iron's local node order).  Returns false if det(GL) <= 0.
+// In float-float they may come as doubles, whose edges are then formed exactly (f3).
 template <typename T>
-__device__ __forceinline__ bool hex8_metrics(const T (&x)[3][8], T kappa, T p, T q, T (&M)[8][6]) {
+__device__ __forceinline__ T edge(T y, T x) {
+  return y - x;
+}
+template <typename T, typename X>
+struct EdgeOf {
+  using type = X;
+  static __device__ __forceinline__ X from(X x) { return x; }
+};
+template <>
+struct EdgeOf<f2, double> {
+  using type = f3;
+  static __device__ __forceinline__ f3 from(double x) { return f3_exact(x); }
+};
+template <typename T, typename X>
+__device__ __forceinline__ bool hex8_metrics(const X (&x)[3][8], T kappa, T p, T q, T (&M)[8][6]) {
   const T zero = from_double<T>(0.0);
   // Jacobian columns: Jt[c][a][gd1][gd2]
   T Jt[3][3][2][2];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
+    typename EdgeOf<T, X>::type y[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) y[m] = EdgeOf<T, X>::from(x[c][m]);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const int d1 = a == 0 ? 1 : 0, d2 = a == 2 ? 1 : 2;
@@ -85,7 +103,7 @@ __device__ __forceinline__ bool hex8_metrics(const T (&x)[3][8], T kappa, T p, T
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int m0 = (i << d1) | (j << d2);
-          D[i][j] = x[c][m0 | (1 << a)] - x[c][m0];
+          D[i][j] = edge(y[m0 | (1 << a)], y[m0]);
         }
       if constexpr (std::is_same<T, double>::value) {
         // d0 p + d1 q = d0 + q (d1 - d0) and d0 q + d1 p = d0 + p (d1 - d0): three operations for both
@@ -546,31 +564,15 @@ __device__ __forceinline__ f2 acc_add(f2 a, f2 b) {
 }
 
 // Coordinates are read in the element arithmetic type: the FP32-pipe precisions take them from a
-// copy split once per node (float or float-float), so no element converts FP64 values itself.  The float-float copy
-// is relative to the middle node (elements use differences only), which halves what the split to 48 bits loses on a
-// mesh at the origin and keeps a mesh far from it; it is formed with integer operations (129^3 nodes: 51 us by
-// conversions).
-template <typename T>
-struct CoordSplit {
-  __device__ __forceinline__ CoordSplit(const double*, long long) {}
-  __device__ __forceinline__ T operator()(double x) const { return from_double<T>(x); }
-};
-template <>
-struct CoordSplit<f2> {
-  double r;
-  __device__ __forceinline__ CoordSplit(const double* xc, long long n) : r(__ldg(xc + n / 2)) {
-    if (!isfinite(r)) r = 0.0;
-  }
-  __device__ __forceinline__ f2 operator()(double x) const { return f2_split(x - r); }
-};
+// copy rounded once per node in FP32 (layer calls), so no element converts FP64 values itself; the float-float metric
+// kernel takes the doubles apart with integer operations (layer calls: a copy of the doubles).
 // nodes [a, b) of n, three components
 template <typename T>
 __global__ void split_coords(long long n, long long a, long long b, const double* __restrict__ in, T* __restrict__ out) {
   for (int c = 0; c < 3; ++c) {
-    const CoordSplit<T> split(in + c * n, n);
 #pragma unroll 4
     for (long long i = a + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < b; i += (long long)gridDim.x * blockDim.x)
-      out[c * n + i] = split(__ldg(in + c * n + i));
+      out[c * n + i] = from_double<T>(__ldg(in + c * n + i));
   }
 }
 
@@ -737,9 +739,15 @@ laplace_regular_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__
 
 // Gauss-point metrics of element layers [ez0, ez1) into metrics, tiled by 32 elements (entry k of
 // Gauss point g of element e at (48 (e / 32) + 8 k + g) 32 + e % 32).
+//
+// Coordinates are read as doubles and each element takes its 24 apart (about 15 integer and FP32 operations each).
+// A copy split to float-float once per node, 40 us at 128^3, has to round to 48 bits, and relative to whatever point
+// that is: relative to the origin it loses digits on elements far from it, relative to the mesh's middle node on small
+// elements at its edge (a mesh graded by 1e-6 towards the origin: error 1.4e-12 of the matrix's norm relative to the middle
+// node, 2.8e-14 relative to the origin, 7.7e-15 here; 128^3 jittered cubes 3.0e-14, 5.8e-14, 4.0e-15).
 template <typename T>
 __global__ void __launch_bounds__(128)
-laplace_metric_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__ coords,
+laplace_metric_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __restrict__ coords,
                       const double* __restrict__ kappa, T* __restrict__ metrics, int32_t ez0, int32_t ez1,
                       unsigned* err) {
   const long long EXY = (long long)nx * ny;
@@ -750,12 +758,12 @@ laplace_metric_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__ 
   for (long long e = ez0 * EXY + blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ez1 * EXY;
        e += (long long)gridDim.x * blockDim.x) {
     const long long ex = e % nx, ey = (e / nx) % ny, ez = e / EXY;
-    T x[3][8];
+    double x[3][8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const long long n = (ex + (m & 1)) + (ey + ((m >> 1) & 1)) * NX + (ez + (m >> 2)) * NXY;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c][m] = load_coord(coords + c * N + n);
+      for (int c = 0; c < 3; ++c) x[c][m] = __ldg(coords + c * N + n);
     }
     const double kd = kappa ? __ldg(kappa + e) : 1.0;
     if (!isfinite(kd)) nonfinite = true;
@@ -1132,7 +1140,7 @@ constexpr int kContractThreads = 128;
 
 // Float-float element work of element layers [ez0, ez1): metric kernel, then contraction kernel,
 // each element once, into the workspace's element-matrix array.
-void launch_elements_f2(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const f2* ct, const double* kappa,
+void launch_elements_f2(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const double* coords, const double* kappa,
                         void* ws, int32_t ez0, int32_t ez1, unsigned* err) {
   if (ez1 <= ez0) return;
   const long long cnt = (long long)(ez1 - ez0) * nx * ny;
@@ -1142,7 +1150,7 @@ void launch_elements_f2(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, cons
   const int cgrid = (int)std::min<long long>((cnt + kContractThreads - 1) / kContractThreads, 60ll * gfe::sm_count());
   f2* metrics = reinterpret_cast<f2*>(static_cast<char*>(ws) + regular_coords_bytes(nx, ny, nz, GFE_MIXED_DF));
   f2* Kel = metrics + regular_metric_entries(nx, ny, nz);
-  laplace_metric_kernel<f2><<<grid, kSplitThreads, 0, s>>>(nx, ny, nz, ct, kappa, metrics, ez0, ez1, err);
+  laplace_metric_kernel<f2><<<grid, kSplitThreads, 0, s>>>(nx, ny, nz, coords, kappa, metrics, ez0, ez1, err);
   laplace_contract_kernel<f2><<<cgrid, kContractThreads, 0, s>>>(nx, ny, nz, metrics, Kel, ez0, ez1);
 }
 
@@ -1204,10 +1212,13 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
       return GFE_OK;
     }
   }
-  T* ct = reinterpret_cast<T*>(base);
-  if (split || !ws) split_coords<T><<<4 * gfe::sm_count(), 256, 0, s>>>(n_nodes, 0, n_nodes, coords, ct);
+  // what later layer calls read: rounded coordinates, or a copy of the doubles
+  using C = typename std::conditional<DF, double, T>::type;
+  C* ct = reinterpret_cast<C*>(base);
+  const bool convert = (split || !ws) && (keep || !DF);
+  if (convert) split_coords<C><<<4 * gfe::sm_count(), 256, 0, s>>>(n_nodes, 0, n_nodes, coords, ct);
   if constexpr (DF) {
-    launch_elements_f2(s, nx, ny, nz, ct, kappa, base, std::max(l0 - 1, 0), std::min(l1, nz), err);
+    launch_elements_f2(s, nx, ny, nz, keep ? ct : coords, kappa, base, std::max(l0 - 1, 0), std::min(l1, nz), err);
     launch_gather<f2>(s, nx, ny, nz, element_matrices_f2(base, nx, ny, nz), rp, values, values32, rhs, l0, l1);
   } else {
     const size_t smem = 2 * 36 * kRThreads * sizeof(typename StoreOf<T>::type);
@@ -1341,7 +1352,7 @@ int assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* co
       return gfe::set_error(GFE_ERR_ARG, "%s: an empty layer range needs a workspace and convert_coords", fn);
     const long long n = (nx + 1ll) * (ny + 1) * (nz + 1);
     if (precision == GFE_MIXED) split_coords<float><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (float*)workspace);
-    else if (precision == GFE_MIXED_DF) split_coords<f2><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (f2*)workspace);
+    else if (precision == GFE_MIXED_DF) split_coords<double><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (double*)workspace);
     GFE_LAUNCH_CHECK(fn);
     return GFE_OK;
   }
@@ -1463,11 +1474,6 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
   // every pipeline stream starts after the work already on `stream`
   GFE_CUDA_TRY(cudaEventRecord(ev[0], s));
   for (cudaStream_t t : {hp->in, hp->comp[0], hp->comp[1], hp->out}) GFE_CUDA_TRY(cudaStreamWaitEvent(t, ev[0], 0));
-  // the middle node's coordinates, which the others are split relative to, ahead of their layer
-  if (coords_host && precision == GFE_MIXED_DF)
-    for (int c = 0; c < 3; ++c)
-      GFE_CUDA_TRY(cudaMemcpyAsync(coords + c * N + N / 2, coords_host + c * N + N / 2, sizeof(double),
-                                   cudaMemcpyHostToDevice, hp->in));
   long long node_hi = 0, elem_hi = 0;  // node / element layers uploaded so far
   const int cvt_grid = 2 * gfe::sm_count();
   for (int i = 0; i < n_slabs; ++i) {
@@ -1485,8 +1491,6 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
       if (precision == GFE_MIXED)
         split_coords<float><<<cvt_grid, 256, 0, hp->in>>>(N, node_hi * NXY, nh * NXY, coords,
                                                           static_cast<float*>(workspace));
-      else if (precision == GFE_MIXED_DF)
-        split_coords<f2><<<cvt_grid, 256, 0, hp->in>>>(N, node_hi * NXY, nh * NXY, coords, static_cast<f2*>(workspace));
       node_hi = nh;
     }
     if (kappa_host && eh > elem_hi) {
@@ -1497,7 +1501,7 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
     // float-float: the element work of the slab's own element layers on the input stream, in slab
     // order, so the next slab's rows find the matrices of the element layer below them written
     if (precision == GFE_MIXED_DF)
-      launch_elements_f2(hp->in, nx, ny, nz, static_cast<const f2*>(workspace), kappa, workspace, l0,
+      launch_elements_f2(hp->in, nx, ny, nz, coords, kappa, workspace, l0,
                          std::min<int32_t>(l1, nz), err);
     GFE_CUDA_TRY(cudaEventRecord(ev_in, hp->in));
     // the slab on alternating compute streams: one slab's last wave overlaps the next one's first
