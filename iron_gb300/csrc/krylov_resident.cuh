@@ -491,15 +491,17 @@ minres_resident(int n, int n_node, const int32_t* __restrict__ rp, const int32_t
               }
             }
           } else {
+            // rows that shared memory does not hold are read again every iteration: they should stay in the L2 (an
+            // 11^3 tangent, 56 MB in FP32: 11.7 us an iteration; 13.9 with evict-first loads, FP64 36 and 57)
             for (int t0 = sub; t0 < len; t0 += kNodalBatch * LPR) {
               int c[kNodalBatch];
               TM v[NC][kNodalBatch];
 #pragma unroll
               for (int u = 0; u < kNodalBatch; ++u) {
                 const int k = t0 + u * LPR;
-                c[u] = k < len ? __ldcs(ci + k0[0] + k) : 0;
+                c[u] = k < len ? __ldg(ci + k0[0] + k) : 0;
 #pragma unroll
-                for (int m = 0; m < NC; ++m) v[m][u] = k < len && (m == 0 || multi) ? __ldcs(val + k0[m] + k) : TM(0);
+                for (int m = 0; m < NC; ++m) v[m][u] = k < len && (m == 0 || multi) ? __ldg(val + k0[m] + k) : TM(0);
               }
 #pragma unroll
               for (int u = 0; u < kNodalBatch; ++u)
