@@ -324,7 +324,8 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
 // CTAs with the longest rows (a triquadratic node has 89 to 402 entries, by lines of the mesh) held the others up at
 // the first barrier: an FP64 Newton solve at 8^3, bound by the FP64 pipe, takes 45.6 instead of 51.0 ms.  An FP32
 // group costs its latency more than its entries: with 32 entries' worth as in FP64 an iteration took 10.4 us, with
-// 256 it takes the 9.4 of equal numbers.  `nodes` groups of NC rows, then single rows; e0, total: entries of the nodes'
+// 256 it takes the 9.4 of equal numbers.  (Between 3^3 and 13^3 a quarter of either value changes an iteration by -7
+// to +6 %, four times by -10 to +16 %.)  `nodes` groups of NC rows, then single rows; e0, total: entries of the nodes'
 // rows of one component, and the cost of all groups.
 template <int NC>
 __device__ int minres_share(const int32_t* __restrict__ rp, int nodes, int n_groups, long long e0, long long c0,

@@ -483,6 +483,11 @@ struct MinresScalars {
 constexpr int kNodalBatch = 8;  // entries a lane loads at once in the MINRES products
 
 constexpr long long kResidentBytes = 100ll << 20;  // matrix of a resident solve: within the 129 MB L2
+// and its copy with padding, where no other form uses one (FP64).  60,000 rows, one of 200 (420) entries in each slice,
+// 126 MB (232): a solve takes 2.03 (3.26) ms resident and 2.19 (2.99) launched; 200,000 rows, 360 MB: 3.39 and 2.88.
+// In mixed precision both forms run on the copy and the resident one is no slower at any padding (255 MB: 2.83 and
+// 4.16 ms; 186 MB: 4.70 and 4.78)
+constexpr long long kResidentPadded = 150ll << 20;
 
 }  // namespace
 
@@ -491,9 +496,8 @@ constexpr long long kResidentBytes = 100ll << 20;  // matrix of a resident solve
 namespace {
 
 // Builds the sliced-ELL copy of (rp, ci, val) in two scratch allocations bufs[0], bufs[1] (the
-// caller frees both with scratch_free).  Synchronises the stream once (the copy's size).  *resident is cleared when
-// the copy, with its padding, is larger than kResidentBytes; when only the resident kernels would use it
-// (resident_only), none is made then.
+// caller frees both with scratch_free).  Synchronises the stream once (the copy's size).  *resident is cleared and no
+// copy made when only the resident kernels would use it (resident_only) and it is larger than kResidentPadded.
 template <typename TM>
 int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaStream_t s, void* bufs[2],
                SellCopy<TM>* out, bool* resident, bool resident_only) {
@@ -520,8 +524,8 @@ int build_sell(int n, const int32_t* rp, const int32_t* ci, const TM* val, cudaS
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) { scratch_free(head, s); return set_error(GFE_ERR_CUDA, "sliced-ELL size: %s", cudaGetErrorString(e)); }
   out->is_near = size.reach <= 32767;
-  if (size.total * (long long)(sizeof(TM) + (out->is_near ? 2 : 4)) > kResidentBytes) *resident = false;
-  if (resident_only && !*resident) {
+  if (resident_only && size.total * (long long)(sizeof(TM) + (out->is_near ? 2 : 4)) > kResidentPadded) {
+    *resident = false;
     scratch_free(head, s);
     return GFE_OK;
   }
@@ -1352,7 +1356,8 @@ int run_minres_resident(cudaStream_t s, int n, const int32_t* rp, const int32_t*
   const bool nodes = nodal.n_node > 0 && nodal.nc == 3;
   const int n_node = nodes ? nodal.n_node : 0, groups = nodes ? n - 2 * n_node : n, sms = gfe::sm_count();
   // lanes a group: FP64 8 (the shuffle sums run on the FP64 pipe); FP32 a warp, or half a warp where that lets
-  // one pass of a CTA cover its groups.  At least eight groups a CTA: below that the barriers cost more
+  // one pass of a CTA cover its groups (half a warp beyond that as well: 9^3 9.5 -> 11.5 us an iteration, 12^3
+  // 14.6 -> 19.1).  At least eight groups a CTA: below that the barriers cost more
   const int grid = std::min({sms, kResMaxGrid, (groups + 7) / 8});
   const int share = (groups + grid - 1) / grid;  // groups a CTA on average
   const int lpr = std::is_same<TV, double>::value ? 8 : (share > kMinresWorkers && share <= 2 * kMinresWorkers ? 16 : 32);

@@ -1,5 +1,5 @@
-"""Which CG systems run in the resident kernels: at most three slices of 32 rows a warp (31 warps an SM) and a
-sliced-ELL copy, with its padding, of at most 100 MB.  The profiler counts one launch per resident kernel of up to 200
+"""Which CG systems run in the resident kernels: at most three slices of 32 rows a warp (31 warps an SM) and, in FP64,
+where no other form uses it, a sliced-ELL copy of at most 150 MB with its padding.  The profiler counts one launch per resident kernel of up to 200
 iterations and one per product of the launched form (chunks of 50), so the count says which form ran and that
 no other one was tried first; the solution is checked by its residual formed in torch (1 % above the tolerance is
 far more than the rounding of forming it again)."""
@@ -74,7 +74,7 @@ def test_form_by_size_and_padding(gfe_cuda, case, mixed):
     n, nnz = sys[0].numel() - 1, sys[1].numel()
     assert nnz / n <= 32 and 12 * nnz <= 100 << 20
     it, launches = _solve(sys, mixed)
-    if case in ("three slices", "padding fits"):
+    if case in ("three slices", "padding fits") or (case == "too much padding" and mixed):
         # at least one kernel for each 200 iterations and each restart of the refinement, and no product launched
         assert math.ceil(it / 200) <= launches <= math.ceil(it / 200) + 40 and launches < it
     else:
