@@ -66,6 +66,7 @@ class _Workspace:
         self.buf = buf  # None: there is no room for it
         self.handle = stream.cuda_stream
         self.done = None  # event after the last use, None once the host has waited for it
+        self.event = None
 
     def take(self, stream) -> None:
         """Before a use on another stream than the last."""
@@ -76,11 +77,14 @@ class _Workspace:
         self.buf.record_stream(stream)
         self.handle = stream.cuda_stream
 
-    def mark(self, stream) -> None:
-        """After a use that the host does not wait for."""
-        if not _capturing(stream):
-            self.done = torch.cuda.Event()
-            self.done.record(stream)
+    def mark(self, stream, current: bool) -> None:
+        """After a use that the host does not wait for (current: `stream` is torch's current one)."""
+        if torch.cuda.is_current_stream_capturing() if current else _capturing(stream):
+            return
+        if self.event is None:
+            self.event = torch.cuda.Event()
+        self.event.record(stream)
+        self.done = self.event
 
 
 class LaplaceAssembly:
@@ -259,7 +263,7 @@ class LaplaceAssembly:
                 ws.done = None  # the check waits for the stream
             _lib.raise_device_errors("gfe_laplace_assemble", st)
         elif ws is not None:
-            ws.mark(st)
+            ws.mark(st, stream is None)
         return self.values
 
     def assemble_generalised(self, conductivity, fibre=None, stream=None, check: bool = True) -> torch.Tensor:
@@ -318,7 +322,7 @@ class LaplaceAssembly:
                   _lib.ptr(self.values), _lib.host_ptr(values_host), _lib.ptr(self.rhs), prec,
                   _lib.ptr(ws.buf if ws is not None else None), int(slab_layers), _lib.stream_handle(st))
         if ws is not None:
-            ws.mark(st)
+            ws.mark(st, stream is None)
         return values_host
 
     def __getstate__(self):
