@@ -48,7 +48,7 @@ def parse():
                          "assembly (32^3); mr_newton: load-stepped Newton solve of the uniaxial stretch (32^3); "
                          "mr_adjoint: batched residual adjoint (16^3 x 64); serve: request stream")
     ap.add_argument("--path", default="auto", choices=["auto", "regular", "general"],
-                    help="assembly kernel: regular-mesh tiled kernel (auto for generated meshes) or colour scatter")
+                    help="assembly kernel: regular-mesh kernels (auto for generated meshes) or colour scatter")
     ap.add_argument("--no-solve", action="store_true")
     ap.add_argument("--headline-only", action="store_true",
                     help="skip the Mooney-Rivlin keys of the headline line (for profiling runs)")
@@ -155,7 +155,7 @@ def measured_peaks():
 
 
 def profile_traffic_per_unit(kernel: str):
-    """DRAM bytes (read + write) per element of `kernel` (e.g. "laplace_regular_kernel<f2>") from
+    """DRAM bytes (read + write) per element of `kernel` (e.g. "laplace_gather_kernel<f2>") from
     the committed ncu summary profiles/laplace_kernels_traffic.txt, if it lists the kernel."""
     p = ROOT / "profiles" / "laplace_kernels_traffic.txt"
     if not p.exists():
@@ -387,16 +387,18 @@ def run_gfe(args):
                 head = prec
     T = timings[head]
     if path == "auto":
-        used_path = "general" if (head == "fp64" or A.regular is None) else "regular"
+        used_path = "general" if A.regular is None else "regular"
     else:
         used_path = path
     value = replicas.job_throughput(E, T["ms_per_step"], ws)
     bytes_per_elem = algorithmic_bytes(E, N, nnz) / E
     peak, peak_kind = measured_peaks()
-    if used_path == "regular" and head == "mixed_df":
-        # float-float on the regular mesh: three kernels per assembly (Gauss-point metrics,
-        # contraction, row gather); the roofline is that of the whole assembly
-        knames = ["laplace_metric_kernel<f2>", "laplace_contract_kernel<f2>", "laplace_gather_kernel<f2>"]
+    if used_path == "regular" and (path == "auto" or head != "fp64"):
+        # on the regular mesh: the element matrices (float-float: Gauss-point metrics, then the contraction)
+        # and the row gather; the roofline is that of the whole assembly
+        t = {"fp64": "double", "mixed_df": "f2", "mixed": "float"}[head]
+        knames = (["laplace_metric_kernel<f2>", "laplace_contract_kernel<f2>"] if head == "mixed_df" else
+                  [f"laplace_matrix_kernel<{t}>"]) + [f"laplace_gather_kernel<{t}>"]
         per_launch_ms = T["kernel_ms_total"] / max(args.steps, 1)
         units_per_launch = E
     else:
@@ -421,9 +423,8 @@ def run_gfe(args):
         "clocks": T["clocks"],
         "e2e": {"value": replicas.job_throughput(E, e2e[head], ws), "unit": "elements/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
-        # element kernel launches + one coordinate split (regular path) or FP32 copy (colour path)
-        # per step for the FP32-pipe precisions
-        "gpu_launches": int(T["launches"]) + (args.steps if head != "fp64" else 0),
+        # element and gather kernels; on the colour path also one FP32 copy a step for the FP32-pipe precisions
+        "gpu_launches": int(T["launches"]) + (args.steps if head != "fp64" and used_path == "general" else 0),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind,
                      "traffic": None if tpu is None else tpu * units_per_launch,

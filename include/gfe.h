@@ -288,7 +288,7 @@ int gfe_laplace_assemble_regular_ws(int32_t nx, int32_t ny, int32_t nz, const do
 /* The rows of node layers [layer_begin, layer_end) only (layer = node index along xi3; layer_begin a
  * multiple of 8): those rows form one contiguous range of the CSR values, so an assembly split into
  * layer slabs can copy each slab's values to the host while the next slab computes.
- * convert_coords: convert the coordinates into the workspace first (needed in the first call of an
+ * convert_coords: convert (GFE_MIXED_DF: copy) the coordinates into the workspace first (needed in the first call of an
  * assembly; later calls of the same assembly pass 0 and reuse it; requires a workspace).  An empty
  * range (layer_begin == layer_end) with convert_coords only converts, so that slab calls on
  * several streams can all start once the conversion is done.
@@ -310,8 +310,8 @@ int gfe_laplace_assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, cons
  * uploads fill (coords_host / kappa_host NULL: the device copy is already current; kappa NULL:
  * unit conductivity); values [nnz] is the device CSR value array.  Host buffers should be pinned
  * for the copies to overlap.  The FP32-pipe precisions need a 16-byte aligned workspace: GFE_MIXED_DF of
- * gfe_laplace_regular_workspace_bytes bytes, GFE_MIXED of 12 bytes a node; nothing is allocated.  Asynchronous: the pipeline's
- * own streams start after the work already on `stream`, and `stream` waits for all of them, so
+ * gfe_laplace_regular_workspace_bytes bytes, GFE_MIXED of 12 bytes a node; nothing is allocated.  Asynchronous: the
+ * pipeline's own streams start after the work already on `stream`, and `stream` waits for all of them, so
  * values_host is complete once `stream` has reached this point.  Slab boundaries come from the
  * closed-form entry count of the clipped 27-point stencil, so row_ptr must be the structure of the
  * regular mesh (gfe_laplace_regular_check). */

@@ -73,8 +73,9 @@ __device__ __forceinline__ void finish(float&) {}
 
 // Forms without the final renormalisation (8 operations a sum instead of 11), for chains whose values do not cancel:
 // `lo` then reaches a few ulp(hi), and only products of two such values lose by it (they drop lo lo), so a
-// value is renormalised before it enters a product with another one.  Sums that cancel on sheared or flat elements (the
-// Gram products and their minors) are normalised: left raw, they cost 7 and 8 % in the error of an element sheared by 10.
+// value is renormalised before it enters a product with another one.  Sums that cancel on sheared or flat elements
+// (the Gram products and their minors) are normalised: left raw, they cost 7 and 8 % in the error of an element
+// sheared by 10.
 __device__ __forceinline__ f2 add_raw(f2 a, f2 b) {
   accum(a, b);
   return a;

@@ -54,8 +54,8 @@ void stage_end(int stage, void* token, cudaStream_t s, int launches);
 
 // Chains of small kernels, each adding one colour's entries: with `overlap` a launch may start once every CTA of the
 // kernel before it has called chain_release (or has ended), so its launch and first loads run under that kernel's end;
-// what the kernels before it wrote may be read (past the L1: __ldcg) or written after chain_wait only.  A kernel calls chain_wait before
-// chain_release: what precedes the whole chain is then complete when the next one starts.
+// what the kernels before it wrote may be read (past the L1: __ldcg) or written after chain_wait only.  A kernel calls
+// chain_wait before chain_release: what precedes the whole chain is then complete when the next one starts.
 namespace gfe {
 template <typename... Params, typename... Args>
 cudaError_t launch_chained(bool overlap, void (*kernel)(Params...), int grid, int block, cudaStream_t s, Args... args) {

@@ -18,14 +18,16 @@
 // (Slots that carry a barrier's number beside the value, read until all are current, save a round trip to the
 // L2 but have every CTA poll every slot: slower, 16 instead of 10 us an iteration.)
 // Measured, launched form -> resident: CG on the 64^3 Laplace system, FP32 matrix, 42 -> 12.3 us an iteration (the
-// sliced-ELL copy 47 MB, of which 32 MB are held on chip), FP64 52 -> 29 us (bound by the FP64 pipe); MINRES on the 8^3 Mooney-Rivlin
-// tangent, FP32, 24 -> 9.4 us an iteration.  MINRES chains two FP64 sums and two barriers behind 2 us of product.
+// sliced-ELL copy 47 MB, of which 32 MB are held on chip), FP64 52 -> 29 us (bound by the FP64 pipe); MINRES on the 8^3
+// Mooney-Rivlin tangent, FP32, 24 -> 9.4 us an iteration, on the 13^3 one (93 MB) 38 -> 17.  MINRES chains two FP64 sums
+// and two barriers behind 2 us of product.
 // A wait is bounded; when it runs out every CTA leaves and the solve returns GFE_ERR_TIMEOUT.
 #pragma once
 
 namespace {
 
-constexpr int kCgThreads = 1024;     // more warps hide the product's loads: at 768 threads an iteration at 64^3 took a fifth longer
+// more warps hide the product's loads: at 768 threads an iteration at 64^3 took a fifth longer
+constexpr int kCgThreads = 1024;
 constexpr int kMinresThreads = 768;  // 80 registers a thread, no spills: the waits invalidate the L1, so that a spill
                                      // costs an L2 round trip an iteration
 constexpr int kResPolls = 1 << 21;  // about a second
@@ -162,7 +164,8 @@ cg_resident(int n, SellMatrix<TM, IT> A, TV* x, TV* r, TV* z, TV* p, TV* q, cons
   }
   // this CTA's contiguous, equal share of the slices; as much of it as fits goes to shared memory
   const int slices = (n + kSell - 1) / kSell;
-  const int s0 = (int)((long long)slices * blockIdx.x / gridDim.x), s1 = (int)((long long)slices * (blockIdx.x + 1) / gridDim.x);
+  const int s0 = (int)((long long)slices * blockIdx.x / gridDim.x);
+  const int s1 = (int)((long long)slices * (blockIdx.x + 1) / gridDim.x);
   const long long e0 = s0 < s1 ? __ldg(A.sptr + s0) : 0;
   const int held = s0 < s1 ? (int)min((long long)cap, __ldg(A.sptr + s1 - 1) + __ldg(A.slen + s1 - 1) - e0) : 0;
   for (int i = threadIdx.x; i < held; i += kCgThreads) {

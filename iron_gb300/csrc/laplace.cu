@@ -287,7 +287,7 @@ __device__ __forceinline__ void pair_sums(T s0, T s1, T r, T pp1, T (&o)[3]) {
 // values (metric_scale), the symmetric part of each entry formed once per distinct triple of pairs (27 of
 // the 36 entries) and the two orders of each off-diagonal term added before they meet the entries.
 // Float-float sums stay unnormalised (df.cuh): the kernel is bound by its FP32 instructions and their fetch.  128^3:
-// metrics 405 -> 376 us, contraction 431 -> 382 (fewer operations) -> 328 us, assembly 1.27 -> 1.13 ms.
+// contraction 431 -> 382 (fewer operations) -> 328 us, assembly 1.27 -> 1.13 ms.
 template <typename T, typename MetricAt>
 __device__ __forceinline__ void hex8_contract_scaled(MetricAt Mg, T (&K)[36]) {
   const T r = from_double<T>(kPoverQ), pp1 = from_double<T>(kPP1);
@@ -568,10 +568,12 @@ __device__ __forceinline__ f2 acc_add(f2 a, f2 b) {
 // kernel takes the doubles apart with integer operations (layer calls: a copy of the doubles).
 // nodes [a, b) of n, three components
 template <typename T>
-__global__ void split_coords(long long n, long long a, long long b, const double* __restrict__ in, T* __restrict__ out) {
+__global__ void split_coords(long long n, long long a, long long b, const double* __restrict__ in,
+                             T* __restrict__ out) {
+  const long long step = (long long)gridDim.x * blockDim.x;
   for (int c = 0; c < 3; ++c) {
 #pragma unroll 4
-    for (long long i = a + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < b; i += (long long)gridDim.x * blockDim.x)
+    for (long long i = a + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < b; i += step)
       out[c * n + i] = from_double<T>(__ldg(in + c * n + i));
   }
 }
@@ -730,7 +732,7 @@ laplace_regular_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__
 // ---------------------------------------------------------------------------------------------
 // Float-float on Iron's regular mesh: element work in two kernels, then a row gather
 // ---------------------------------------------------------------------------------------------
-// The float-float element routine is about 9 k instructions of straight-line code per element; inside
+// The float-float element routine is about 9.7 k instructions of straight-line code per element; inside
 // the row-owning kernel its instruction stream does not fit the SM's instruction cache and warps
 // stall on instruction fetch.  Split, each kernel's code fits: the metric kernel forms the 8
 // Gauss-point metrics of every element once, the contraction kernel turns them into the 36 element
@@ -743,8 +745,9 @@ laplace_regular_kernel(int32_t nx, int32_t ny, int32_t nz, const T* __restrict__
 // Coordinates are read as doubles and each element takes its 24 apart (about 15 integer and FP32 operations each).
 // A copy split to float-float once per node, 40 us at 128^3, has to round to 48 bits, and relative to whatever point
 // that is: relative to the origin it loses digits on elements far from it, relative to the mesh's middle node on small
-// elements at its edge (a mesh graded by 1e-6 towards the origin: error 1.4e-12 of the matrix's norm relative to the middle
-// node, 2.8e-14 relative to the origin, 7.7e-15 here; 128^3 jittered cubes 3.0e-14, 5.8e-14, 4.0e-15).
+// elements at its edge.  Error against FP64, relative to the middle node, relative to the origin, and here: 1.4e-12,
+// 2.8e-14 and 7.7e-15 on a mesh graded by 1e-6 towards the origin, 3.0e-14, 5.8e-14 and 4.0e-15 at 128^3 jittered cubes.
+// The kernel takes 437 us there, 378 with split coordinates and its Gram products left unnormalised.
 template <typename T>
 __global__ void __launch_bounds__(128)
 laplace_metric_kernel(int32_t nx, int32_t ny, int32_t nz, const double* __restrict__ coords,
@@ -1205,8 +1208,8 @@ int launch_regular(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, const dou
     if (gather) {
       const long long E = (long long)nx * ny * nz;
       T* Kel = reinterpret_cast<T*>(base + cb);
-      laplace_matrix_kernel<T><<<(int)std::min<long long>((E + 127) / 128, 1 << 20), 128, 0, s>>>(nx, ny, nz, coords, kappa,
-                                                                                                  Kel, err);
+      const int grid = (int)std::min<long long>((E + 127) / 128, 1 << 20);
+      laplace_matrix_kernel<T><<<grid, 128, 0, s>>>(nx, ny, nz, coords, kappa, Kel, err);
       launch_gather<T>(s, nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
       if (!ws) gfe::scratch_free(base, s);
       return GFE_OK;
@@ -1248,9 +1251,10 @@ int launch_regular<double>(cudaStream_t s, int32_t nx, int32_t ny, int32_t nz, c
     const long long E = (long long)nx * ny * nz;
     if (E <= 64ll * gfe::sm_count())
       laplace_element64_small_kernel<<<(int)((E + 15) / 16), 128, 0, s>>>(nx, ny, nz, coords, kappa, Kel, err);
-    else
-      laplace_matrix_kernel<double><<<(int)std::min<long long>((E + 127) / 128, 1 << 20), 128, 0, s>>>(nx, ny, nz, coords,
-                                                                                                     kappa, Kel, err);
+    else {
+      const int grid = (int)std::min<long long>((E + 127) / 128, 1 << 20);
+      laplace_matrix_kernel<double><<<grid, 128, 0, s>>>(nx, ny, nz, coords, kappa, Kel, err);
+    }
     launch_gather<double>(s, nx, ny, nz, Kel, rp, values, values32, rhs, l0, l1);
     return GFE_OK;
   }
@@ -1351,8 +1355,9 @@ int assemble_regular_layers(int32_t nx, int32_t ny, int32_t nz, const double* co
     if (!workspace || !convert_coords)
       return gfe::set_error(GFE_ERR_ARG, "%s: an empty layer range needs a workspace and convert_coords", fn);
     const long long n = (nx + 1ll) * (ny + 1) * (nz + 1);
-    if (precision == GFE_MIXED) split_coords<float><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (float*)workspace);
-    else if (precision == GFE_MIXED_DF) split_coords<double><<<4 * gfe::sm_count(), 256, 0, s>>>(n, 0, n, coords, (double*)workspace);
+    const int grid = 4 * gfe::sm_count();
+    if (precision == GFE_MIXED) split_coords<float><<<grid, 256, 0, s>>>(n, 0, n, coords, (float*)workspace);
+    else if (precision == GFE_MIXED_DF) split_coords<double><<<grid, 256, 0, s>>>(n, 0, n, coords, (double*)workspace);
     GFE_LAUNCH_CHECK(fn);
     return GFE_OK;
   }
@@ -1515,7 +1520,8 @@ extern "C" int gfe_laplace_assemble_regular_host(int32_t nx, int32_t ny, int32_t
       rc = launch_regular<float>(cs, nx, ny, nz, coords, kappa, row_ptr, values, nullptr, rhs, err, workspace,
                                  l0, l1, false, true);
     else {
-      launch_gather<f2>(cs, nx, ny, nz, element_matrices_f2(workspace, nx, ny, nz), row_ptr, values, nullptr, rhs, l0, l1);
+      launch_gather<f2>(cs, nx, ny, nz, element_matrices_f2(workspace, nx, ny, nz), row_ptr, values, nullptr, rhs, l0,
+                        l1);
       rc = GFE_OK;
     }
     if (rc) return rc;

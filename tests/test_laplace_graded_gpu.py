@@ -40,7 +40,8 @@ def test_graded_mesh(gfe_cuda, ne, kind, span):
     got = A.assemble("mixed_df").clone()
     assert (got - ref).abs().max().item() <= 64 * 2.0 ** -48 * ref.abs().max().item()
     nx, ny, nz = ne
-    ws = torch.empty(int(_lib.load().gfe_laplace_regular_workspace_bytes(nx, ny, nz, 2)), dtype=torch.uint8, device="cuda")
+    nbytes = int(_lib.load().gfe_laplace_regular_workspace_bytes(nx, ny, nz, 2))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
     A.values.fill_(-7.0)
     coords = A.coords.clone()
     for l0 in range(0, nz + 1, 8):
